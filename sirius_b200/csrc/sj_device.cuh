@@ -35,6 +35,16 @@ __host__ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
   return x;
 }
 
+// The top 31 bits of mix64(x) in bits 31..1 of the result: the last xor-shift reaches bits 32..0 only,
+// and of the second product the high word alone is computed.
+__device__ __forceinline__ uint32_t mix64_high(uint64_t x) {
+  x ^= x >> 30;
+  x *= 0xbf58476d1ce4e5b9ull;
+  x ^= x >> 27;
+  const uint32_t lo = (uint32_t)x, hi = (uint32_t)(x >> 32);
+  return __umulhi(lo, 0x133111ebu) + lo * 0x94d049bbu + hi * 0x133111ebu;
+}
+
 template <typename K>
 __host__ __device__ __forceinline__ uint64_t key_u64(K k);
 // Keys enter the hash sign-extended to 64 bits, so an int32 key and its (key - key_min) + key_min
@@ -61,7 +71,7 @@ struct TableDev {
 };
 
 __device__ __forceinline__ uint32_t home_bucket(const TableDev& t, uint64_t kb) {
-  return t.log2_nb ? (uint32_t)(mix64(kb) >> (64 - t.log2_nb)) : 0u;
+  return t.log2_nb ? mix64_high(kb) >> (32 - t.log2_nb) : 0u;  // log2_nb <= 31
 }
 __device__ __forceinline__ uint32_t next_bucket(uint32_t b, uint32_t segmask) {
   return (b & ~segmask) | ((b + 1) & segmask);

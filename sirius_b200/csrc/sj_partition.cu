@@ -27,7 +27,7 @@ constexpr int kPartThreads = 256;
 constexpr int kMaxPartBits = kMaxPartitionBits;
 
 __device__ __forceinline__ int partition_of(uint64_t kb, int pbits) {
-  return pbits ? (int)(mix64(kb) >> (64 - pbits)) : 0;
+  return pbits ? (int)(mix64_high(kb) >> (32 - pbits)) : 0;
 }
 
 template <typename K>
@@ -48,26 +48,40 @@ __device__ __forceinline__ void hist_load4(const K* keys, int64_t i0, int64_t hi
 }
 
 // Histogram pass: each thread loads 4 groups of 4 consecutive keys (16-byte loads) per step, all
-// before counting them, so 8 (int64) or 4 (int32) vector loads per thread are in flight.
-template <typename K>
-__global__ void __launch_bounds__(kPartThreads) part_hist_kernel(PartSrc s, int pbits, int64_t chunk, bool vec,
-                                                                 int32_t* hist) {
+// before counting them, so 8 (int64) or 4 (int32) vector loads per thread are in flight. Whole steps
+// of columns without NULLs are counted without a check per row. 64M int64 keys, 64 partitions, two
+// CTAs of 1024 threads per SM: 97 us (5.5 TB/s); with a check of every row and the whole 64-bit hash
+// 116 us. Eight counters per partition, chosen by lane, changed nothing: not the atomics' conflicts.
+template <typename K, int THREADS = kPartThreads>
+__global__ void __launch_bounds__(THREADS) part_hist_kernel(PartSrc s, int pbits, int64_t chunk, bool vec,
+                                                            int32_t* hist) {
   extern __shared__ int32_t h[];
   constexpr int kGroups = 4;
+  constexpr uint32_t kStep = THREADS * 4;
   const int P = 1 << pbits;
-  for (int p = threadIdx.x; p < P; p += blockDim.x) h[p] = 0;
+  for (int p = threadIdx.x; p < P; p += THREADS) h[p] = 0;
   __syncthreads();
   const int64_t lo = (int64_t)blockIdx.x * chunk;
   const int64_t hi = lo + chunk < s.n ? lo + chunk : s.n;
   const K* keys = static_cast<const K*>(s.keys);
-  const int64_t step = (int64_t)blockDim.x * 4;
-  for (int64_t base = lo; base < hi; base += step * kGroups) {
+  const bool plain = s.kvalid == nullptr && vec;
+  for (int64_t base = lo; base < hi; base += kStep * kGroups) {
     K k[kGroups][4];
+    const K* mine = keys + base + threadIdx.x * 4;
+    if (plain && base + kStep * kGroups <= hi) {
 #pragma unroll
-    for (int g = 0; g < kGroups; ++g) hist_load4<K>(keys, base + g * step + (int64_t)threadIdx.x * 4, hi, vec, k[g]);
+      for (int g = 0; g < kGroups; ++g) hist_load4<K>(mine, g * kStep, (int64_t)kStep * kGroups, true, k[g]);
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) atomicAdd(&h[partition_of(key_u64<K>(k[g][j]), pbits)], 1);
+      continue;
+    }
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) hist_load4<K>(keys, base + g * kStep + threadIdx.x * 4, hi, vec, k[g]);
 #pragma unroll
     for (int g = 0; g < kGroups; ++g) {
-      const int64_t i0 = base + g * step + (int64_t)threadIdx.x * 4;
+      const int64_t i0 = base + g * kStep + threadIdx.x * 4;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         if (i0 + j < hi && bit_valid(s.kvalid, s.kvoff, i0 + j))
@@ -75,7 +89,7 @@ __global__ void __launch_bounds__(kPartThreads) part_hist_kernel(PartSrc s, int 
     }
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < P; p += blockDim.x) hist[(int64_t)p * gridDim.x + blockIdx.x] = h[p];
+  for (int p = threadIdx.x; p < P; p += THREADS) hist[(int64_t)p * gridDim.x + blockIdx.x] = h[p];
 }
 
 // Scatter pass, staged through shared memory one tile of kTile rows at a time: the tile's rows
@@ -626,6 +640,229 @@ sj_status radix_partition(const PartSrc& src, int key_type, int pbits, const Par
     KernelTimer timer("partition_scatter", s);
     part_scatter_kernel<int64_t><<<G, kPartThreads, m.total, s>>>(src, pbits, chunk, offs, dst, m);
   }
+  SJ_CUDA_TRY(cudaGetLastError());
+  *d_total_out = offs + PG;
+  *d_offs_out = offs;
+  *grid_out = G;
+  return SJ_OK;
+}
+
+// ------------------------------------------------------------------------------------------------
+// Column scatter of the partition operator: no row ids and no copy of the partition key are written,
+// only the caller's columns (1..8 bytes wide, any number). A tile of kColTile rows is ranked by
+// partition once (shared-memory atomics) and its output positions are kept sorted in shared memory;
+// each column then goes through one staging buffer: placed at the rows' sorted slots, written out in
+// partition runs with consecutive threads on consecutive positions. The loads of the next column (or
+// of the next tile's keys) are in registers before a column is written, so reads overlap writes. The
+// key column, when the caller wants it reordered too, is staged from the registers it was hashed in.
+// 4096-row tiles: a run holds 4096 / P rows, twice the length of the 2048-row tiles above. 64M int64
+// keys and one int64 column into 64 partitions: 1,114 us with row ids and a key copy written by
+// part_scatter_fast_kernel, 502 us here (4.3 TB/s of 2.1 GB; while it took 514 us, other shapes of
+// threads x rows x CTAs per SM took 542 (256x8x4), 541 (512x4x3), 524 (256x16x2), 526 us (1024x4x2)). It is bound by its write fronts, P per CTA, that
+// advance by one run of a tile at a time.
+// ------------------------------------------------------------------------------------------------
+constexpr int kColThreads = 512;
+constexpr int kColRows = 8;      // rows per thread
+constexpr int kColCtasPerSm = 2;
+constexpr int kColHistThreads = 1024;
+constexpr int kColTile = kColThreads * kColRows;
+
+// Row of a tile that thread t holds as its j-th: consecutive row pairs, as fast_row.
+__device__ __forceinline__ int col_row(int j, int t) { return (j >> 1) * 2 * kColThreads + 2 * t + (j & 1); }
+
+template <typename T>
+__device__ __forceinline__ void col_load_t(const T* src, bool pairs, uint32_t t0, uint32_t hi, uint64_t (&v)[kColRows]) {
+#pragma unroll
+  for (int j = 0; j < kColRows; j += 2) {
+    const uint32_t i = t0 + col_row(j, threadIdx.x);
+    v[j] = v[j + 1] = 0;
+    if constexpr (sizeof(T) >= 4) {
+      if (pairs && i + 1 < hi) {
+        ld_pair_cs(src + i, v[j], v[j + 1]);
+        continue;
+      }
+    }
+    if (i < hi) v[j] = (uint64_t)__ldcs(src + i);
+    if (i + 1 < hi) v[j + 1] = (uint64_t)__ldcs(src + i + 1);
+  }
+}
+
+__device__ __forceinline__ void col_load(const PartColumn& c, uint32_t t0, uint32_t hi, uint64_t (&v)[kColRows]) {
+  if (c.bits) {
+#pragma unroll
+    for (int j = 0; j < kColRows; ++j) {
+      const uint32_t i = t0 + col_row(j, threadIdx.x);
+      v[j] = i < hi && bit_valid(c.bits, c.voff, i) ? 1 : 0;
+    }
+    return;
+  }
+  switch (c.width) {
+    case 8: return col_load_t(static_cast<const unsigned long long*>(c.src), c.pairs, t0, hi, v);
+    case 4: return col_load_t(static_cast<const unsigned int*>(c.src), c.pairs, t0, hi, v);
+    case 2: return col_load_t(static_cast<const unsigned short*>(c.src), false, t0, hi, v);
+    default: return col_load_t(static_cast<const unsigned char*>(c.src), false, t0, hi, v);
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void col_stage(void* stage, int tile_n, const uint16_t (&slot)[kColRows],
+                                          const uint64_t (&v)[kColRows]) {
+#pragma unroll
+  for (int j = 0; j < kColRows; ++j)
+    if (col_row(j, threadIdx.x) < tile_n) static_cast<T*>(stage)[slot[j]] = (T)v[j];
+}
+
+template <typename T>
+__device__ __forceinline__ void col_write(const void* stage, const uint32_t* sdst, void* dst, int tile_n) {
+#pragma unroll
+  for (int q = 0; q < kColRows; ++q) {
+    const int s = q * kColThreads + threadIdx.x;
+    if (s < tile_n) static_cast<T*>(dst)[sdst[s]] = static_cast<const T*>(stage)[s];
+  }
+}
+
+template <typename K>
+__global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_columns_kernel(const K* __restrict__ keys, bool key_pairs,
+                                                                      uint32_t n, int pbits, uint32_t chunk,
+                                                                      const int64_t* __restrict__ off, PartColumns cols) {
+  using U = std::conditional_t<sizeof(K) == 8, unsigned long long, unsigned int>;
+  __shared__ __align__(16) unsigned char stage[kColTile * 8];
+  __shared__ unsigned int s_wsum[kColThreads / 32];
+  extern __shared__ uint32_t s_col[];
+  const int P = 1 << pbits;
+  uint32_t* sdst = s_col;              // output position of each sorted slot
+  uint32_t* cur = sdst + kColTile;     // next output position of each partition
+  uint32_t* gbase = cur + P;           // output position of a row = gbase[its partition] + its sorted slot
+  uint32_t* tcnt = gbase + P;          // the tile's rows of each partition
+  uint32_t* tbase = tcnt + P;          // their first sorted slot
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  for (int p = tid; p < P; p += kColThreads) {
+    cur[p] = (uint32_t)off[(int64_t)p * gridDim.x + blockIdx.x];
+    tcnt[p] = 0;
+  }
+  const uint32_t lo = min(n, blockIdx.x * chunk), hi = min(n, lo + chunk);
+  uint64_t v[kColRows];
+  const U* ukeys = reinterpret_cast<const U*>(keys);
+  if (lo < hi) col_load_t(ukeys, key_pairs, lo, hi, v);
+  __syncthreads();
+  for (uint32_t t0 = lo; t0 < hi; t0 += kColTile) {
+    const int tile_n = (int)(hi - t0 < kColTile ? hi - t0 : kColTile);
+    // 1. rank every row within its partition
+    uint32_t pr[kColRows];  // partition << 16 | rank
+#pragma unroll
+    for (int j = 0; j < kColRows; ++j) {
+      if (col_row(j, tid) >= tile_n) continue;
+      const uint32_t p = (uint32_t)partition_of(key_u64<K>((K)v[j]), pbits);
+      pr[j] = p << 16 | atomicAdd(&tcnt[p], 1u);
+    }
+    __syncthreads();
+    // 2. exclusive scan of the tile's counts
+    constexpr int kBins = (1 << kMaxPartBits) / kColThreads;
+    uint32_t c[kBins], acc = 0;
+#pragma unroll
+    for (int q = 0; q < kBins; ++q) {
+      const int p = tid * kBins + q;
+      c[q] = p < P ? tcnt[p] : 0;
+      acc += c[q];
+    }
+    uint32_t incl = warp_inclusive_sum(acc);
+    if (lane == 31) s_wsum[wid] = incl;
+    __syncthreads();
+    uint32_t run = incl - acc;
+    for (int w = 0; w < wid; ++w) run += s_wsum[w];
+#pragma unroll
+    for (int q = 0; q < kBins; ++q) {
+      const int p = tid * kBins + q;
+      if (p < P) {
+        tbase[p] = run;
+        tcnt[p] = 0;
+        gbase[p] = cur[p] - run;
+        cur[p] += c[q];
+      }
+      run += c[q];
+    }
+    __syncthreads();
+    // 3. the rows' sorted slots and the slots' output positions
+    uint16_t slot[kColRows];
+#pragma unroll
+    for (int j = 0; j < kColRows; ++j) {
+      slot[j] = 0;
+      if (col_row(j, tid) >= tile_n) continue;
+      const uint32_t p = pr[j] >> 16;
+      slot[j] = (uint16_t)(tbase[p] + (pr[j] & 0xffffu));
+      sdst[slot[j]] = gbase[p] + slot[j];
+    }
+    __syncthreads();
+    // 4. column by column (the key column, if wanted, comes first and is already in registers)
+    const uint32_t t1 = t0 + kColTile;
+    if (cols.n == 0 || !cols.c[0].is_key) {
+      if (cols.n > 0) col_load(cols.c[0], t0, hi, v);
+      else if (t1 < hi) col_load_t(ukeys, key_pairs, t1, hi, v);
+    }
+    for (int q = 0; q < cols.n; ++q) {
+      const PartColumn& col = cols.c[q];
+      switch (col.width) {
+        case 8: col_stage<unsigned long long>(stage, tile_n, slot, v); break;
+        case 4: col_stage<unsigned int>(stage, tile_n, slot, v); break;
+        case 2: col_stage<unsigned short>(stage, tile_n, slot, v); break;
+        default: col_stage<unsigned char>(stage, tile_n, slot, v); break;
+      }
+      __syncthreads();
+      if (q + 1 < cols.n) col_load(cols.c[q + 1], t0, hi, v);
+      else if (t1 < hi) col_load_t(ukeys, key_pairs, t1, hi, v);
+      switch (col.width) {
+        case 8: col_write<unsigned long long>(stage, sdst, col.dst, tile_n); break;
+        case 4: col_write<unsigned int>(stage, sdst, col.dst, tile_n); break;
+        case 2: col_write<unsigned short>(stage, sdst, col.dst, tile_n); break;
+        default: col_write<unsigned char>(stage, sdst, col.dst, tile_n); break;
+      }
+      __syncthreads();
+    }
+    if (cols.n == 0) __syncthreads();
+  }
+}
+
+static size_t columns_smem(int pbits) {
+  return ((size_t)kColTile + 4 * ((size_t)1 << pbits)) * sizeof(uint32_t);
+}
+
+sj_status partition_columns(const void* keys, int key_type, int64_t n, int pbits, const PartColumns& cols, void* scratch,
+                            int device, cudaStream_t s, const int64_t** d_total_out, const int64_t** d_offs_out,
+                            int* grid_out) {
+  if (pbits < 0 || pbits > kMaxPartBits) return set_error(SJ_ERR_INVALID, "partition bits out of range");
+  const int G = sm_count(device) * kColCtasPerSm;  // one chunk per CTA, all resident
+  const int P = 1 << pbits;
+  const size_t PG = (size_t)P * G;
+  char* base = static_cast<char*>(scratch);
+  int32_t* hist = reinterpret_cast<int32_t*>(base);
+  int64_t* offs = reinterpret_cast<int64_t*>(base + ((PG * 4 + 255) & ~(size_t)255));
+  int64_t* tmp = reinterpret_cast<int64_t*>(base + ((PG * 4 + 255) & ~(size_t)255) + (((PG + 1) * 8 + 255) & ~(size_t)255));
+  const int64_t chunk = std::max<int64_t>(4, ((n + G - 1) / G + 3) / 4 * 4);
+  const int kw = key_type == SJ_INT32 ? 4 : 8;
+  const bool vec = ((uintptr_t)keys & 15u) == 0, key_pairs = ((uintptr_t)keys % (2 * kw)) == 0;
+  PartSrc src{};
+  src.keys = keys;
+  src.n = n;
+  {
+    KernelTimer timer("partition_hist", s);
+    if (key_type == SJ_INT32)
+      part_hist_kernel<int32_t, kColHistThreads><<<G, kColHistThreads, P * sizeof(int32_t), s>>>(src, pbits, chunk, vec, hist);
+    else
+      part_hist_kernel<int64_t, kColHistThreads><<<G, kColHistThreads, P * sizeof(int32_t), s>>>(src, pbits, chunk, vec, hist);
+  }
+  {
+    KernelTimer timer("partition_scan", s);
+    device_exclusive_scan<int32_t, int64_t>(hist, offs, nullptr, (int64_t)PG, tmp, s);
+  }
+  auto go = [&](auto k) -> sj_status {
+    using K = decltype(k);
+    const size_t smem = columns_smem(pbits);
+    SJ_CUDA_TRY(cudaFuncSetAttribute(part_columns_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KernelTimer timer("partition_scatter", s);
+    part_columns_kernel<K><<<G, kColThreads, smem, s>>>(static_cast<const K*>(keys), key_pairs, (uint32_t)n, pbits, (uint32_t)chunk, offs, cols);
+    return SJ_OK;
+  };
+  if (cols.n > 0 && n > 0) SJ_TRY(key_type == SJ_INT32 ? go(int32_t{}) : go(int64_t{}));
   SJ_CUDA_TRY(cudaGetLastError());
   *d_total_out = offs + PG;
   *d_offs_out = offs;

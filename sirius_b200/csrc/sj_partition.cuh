@@ -40,4 +40,25 @@ sj_status radix_partition(const PartSrc& src, int key_type, int pbits, const Par
                           int device, cudaStream_t s, const int64_t** d_total_out, const int64_t** d_offs_out,
                           int* grid_out);
 
+// Partitioning of columns alone (the partition operator): every row is valid, and no row ids or key
+// copies are made. A column is `width` bytes per row at src, or one validity bit per row (bits != NULL)
+// written as one byte; is_key: the partition key itself (same type), which must come first; pairs: src
+// starts on a multiple of twice the width (row pairs are vector loads).
+struct PartColumn {
+  const void* src;
+  const uint32_t* bits;
+  int64_t voff;
+  void* dst;
+  int32_t width;
+  int16_t is_key;
+  int16_t pairs;
+};
+struct PartColumns {
+  int32_t n;
+  PartColumn c[2 * kMaxPayload];
+};
+sj_status partition_columns(const void* keys, int key_type, int64_t n, int pbits, const PartColumns& cols, void* scratch,
+                            int device, cudaStream_t s, const int64_t** d_total_out, const int64_t** d_offs_out,
+                            int* grid_out);
+
 }  // namespace sj

@@ -1,8 +1,8 @@
 // Hash partitioning of a table (the partition operator's hash_partition,
 // src/op/partition/gpu_partition_impl.cpp:29-110, which feeds partitioned joins): rows are
 // reordered so that partition p occupies [offsets[p], offsets[p+1]). It runs the join's own
-// radix partition (sj_partition.cu: per-CTA histogram, scan, shared-memory counting-sort scatter)
-// on a 64-bit partition key:
+// radix partition (sj_partition.cu: per-CTA histogram, scan, and the column scatter, which writes the
+// caller's columns and nothing else) on a 64-bit partition key:
 //   - one key column without NULLs: the key itself (the partition is the top bits of mix64(key),
 //     the same function that splits a partitioned hash table into segments);
 //   - NULLs or several key columns: a folded key (k0, then mix64(h) ^ k_c per further column), and
@@ -84,11 +84,8 @@ sj_status hash_partition(const sj_column* keys, int n_keys, const sj_column* col
   int device = 0;
   cudaGetDevice(&device);
   const bool folded = n_keys > 1 || keys[0].validity != nullptr;
-  const int kw = folded || keys[0].type == SJ_INT64 ? 8 : 4;
   auto a256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  size_t bytes = a256((size_t)std::max<int64_t>(n, 1) * kw) * (folded ? 2 : 1)  // folded key + partitioned keys
-                 + a256((size_t)std::max<int64_t>(n, 1) * 4)                     // row ids
-                 + partition_scratch_bytes(pbits, device);
+  size_t bytes = (folded ? a256((size_t)std::max<int64_t>(n, 1) * 8) : 0) + partition_scratch_bytes(pbits, device);
   for (int c = 0; c < n_cols; ++c) bytes += cols[c].validity ? a256((size_t)std::max<int64_t>(n, 1)) : 0;
   Scratch sc;
   SJ_TRY(sc.get(alloc, bytes, s));
@@ -116,27 +113,33 @@ sj_status hash_partition(const sj_column* keys, int n_keys, const sj_column* col
     }
     key_data = hk;
   }
-  PartSrc ps{};
-  PartDst pd{};
-  ps.keys = key_data;
-  ps.n = n;
-  ps.n_pay = n_cols;
-  pd.keys = carve((size_t)std::max<int64_t>(n, 1) * kw);
-  pd.rid = reinterpret_cast<int32_t*>(carve((size_t)std::max<int64_t>(n, 1) * 4));
+  // the columns, and a byte per row for each one that has NULLs; the key column, if it is among them,
+  // goes first (it is already in registers when its tile is ranked)
+  PartColumns pc{};
+  uint8_t* valid8[kMaxPayload] = {};
+  auto add = [&](const void* src, const uint32_t* bits, int64_t voff, void* dst, int width, bool is_key) {
+    pc.c[pc.n++] = PartColumn{src, bits, voff, dst, width, (int16_t)is_key, (int16_t)((uintptr_t)src % (2 * width) == 0)};
+  };
+  int key_col = -1;
+  for (int c = n_cols - 1; c >= 0; --c)
+    if (!folded && cols[c].data == key_data && type_width(cols[c].type) == type_width(key_type)) key_col = c;
+  if (key_col >= 0) add(key_data, nullptr, 0, out[key_col].data, type_width(key_type), true);
   for (int c = 0; c < n_cols; ++c) {
-    ps.pay[c] = column_payload(cols[c].data, cols[c].validity, cols[c].validity_offset, type_width(cols[c].type));
-    pd.pay[c] = out[c].data;
-    pd.valid8[c] = cols[c].validity ? reinterpret_cast<uint8_t*>(carve((size_t)std::max<int64_t>(n, 1))) : nullptr;
+    const int w = type_width(cols[c].type);
+    if (c != key_col) add(cols[c].data, nullptr, 0, out[c].data, w, false);
+    if (!cols[c].validity) continue;
+    valid8[c] = reinterpret_cast<uint8_t*>(carve((size_t)std::max<int64_t>(n, 1)));
+    add(nullptr, cols[c].validity, cols[c].validity_offset, valid8[c], 1, false);
   }
   void* pscratch = carve(partition_scratch_bytes(pbits, device));
   const int64_t *d_total, *d_offs;
   int G;
-  SJ_TRY(radix_partition(ps, key_type, pbits, pd, pscratch, device, s, &d_total, &d_offs, &G));
+  SJ_TRY(partition_columns(key_data, key_type, n, pbits, pc, pscratch, device, s, &d_total, &d_offs, &G));
   partition_starts_kernel<<<1, 1024, 0, s>>>(d_offs, d_total, 1 << pbits, G, d_offsets);
   for (int c = 0; c < n_cols; ++c) {
-    if (!pd.valid8[c] || n == 0) continue;
+    if (!valid8[c] || n == 0) continue;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sm_count(device) * 8));
-    bytes_to_bits_kernel<<<grid, 256, 0, s>>>(pd.valid8[c], n, out[c].validity);
+    bytes_to_bits_kernel<<<grid, 256, 0, s>>>(valid8[c], n, out[c].validity);
   }
   SJ_CUDA_TRY(cudaGetLastError());
   return SJ_OK;
