@@ -125,11 +125,9 @@ typedef enum sj_slot_kind {
   SJ_SLOT_WIDE128  = 1  /* {int64 key, row id} pair, inserted by 128-bit atomicCAS */
 } sj_slot_kind;
 
-/* Output reservation of the single-pass probe: matches are always compacted warp-aggregated
- * (prefix over the lanes' hit counts); the range is then reserved with one atomicAdd per warp or
- * one per CTA tile. AUTO picks per-CTA for probes of 2^20 rows or more. */
-/* How probe matches reserve output positions: one atomicAdd per warp, per CTA tile (for probes of
- * 2^20 rows or more under AUTO), or per warp with warps taking tiles from a shared counter. */
+/* How probe matches reserve output positions. A CTA of the unit probe reserves once for its 256 or 1024
+ * rows, whatever is asked for here; the staged kernel reserves per warp or per CTA tile (AUTO: per CTA for
+ * probes of 2^20 rows or more). */
 typedef enum sj_aggregation {
   SJ_AGG_AUTO = 0,
   SJ_AGG_WARP = 1,
@@ -139,12 +137,11 @@ typedef enum sj_aggregation {
 
 /* Tunables. Zero-initialised fields take defaults (sj_default_params fills them in). */
 /* How a DISTINCT probe reads its rows and writes its output. DIRECT: lanes write their own
- * matches at positions ranked by warp ballots (no shared-memory staging of matches); it serves
- * outputs of row ids, up to 2 probe payloads and up to 3 build payloads of 4 or 8 bytes without
- * NULLs (attached build payloads: 8-byte fields). DIRECT_TMA: DIRECT with the probe rows (keys,
- * payloads) bulk-copied into shared memory two tiles ahead by the TMA engine; needs 16-byte
- * aligned probe columns. STAGED: matches are staged per warp in shared memory and written column
- * by column; it serves every output shape. AUTO takes DIRECT where it applies, else STAGED. */
+ * matches at positions ranked by warp ballots (no staging of matches); it serves outputs of row ids,
+ * up to 2 probe payloads and up to 3 build payloads of 4 or 8 bytes without NULLs. DIRECT_TMA: DIRECT
+ * with the probe rows (keys, payloads) bulk-copied into shared memory two tiles ahead by the TMA engine;
+ * needs 16-byte aligned probe columns. STAGED: matches are staged per warp in shared memory and written
+ * column by column; it serves every output shape. AUTO takes DIRECT where it applies, else STAGED. */
 typedef enum sj_probe_kernel {
   SJ_PROBE_KERNEL_AUTO = 0,
   SJ_PROBE_KERNEL_STAGED = 1,
@@ -173,13 +170,13 @@ typedef struct sj_join_params {
                                1..10 = that many bits (2^bits partitions) */
   int32_t force_wide;       /* 1 = use SJ_SLOT_WIDE128 even when the packed encoding fits */
   int32_t ctas_per_sm;      /* grid = ctas_per_sm * SM count for grid-stride kernels; default 4 */
-  int32_t aggregation;      /* sj_aggregation: how probe matches reserve output positions */
+  int32_t aggregation;      /* sj_aggregation: how the staged probe reserves output positions */
   int32_t probe_kernel;     /* sj_probe_kernel: write-out of DISTINCT probes; default AUTO */
-  int32_t rows_per_lane;    /* probe rows per lane and tile of the direct kernel: 2 or 4; 0 = 2 */
+  int32_t rows_per_lane;    /* 0, 2, 3 or 4: accepted and ignored (the unit probe holds 1 or 4 rows per
+                               lane, by the probe's size) */
   int32_t probe_partition_mb; /* partitioned probe: table megabytes per probe partition (the part
                                  of the table one sweep keeps in L2); 0 = default (48) */
-  int32_t table_l2_priority;  /* sj_l2_priority of the table's slot and record loads in the
-                                 direct probe kernels */
+  int32_t table_l2_priority;  /* sj_l2_priority of the table's slot loads in the DIRECT_TMA probe */
   int32_t bloom_bits_per_key; /* > 0: the build also produces the join's dynamic filter (the
                                  blocked Bloom filter of sj_bloom_build, that many bits per build
                                  row), its bits set by the insert pass itself, so the filter costs no

@@ -321,8 +321,10 @@ static TableDev make_dev(const sj_table* t) {
   d.slots = t->slots;
   d.grp_off = t->grp_off;
   d.grp_rid = t->grp_rid;
+  // A table without valid keys has EMPTY slots only. Its range is [0, 0]: key 0 may be looked up (its key
+  // field is not EMPTY's), a key whose key field is all ones may not.
   d.kmin = t->kmin;
-  d.kmax = t->kmax;
+  d.kmax = std::max(t->kmin, t->kmax);
   d.log2_nb = (uint32_t)t->log2_nb;
   d.segmask = (uint32_t)((1ull << t->seg_log2) - 1);
   d.rbits = (uint32_t)t->rid_bits;

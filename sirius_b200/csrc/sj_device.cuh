@@ -63,7 +63,7 @@ struct TableDev {
   const void* slots;
   const int32_t* grp_off;  // GROUPED only
   const int32_t* grp_rid;  // GROUPED only
-  int64_t kmin, kmax;      // valid key range; kmax < kmin for an empty table
+  int64_t kmin, kmax;      // valid key range ([0, 0] for a table without valid keys)
   uint32_t log2_nb;
   uint32_t segmask;        // (1 << seg_log2) - 1
   uint32_t rbits;

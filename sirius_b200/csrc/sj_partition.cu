@@ -344,16 +344,11 @@ __device__ __forceinline__ void fast_load_tile(const PartSrc& s, int64_t t0, int
   }
 }
 
-// LOCAL: no global offsets — every tile is written back in place, sorted by partition, and its
-// per-partition runs go to run_off / run_cnt[tile * P + p] (the probe walks them partition-major).
-// VEC: the source columns take pair loads (fast_load_tile) and, when LOCAL, the destination
-// columns pair stores. 16-byte loads and stores took the tile-local scatter of 64M int64 rows with
-// one 8-byte payload from 0.492 to 0.482 ms (same box, 30 steps, two runs each).
-template <typename K, int NP, bool LOCAL = false, bool VEC = false>
+// VEC: the source columns take pair loads (fast_load_tile).
+template <typename K, int NP, bool VEC = false>
 __global__ void __launch_bounds__(kPartThreads, 3) part_scatter_fast_kernel(PartSrc s, int pbits, int64_t chunk,
                                                                          const int64_t* __restrict__ off, PartDst d,
-                                                                         FastSmem m, int32_t* run_off = nullptr,
-                                                                         int32_t* run_cnt = nullptr) {
+                                                                         FastSmem m) {
   extern __shared__ __align__(16) unsigned char sm[];
   unsigned long long* cur = reinterpret_cast<unsigned long long*>(sm + m.cur);
   unsigned int* tcnt = reinterpret_cast<unsigned int*>(sm + m.tcnt);
@@ -364,8 +359,7 @@ __global__ void __launch_bounds__(kPartThreads, 3) part_scatter_fast_kernel(Part
   __shared__ unsigned int s_wsum[kPartThreads / 32];
   const int P = 1 << pbits;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (!LOCAL)
-    for (int p = tid; p < P; p += kPartThreads) cur[p] = (unsigned long long)off[(int64_t)p * gridDim.x + blockIdx.x];
+  for (int p = tid; p < P; p += kPartThreads) cur[p] = (unsigned long long)off[(int64_t)p * gridDim.x + blockIdx.x];
   const int64_t lo = (int64_t)blockIdx.x * chunk;
   const int64_t hi = lo + chunk < s.n ? lo + chunk : s.n;
   K* okeys = static_cast<K*>(d.keys);
@@ -419,13 +413,6 @@ __global__ void __launch_bounds__(kPartThreads, 3) part_scatter_fast_kernel(Part
     unsigned tile_valid = 0;
     for (int w = 0; w < kPartThreads / 32; ++w) tile_valid += s_wsum[w];
     __syncthreads();
-    if (LOCAL) {  // after the barrier: toff[p] is written by thread p / kBinsPerThread
-      const int64_t ti = t0 / kTile;
-      for (int p = tid; p < P; p += kPartThreads) {
-        run_off[ti * P + p] = (int32_t)(t0 + toff[p]);
-        run_cnt[ti * P + p] = (int32_t)tcnt[p];
-      }
-    }
     // 3. counting-sort the tile into shared memory (payloads straight to their sorted slot, with
     //    each row's output position, so the write-out reads nothing per partition)
 #pragma unroll
@@ -434,55 +421,27 @@ __global__ void __launch_bounds__(kPartThreads, 3) part_scatter_fast_kernel(Part
       const unsigned slot = toff[pr[j]] + rank[j];
       skey[slot] = kk[j];
       srid[slot] = (int32_t)fast_row(t0, j, tid);
-      if (!LOCAL) sdst[slot] = (uint32_t)cur[pr[j]] + rank[j];  // LOCAL: the tile's own rows
+      sdst[slot] = (uint32_t)cur[pr[j]] + rank[j];
 #pragma unroll
       for (int c = 0; c < NP; ++c) reinterpret_cast<uint64_t*>(sm + m.pay[c])[slot] = pv[c][j];
     }
     __syncthreads();
     // 4. loads of the next tile go out before this tile's write-out
     if (t0 + kTile < hi) fast_load_tile<K, NP, VEC>(s, t0 + kTile, hi, kk, pv, live);
-    if constexpr (LOCAL && VEC) {  // row pairs: t0 and the staging slots are even
-      using K2 = std::conditional_t<sizeof(K) == 8, longlong2, int2>;
-      for (unsigned slot = 2 * tid; slot < tile_valid; slot += 2 * kPartThreads) {
-        const uint32_t pos = (uint32_t)t0 + slot;
-        if (slot + 1 < tile_valid) {
-          *reinterpret_cast<K2*>(okeys + pos) = *reinterpret_cast<const K2*>(skey + slot);
-          *reinterpret_cast<int2*>(d.rid + pos) = *reinterpret_cast<const int2*>(srid + slot);
+    for (unsigned slot = tid; slot < tile_valid; slot += kPartThreads) {
+      const uint32_t pos = sdst[slot];
+      okeys[pos] = skey[slot];
+      d.rid[pos] = srid[slot];
 #pragma unroll
-          for (int c = 0; c < NP; ++c) {
-            const ulonglong2 x = reinterpret_cast<const ulonglong2*>(sm + m.pay[c])[slot >> 1];
-            if (s.pay[c].width == 8) *reinterpret_cast<ulonglong2*>(static_cast<unsigned long long*>(d.pay[c]) + pos) = x;
-            else *reinterpret_cast<uint2*>(static_cast<unsigned int*>(d.pay[c]) + pos) = make_uint2((unsigned)x.x, (unsigned)x.y);
-          }
-        } else {
-          okeys[pos] = skey[slot];
-          d.rid[pos] = srid[slot];
-#pragma unroll
-          for (int c = 0; c < NP; ++c) {
-            const uint64_t x = reinterpret_cast<const uint64_t*>(sm + m.pay[c])[slot];
-            if (s.pay[c].width == 8) static_cast<unsigned long long*>(d.pay[c])[pos] = x;
-            else static_cast<unsigned int*>(d.pay[c])[pos] = (unsigned int)x;
-          }
-        }
-      }
-    } else {
-      for (unsigned slot = tid; slot < tile_valid; slot += kPartThreads) {
-        const uint32_t pos = LOCAL ? (uint32_t)t0 + slot : sdst[slot];
-        okeys[pos] = skey[slot];
-        d.rid[pos] = srid[slot];
-#pragma unroll
-        for (int c = 0; c < NP; ++c) {
-          const uint64_t x = reinterpret_cast<const uint64_t*>(sm + m.pay[c])[slot];
-          if (s.pay[c].width == 8) static_cast<unsigned long long*>(d.pay[c])[pos] = x;
-          else static_cast<unsigned int*>(d.pay[c])[pos] = (unsigned int)x;
-        }
+      for (int c = 0; c < NP; ++c) {
+        const uint64_t x = reinterpret_cast<const uint64_t*>(sm + m.pay[c])[slot];
+        if (s.pay[c].width == 8) static_cast<unsigned long long*>(d.pay[c])[pos] = x;
+        else static_cast<unsigned int*>(d.pay[c])[pos] = (unsigned int)x;
       }
     }
     __syncthreads();
-    if (!LOCAL) {
-      for (int p = tid; p < P; p += kPartThreads) cur[p] += tcnt[p];
-      __syncthreads();
-    }
+    for (int p = tid; p < P; p += kPartThreads) cur[p] += tcnt[p];
+    __syncthreads();
   }
 }
 
@@ -501,13 +460,13 @@ static sj_status launch_fast_scatter(const PartSrc& src, int pbits, int64_t chun
   auto go = [&](auto kernel) -> sj_status {
     SJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m.total));
     KernelTimer timer("partition_scatter", s);
-    kernel<<<G, kPartThreads, m.total, s>>>(src, pbits, chunk, offs, dst, m, nullptr, nullptr);
+    kernel<<<G, kPartThreads, m.total, s>>>(src, pbits, chunk, offs, dst, m);
     return SJ_OK;
   };
   if (pair_aligned_src(src, sizeof(K))) {
-    if (src.n_pay == 0) return go(part_scatter_fast_kernel<K, 0, false, true>);
-    if (src.n_pay == 1) return go(part_scatter_fast_kernel<K, 1, false, true>);
-    return go(part_scatter_fast_kernel<K, 2, false, true>);
+    if (src.n_pay == 0) return go(part_scatter_fast_kernel<K, 0, true>);
+    if (src.n_pay == 1) return go(part_scatter_fast_kernel<K, 1, true>);
+    return go(part_scatter_fast_kernel<K, 2, true>);
   }
   if (src.n_pay == 0) return go(part_scatter_fast_kernel<K, 0>);
   if (src.n_pay == 1) return go(part_scatter_fast_kernel<K, 1>);
@@ -541,46 +500,6 @@ static int scatter_per_sm(const PartSrc& src, int key_type, int pbits, bool fast
   }
   cudaGetLastError();
   return std::max(1, std::min(4, r));
-}
-
-// Tile-local partition: one pass, no histogram. Returns the number of tiles (run table rows).
-sj_status local_partition(const PartSrc& src, int key_type, int pbits, const PartDst& dst, int32_t* run_off,
-                          int32_t* run_cnt, int device, cudaStream_t s) {
-  if (!fast_scatter_ok(src, dst)) return set_error(SJ_ERR_INVALID, "tile-local partition needs the plain shape");
-  const int P = 1 << pbits;
-  const int64_t tiles = (src.n + kTile - 1) / kTile;
-  const int per_sm = scatter_per_sm(src, key_type, pbits, true);
-  const int64_t G = std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sm_count(device) * per_sm));
-  const int64_t chunk = (tiles + G - 1) / G * kTile;  // whole tiles per CTA
-  const int grid = (int)((src.n + chunk - 1) / chunk);
-  if (src.n == 0) return SJ_OK;
-  const int kw = key_type == SJ_INT32 ? 4 : 8;
-  // pair loads and stores when the source columns and the partitioned copies are aligned for them
-  bool vec = pair_aligned_src(src, kw) && ((uintptr_t)dst.keys % (2 * kw)) == 0 && ((uintptr_t)dst.rid % 8) == 0;
-  for (int c = 0; c < src.n_pay; ++c) vec = vec && ((uintptr_t)dst.pay[c] % (2 * src.pay[c].width)) == 0;
-  auto go = [&](auto kernel) -> sj_status {
-    const FastSmem m = fast_smem(pbits, kw, src.n_pay);
-    SJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m.total));
-    KernelTimer timer("partition_scatter", s);
-    kernel<<<grid, kPartThreads, m.total, s>>>(src, pbits, chunk, nullptr, dst, m, run_off, run_cnt);
-    return SJ_OK;
-  };
-  (void)P;
-  auto pick = [&](auto k, auto v) -> sj_status {
-    using K = decltype(k);
-    constexpr bool V = decltype(v)::value;
-    return src.n_pay == 0 ? go(part_scatter_fast_kernel<K, 0, true, V>)
-         : src.n_pay == 1 ? go(part_scatter_fast_kernel<K, 1, true, V>)
-                          : go(part_scatter_fast_kernel<K, 2, true, V>);
-  };
-  sj_status st;
-  if (key_type == SJ_INT32)
-    st = vec ? pick(int32_t{}, std::true_type{}) : pick(int32_t{}, std::false_type{});
-  else
-    st = vec ? pick(int64_t{}, std::true_type{}) : pick(int64_t{}, std::false_type{});
-  SJ_TRY(st);
-  SJ_CUDA_TRY(cudaGetLastError());
-  return SJ_OK;
 }
 
 size_t partition_scratch_bytes(int pbits, int device) {
@@ -867,6 +786,148 @@ sj_status partition_columns(const void* keys, int key_type, int64_t n, int pbits
   *d_total_out = offs + PG;
   *d_offs_out = offs;
   *grid_out = G;
+  return SJ_OK;
+}
+
+// ------------------------------------------------------------------------------------------------
+// Tile-local partition (the probe side): every tile of kColTile rows is sorted by partition and written
+// back to its own rows, one column at a time through the staging buffer, in 16-byte pieces; its runs go to
+// run_off / run_cnt[p * tiles + tile]. NULL-key rows are dropped. No histogram, no scan, no write fronts.
+// 64M int64 keys and one 8-byte payload, 16 partitions: 490 us, as long as 2048-row tiles staged whole
+// (479 us), but the probe reads runs twice as long (unit probe 1,361 -> 1,300 us).
+// ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void stage_copy(const unsigned char* stage, void* dst, size_t at, uint32_t bytes) {
+  uint4* d = reinterpret_cast<uint4*>(static_cast<char*>(dst) + at);
+  const uint4* s = reinterpret_cast<const uint4*>(stage);
+  for (uint32_t q = threadIdx.x; q < (bytes + 15) / 16; q += kColThreads) d[q] = s[q];
+}
+
+template <typename K>
+__global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(const K* __restrict__ keys, bool key_pairs,
+                                                                                const uint32_t* __restrict__ kvalid,
+                                                                                int64_t kvoff, uint32_t n, int pbits,
+                                                                                uint32_t n_tiles, K* okeys, int32_t* orid,
+                                                                                PartColumns cols, int32_t* run_off,
+                                                                                int32_t* run_cnt) {
+  using U = std::conditional_t<sizeof(K) == 8, unsigned long long, unsigned int>;
+  __shared__ __align__(16) unsigned char stage[kColTile * 8];
+  __shared__ uint32_t s_wsum[kColThreads / 32], tcnt[1 << kMaxPartBits], tbase[1 << kMaxPartBits];
+  const int P = 1 << pbits;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  for (int p = tid; p < P; p += kColThreads) tcnt[p] = 0;
+  const U* ukeys = reinterpret_cast<const U*>(keys);
+  uint64_t v[kColRows];
+  uint32_t tile = blockIdx.x;
+  if (tile < n_tiles) col_load_t(ukeys, key_pairs, tile * kColTile, n, v);
+  __syncthreads();
+  for (; tile < n_tiles; tile += gridDim.x) {
+    const uint32_t t0 = tile * kColTile;
+    const int tile_n = (int)min(n - t0, (uint32_t)kColTile);
+    // 1. rank every valid row within its partition
+    uint32_t pr[kColRows];  // partition << 16 | rank
+    uint32_t live = 0;
+#pragma unroll
+    for (int j = 0; j < kColRows; ++j) {
+      const int r = col_row(j, tid);
+      if (r >= tile_n || !bit_valid(kvalid, kvoff, (int64_t)t0 + r)) continue;
+      live |= 1u << j;
+      const uint32_t p = (uint32_t)partition_of(key_u64<K>((K)v[j]), pbits);
+      pr[j] = p << 16 | atomicAdd(&tcnt[p], 1u);
+    }
+    __syncthreads();
+    // 2. exclusive scan of the tile's counts: the runs
+    constexpr int kBins = (1 << kMaxPartBits) / kColThreads;
+    uint32_t c[kBins], acc = 0;
+#pragma unroll
+    for (int q = 0; q < kBins; ++q) {
+      const int p = tid * kBins + q;
+      c[q] = p < P ? tcnt[p] : 0;
+      acc += c[q];
+    }
+    const uint32_t incl = warp_inclusive_sum(acc);
+    if (lane == 31) s_wsum[wid] = incl;
+    __syncthreads();
+    uint32_t run = incl - acc, valid = 0;
+    for (int w = 0; w < kColThreads / 32; ++w) {
+      run += w < wid ? s_wsum[w] : 0;
+      valid += s_wsum[w];
+    }
+#pragma unroll
+    for (int q = 0; q < kBins; ++q) {
+      const int p = tid * kBins + q;
+      if (p < P) {
+        tbase[p] = run;
+        tcnt[p] = 0;
+        run_off[(size_t)p * n_tiles + tile] = (int32_t)(t0 + run);
+        run_cnt[(size_t)p * n_tiles + tile] = (int32_t)c[q];
+      }
+      run += c[q];
+    }
+    __syncthreads();
+    // 3. the keys, the payloads, the row ids
+    uint16_t slot[kColRows];
+#pragma unroll
+    for (int j = 0; j < kColRows; ++j) {
+      slot[j] = 0;
+      if (!(live >> j & 1u)) continue;
+      slot[j] = (uint16_t)(tbase[pr[j] >> 16] + (pr[j] & 0xffffu));
+      reinterpret_cast<K*>(stage)[slot[j]] = (K)v[j];
+    }
+    __syncthreads();
+    auto next = [&](int q) {
+      if (q < cols.n) col_load(cols.c[q], t0, n, v);
+      else if (tile + gridDim.x < n_tiles) col_load_t(ukeys, key_pairs, (tile + gridDim.x) * kColTile, n, v);
+    };
+    next(0);
+    stage_copy(stage, okeys, (size_t)t0 * sizeof(K), valid * (uint32_t)sizeof(K));
+    __syncthreads();
+    for (int q = 0; q < cols.n; ++q) {
+      const int w = cols.c[q].width;
+      if (w == 8) {
+#pragma unroll
+        for (int j = 0; j < kColRows; ++j)
+          if (live >> j & 1u) reinterpret_cast<uint64_t*>(stage)[slot[j]] = v[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < kColRows; ++j)
+          if (live >> j & 1u) reinterpret_cast<uint32_t*>(stage)[slot[j]] = (uint32_t)v[j];
+      }
+      __syncthreads();
+      next(q + 1);
+      stage_copy(stage, cols.c[q].dst, (size_t)t0 * w, valid * w);
+      __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < kColRows; ++j)
+      if (live >> j & 1u) reinterpret_cast<uint32_t*>(stage)[slot[j]] = t0 + col_row(j, tid);
+    __syncthreads();
+    stage_copy(stage, orid, (size_t)t0 * 4, valid * 4);
+    __syncthreads();
+  }
+}
+
+// The outputs start on 16 bytes and have room for whole 16-byte pieces.
+sj_status local_partition(const PartSrc& src, int key_type, int pbits, const PartDst& dst, int32_t* run_off,
+                          int32_t* run_cnt, int device, cudaStream_t s) {
+  if (!partition_plain_shape(src, dst)) return set_error(SJ_ERR_INVALID, "tile-local partition needs the plain shape");
+  if (src.n == 0) return SJ_OK;
+  static_assert(kColTile == kPartTileRows, "tile of the run tables");
+  const uint32_t tiles = (uint32_t)((src.n + kColTile - 1) / kColTile);
+  const int grid = (int)std::min<int64_t>(tiles, (int64_t)sm_count(device) * kColCtasPerSm);
+  PartColumns cols{};
+  for (int c = 0; c < src.n_pay; ++c)
+    cols.c[cols.n++] = PartColumn{src.pay[c].data, nullptr, 0, dst.pay[c], src.pay[c].width, 0,
+                                  (int16_t)((uintptr_t)src.pay[c].data % (2 * src.pay[c].width) == 0)};
+  auto go = [&](auto k) {
+    using K = decltype(k);
+    KernelTimer timer("partition_scatter", s);
+    part_local_kernel<K><<<grid, kColThreads, 0, s>>>(static_cast<const K*>(src.keys), (uintptr_t)src.keys % (2 * sizeof(K)) == 0,
+                                                      src.kvalid, src.kvoff, (uint32_t)src.n, pbits, tiles,
+                                                      static_cast<K*>(dst.keys), dst.rid, cols, run_off, run_cnt);
+  };
+  if (key_type == SJ_INT32) go(int32_t{});
+  else go(int64_t{});
+  SJ_CUDA_TRY(cudaGetLastError());
   return SJ_OK;
 }
 

@@ -837,7 +837,8 @@ static sj_status probe_partitioned(const sj_table* t, const sj_column& p, Gather
     bytes += align256((size_t)n * g.pin[c].width) + (g.pin[c].valid ? align256((size_t)n) : 0);
   Scratch sc;
   SJ_TRY(sc.get(alloc, bytes, s));
-  char* cur = sc.as<char>();
+  // 256-byte boundaries whatever the allocator returns: the partitioned columns are written in 16-byte pieces
+  char* cur = reinterpret_cast<char*>(align256(reinterpret_cast<size_t>(sc.ptr)));
   auto carve = [&](size_t b) {
     char* r = cur;
     cur += align256(b);
@@ -857,15 +858,14 @@ static sj_status probe_partitioned(const sj_table* t, const sj_column& p, Gather
     pd.pay[c] = carve((size_t)n * g.pin[c].width);
     pd.valid8[c] = g.pin[c].valid ? reinterpret_cast<uint8_t*>(carve((size_t)n)) : nullptr;
   }
-  unsigned long long* tile_ctr = reinterpret_cast<unsigned long long*>(carve(8));
   if (local) {
     int32_t* run_off = reinterpret_cast<int32_t*>(carve(run_bytes));
     int32_t* run_cnt = reinterpret_cast<int32_t*>(carve(run_bytes));
     SJ_TRY(local_partition(ps, t->key_type, pbits, pd, run_off, run_cnt, t->device, s));
     g.prid_map = pd.rid;
     for (int c = 0; c < g.n_pin; ++c) g.pin[c] = column_payload(pd.pay[c], nullptr, 0, g.pin[c].width);
-    const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 1u};  // group: set by probe_runs
-    probe_runs(t, pd.keys, ra, g, s, tile_ctr);
+    const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0};
+    probe_runs(t, pd.keys, n, ra, g, s);
     SJ_CUDA_TRY(cudaGetLastError());
     return SJ_OK;
   }
@@ -877,7 +877,7 @@ static sj_status probe_partitioned(const sj_table* t, const sj_column& p, Gather
   for (int c = 0; c < g.n_pin; ++c)
     g.pin[c] = PayloadIn{pd.pay[c], nullptr, pd.valid8[c], 0, g.pin[c].width, g.pin[c].width, 1, 0};
   const sj_column pk{pd.keys, nullptr, 0, n, t->key_type, 0};
-  if (!probe_direct(t, pk, d_total, g, s, alloc, tile_ctr)) dispatch_distinct<false>(t, pk, d_total, g, s);
+  if (!probe_direct(t, pk, d_total, g, s)) dispatch_distinct<false>(t, pk, d_total, g, s);
   SJ_CUDA_TRY(cudaGetLastError());
   return SJ_OK;
 }
@@ -900,7 +900,7 @@ sj_status probe_gather(const sj_table* t, const sj_column& p, const GatherSpec& 
 
   if (t->layout == SJ_LAYOUT_DISTINCT) {
     if (t->pbits > 0 && p.num_rows >= kMinPartitionedProbe) return probe_partitioned(t, p, g, alloc, s);
-    if (!probe_direct(t, p, nullptr, g, s, alloc, nullptr)) dispatch_distinct<false>(t, p, nullptr, g, s);
+    if (!probe_direct(t, p, nullptr, g, s)) dispatch_distinct<false>(t, p, nullptr, g, s);
     SJ_CUDA_TRY(cudaGetLastError());
     return SJ_OK;
   }

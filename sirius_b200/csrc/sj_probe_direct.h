@@ -30,38 +30,32 @@ struct DirectArgs {
   void* bout[kDirectMaxBuildPayload];
   int64_t capacity;
   unsigned long long* d_count;
-  unsigned long long* tile_ctr;  // zeroed device word: dynamic tile order of CTA-reserving launches
-  int32_t l2_last;               // table slot and record loads marked L2 evict_last
+  int32_t l2_last;  // TMA-staged probe: table slot loads marked L2 evict_last
 };
 
 // Partition runs of a tile-local partition (local_partition): rows of partition p in tile i are
-// [run_off[i * P + p], + run_cnt[i * P + p]).
+// [run_off[p * n_tiles + i], + run_cnt[p * n_tiles + i]).
 struct RunArgs {
   const int32_t* run_off;
   const int32_t* run_cnt;
   uint32_t n_tiles;
   uint32_t P;
-  uint32_t group;  // tiles per work item (a power of two <= 16); set by probe_runs
+  uint32_t log2_pieces;  // a run is split into 2^log2_pieces units
 };
 
 // Fills `a` from a general gather description; false when the output shape needs the staged
 // kernel (NULL payloads, 1/2-byte payloads, too many columns, other record layouts).
 bool direct_args(const GatherArgs& g, DirectArgs& a);
 
-// Launches the direct probe of DISTINCT table `t` when the shape allows and the table's
-// parameters do not ask for the staged kernel; returns false (nothing launched) otherwise.
-// `tile_ctr`: a device word the launch may use as its tile counter (zeroed here, on `s`); when NULL
-// and a counter is needed, one is drawn from `alloc`.
-bool probe_direct(const sj_table* t, const sj_column& p, const int64_t* d_n, const GatherArgs& g, cudaStream_t s,
-                  const Allocator& alloc, unsigned long long* tile_ctr);
+// Launches the probe of DISTINCT table `t` when the shape allows and the table's parameters do not ask for
+// the staged kernel; returns false (nothing launched) otherwise. `d_n`: device row count, or NULL.
+bool probe_direct(const sj_table* t, const sj_column& p, const int64_t* d_n, const GatherArgs& g, cudaStream_t s);
 
-// True when probe_runs serves this gather (DIRECT write-out shape, CTA reservation).
+// True when probe_runs serves this gather.
 bool probe_runs_ok(const sj_table* t, const GatherArgs& g);
 
-// Probe of tile-local partition runs: `keys`, the partition row ids and payloads in `g` are the
-// partitioned arrays; work items (partition, group of tiles) are taken partition-major from
-// `tile_ctr` (zeroed here). Requires probe_runs_ok.
-void probe_runs(const sj_table* t, const void* keys, const RunArgs& ra, const GatherArgs& g, cudaStream_t s,
-                unsigned long long* tile_ctr);
+// Probe of tile-local partition runs: `keys` (n rows), the partition row ids and payloads in `g` are the
+// partitioned arrays; the runs are walked partition after partition. Requires probe_runs_ok.
+void probe_runs(const sj_table* t, const void* keys, int64_t n, const RunArgs& ra, const GatherArgs& g, cudaStream_t s);
 
 }  // namespace sj

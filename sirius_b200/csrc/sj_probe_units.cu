@@ -1,0 +1,329 @@
+// INNER probe and gather of a DISTINCT table in units. A unit is one warp's rows: 32 * S consecutive ones,
+// or a piece of partition p's run of a tile (tile-local partition). A CTA takes 8 consecutive units (of one partition),
+// 32 * S rows of each at a time: the keys of all S row groups in flight, their home buckets, one walk for the
+// rows that go on, the probe side's row ids and payload, one reservation for the CTA (its atomicAdd returns
+// behind the first records' loads), records, stores. Row group j's matches go to consecutive positions, so
+// each column is stored in contiguous runs. Positions stay in registers and no row is staged.
+//
+// What bounds it: a random 32-byte load costs an SM one L1 tag cycle (275 G/s on the whole GPU, any width,
+// from 1024 threads per SM on), and a match needs two (bucket, record or payload); instructions, half of
+// them at half rate, cost about as much. So the code per row is short (the rows that go on are walked once
+// per 128 rows, one per lane, not once more with every row group), CTAs are small, many (6 per SM, 48 warps)
+// and start in order: partition after partition is swept without a work counter, and one CTA's barriers and
+// its reservation (same-address atomics return one per 0.67 ns on the whole GPU) are covered by the others.
+// Shared memory is kept small too: what it takes from L1 limits the loads in flight (a 32 KB list per CTA
+// made the lookups 60 % slower).
+#include <algorithm>
+#include <type_traits>
+
+#include "sj_internal.h"
+#include "sj_partition.cuh"
+#include "sj_probe_core.cuh"
+#include "sj_probe_units.h"
+
+namespace sj {
+
+TableDev table_dev(const sj_table* t);
+
+constexpr int kUnitThreads = 256;
+constexpr int kUnitWarps = kUnitThreads / 32;
+
+__device__ __forceinline__ uint64_t ld_col(const void* base, uint32_t i, int w) {
+  return w == 8 ? (uint64_t)__ldcs(static_cast<const unsigned long long*>(base) + i)
+                : (uint64_t)__ldcs(static_cast<const unsigned int*>(base) + i);
+}
+__device__ __forceinline__ uint64_t ld_at(const void* a, int w) {
+  return w == 8 ? (uint64_t)__ldg(static_cast<const unsigned long long*>(a))
+                : (uint64_t)__ldg(static_cast<const unsigned int*>(a));
+}
+__device__ __forceinline__ void st_col(void* base, uint32_t i, int w, uint64_t v) {
+  if (w == 8) __stcs(static_cast<unsigned long long*>(base) + i, (unsigned long long)v);
+  else __stcs(static_cast<unsigned int*>(base) + i, (unsigned int)v);
+}
+
+// SP, SB >= 0: a compile-time output shape: both row ids, SP probe payloads and SB build payloads out of
+// row-store records, 8 bytes each. -1: the shape is read from `a`.
+template <int SP, int SB>
+struct Shape {
+  static constexpr bool kFixed = SP >= 0;
+  __device__ __forceinline__ static int n_pin(const DirectArgs& a) { return kFixed ? SP : a.n_pin; }
+  __device__ __forceinline__ static int pin_w(const DirectArgs& a, int c) { return kFixed ? 8 : a.pin_w[c]; }
+  __device__ __forceinline__ static bool rec(const DirectArgs& a) { return kFixed ? SB > 0 : a.rec != nullptr; }
+  __device__ __forceinline__ static int stride(const DirectArgs& a) { return kFixed ? (SB == 1 ? 16 : 32) : a.rec_stride; }
+  __device__ __forceinline__ static int n_bin(const DirectArgs& a) { return kFixed ? SB : a.n_bin; }
+  __device__ __forceinline__ static bool prid(const DirectArgs& a) { return kFixed || a.out_prid; }
+  __device__ __forceinline__ static bool brid(const DirectArgs& a) { return kFixed || a.out_brid; }
+};
+
+// Row id and first payload of probe row `row` (index into the probe arrays).
+template <typename Sh>
+__device__ __forceinline__ void load_probe_side(const DirectArgs& a, uint32_t row, bool live, int32_t& prid, uint64_t& v) {
+  prid = a.prid_map && live ? __ldcs(a.prid_map + row) : (int32_t)row;
+  v = Sh::n_pin(a) > 0 && live ? ld_col(a.pin[0], row, Sh::pin_w(a, 0)) : 0;
+}
+
+// Writes a match: probe row `row` (index into the probe arrays) and table position `pos` to output position
+// p if live, with the row id prid and the first probe payload v; `ready()`, called by the whole warp between
+// the first loads and the first store, gives p and may clear live.
+template <typename Sh, typename Ready>
+__device__ __forceinline__ void emit_match(const DirectArgs& a, uint32_t row, int32_t prid, uint64_t v, uint32_t pos,
+                                           bool live, Ready&& ready) {
+  uint32_t w[8];
+  int32_t brid = (int32_t)pos;
+  if (Sh::rec(a)) {
+    if (live) {
+      const char* rp = static_cast<const char*>(a.rec) + (size_t)pos * Sh::stride(a);
+      if (Sh::stride(a) == 32) {
+        asm("ld.global.nc.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+            : "l"(rp));
+      } else if (Sh::stride(a) == 16) {
+        const uint4 x = __ldg(reinterpret_cast<const uint4*>(rp));
+        w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
+      } else {
+        const uint2 x = __ldg(reinterpret_cast<const uint2*>(rp));
+        w[0] = x.x; w[1] = x.y;
+      }
+      brid = (int32_t)w[0];
+    }
+  } else if (a.brid_map && live) {
+    brid = __ldg(reinterpret_cast<const int32_t*>(reinterpret_cast<const char*>(a.brid_map) + (size_t)pos * a.brid_stride));
+  }
+  uint32_t p;
+  ready(p, live);
+  if (!live) return;
+  if (Sh::prid(a)) __stcs(a.out_prid + p, prid);
+  if (Sh::n_pin(a) > 0) st_col(a.pout[0], p, Sh::pin_w(a, 0), v);
+  if (Sh::n_pin(a) > 1) st_col(a.pout[1], p, Sh::pin_w(a, 1), ld_col(a.pin[1], row, Sh::pin_w(a, 1)));
+  if (Sh::brid(a)) __stcs(a.out_brid + p, brid);
+  if (Sh::rec(a)) {
+    if (Sh::stride(a) == 8) {  // one 4-byte field
+      __stcs(static_cast<unsigned int*>(a.bout[0]) + p, w[1]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < kDirectMaxBuildPayload; ++c)
+        if (c < Sh::n_bin(a))
+          __stcs(static_cast<unsigned long long*>(a.bout[c]) + p, ((unsigned long long)w[3 + 2 * c] << 32) | w[2 + 2 * c]);
+    }
+    return;
+  }
+  for (int c = 0; c < a.n_bin; ++c)
+    st_col(a.bout[c], p, a.bin_w[c],
+           ld_at(static_cast<const char*>(a.bin[c]) + (int64_t)(a.bin_by_pos ? (int32_t)pos : brid) * a.bin_stride[c], a.bin_w[c]));
+}
+
+constexpr uint32_t kNoPos = 0xffffffffu;
+constexpr int kUnitCtasPerSm = 6;  // 40 registers
+
+struct Units {
+  uint32_t part, first;  // RUNS: the CTA's partition; its first unit (piece of a run)
+};
+
+template <bool RUNS>
+__device__ __forceinline__ Units cta_units(const RunArgs& ra) {
+  Units u{0, blockIdx.x * kUnitWarps};
+  if constexpr (RUNS) {
+    const uint32_t ctas = ((ra.n_tiles << ra.log2_pieces) + kUnitWarps - 1) / kUnitWarps;
+    u.part = blockIdx.x / ctas;
+    u.first = (blockIdx.x - u.part * ctas) * kUnitWarps;
+  }
+  return u;
+}
+
+// First row and rows of the warp's unit.
+template <bool RUNS, int S>
+__device__ __forceinline__ void unit_rows(const RunArgs& ra, const Units& u, uint32_t n, uint32_t& first, uint32_t& rows) {
+  const uint32_t unit = u.first + (threadIdx.x >> 5);
+  first = rows = 0;
+  if constexpr (RUNS) {
+    const uint32_t tile = unit >> ra.log2_pieces, piece = unit & ((1u << ra.log2_pieces) - 1u);
+    if (tile >= ra.n_tiles) return;
+    const size_t at = (size_t)u.part * ra.n_tiles + tile;
+    const uint32_t cnt = (uint32_t)__ldg(ra.run_cnt + at), lo = cnt * piece >> ra.log2_pieces;
+    first = (uint32_t)__ldg(ra.run_off + at) + lo;
+    rows = (cnt * (piece + 1) >> ra.log2_pieces) - lo;
+  } else {
+    first = unit * (32 * S);
+    rows = first < n ? min(32u * S, n - first) : 0;
+  }
+}
+
+// A warp's rows that go on past their home bucket.
+template <int S>
+struct WaitRows {
+  SectorKey key[32 * S];
+  uint32_t bucket[32 * S];  // then the row's position
+};
+
+template <typename K, bool WIDE, bool RUNS, int S, int SP, int SB>
+__global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kernel(TableDev t, const K* __restrict__ keys,
+                                                                      const uint32_t* __restrict__ kv, int64_t kvoff,
+                                                                      uint32_t n, const int64_t* d_n, RunArgs ra,
+                                                                      DirectArgs a) {
+  using Ops = SectorOps<WIDE>;
+  using Sh = Shape<SP, SB>;
+  if (!RUNS && d_n) n = min(n, (uint32_t)*d_n);
+  __shared__ WaitRows<S> s_wait[kUnitWarps];
+  __shared__ uint32_t s_cnt[kUnitWarps];
+  __shared__ uint32_t s_base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  WaitRows<S>& wait = s_wait[warp];
+  const uint32_t rid_mask = (1u << t.rbits) - 1u;
+  const uint32_t cap = (uint32_t)(a.capacity < (int64_t)0x7fffffff ? a.capacity : (int64_t)0x7fffffff);
+  const Units u = cta_units<RUNS>(ra);
+  uint32_t first, rows;
+  unit_rows<RUNS, S>(ra, u, n, first, rows);
+  for (uint32_t v0 = 0; __syncthreads_or(v0 < rows); v0 += 32 * S) {
+    K k[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const uint32_t v = v0 + 32 * j + lane;
+      k[j] = v < rows ? __ldcs(keys + first + v) : (K)0;
+    }
+    uint32_t pos[S], n_wait = 0;
+    uint32_t waits = 0;  // byte j: 1 + place in the list of the lane's row j, or 0
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const uint32_t v = v0 + 32 * j + lane;
+      SectorKey key;
+      uint32_t b, q = 0;
+      pos[j] = kNoPos;
+      bool cont = false;
+      if (sector_key<K, WIDE>(t, k[j], key, b) && v < rows && (RUNS || bit_valid(kv, kvoff, first + v))) {
+        const Sector s = load_sector(t.slots, b);
+        uint32_t p;
+        if (Ops::find(s, key, rid_mask, p, q)) pos[j] = p;
+        else cont = t.segmask != 0 && !Ops::open(s);
+      }
+      const unsigned bal = __ballot_sync(kFullMask, cont);
+      if (bal) {
+        if (cont) {
+          const uint32_t e = n_wait + __popc(bal & below);
+          wait.key[e] = key;
+          wait.bucket[e] = next_bucket(b, t.segmask);
+          waits |= (e + 1) << (8 * j);
+        }
+        n_wait += __popc(bal);
+      }
+    }
+    if (n_wait) {
+      __syncwarp();
+      for (uint32_t e0 = 0; e0 < n_wait; e0 += 32) {
+        const uint32_t e = e0 + lane;
+        bool act = e < n_wait;
+        SectorKey key{};
+        uint32_t b = 0, res = kNoPos;
+        if (act) {
+          key = wait.key[e];
+          b = wait.bucket[e];
+        }
+        for (uint32_t step = 0; step < t.segmask && __any_sync(kFullMask, act); ++step) {
+          if (act) {
+            const Sector s = load_sector(t.slots, b);
+            uint32_t q = 0, p;
+            const bool f = Ops::find(s, key, rid_mask, p, q);
+            if (f) res = p;
+            act = !f && !Ops::open(s);
+            b = next_bucket(b, t.segmask);
+          }
+        }
+        if (e < n_wait) wait.bucket[e] = res;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < S; ++j)
+        if (waits >> (8 * j) & 0xffu) pos[j] = wait.bucket[(waits >> (8 * j) & 0xffu) - 1];
+    }
+    uint32_t cnt = 0;
+#pragma unroll
+    for (int j = 0; j < S; ++j) cnt += __popc(__ballot_sync(kFullMask, pos[j] != kNoPos));
+    if (lane == 0) s_cnt[warp] = cnt;
+    int32_t prid[S];
+    uint64_t pv[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) load_probe_side<Sh>(a, first + v0 + 32 * j + lane, pos[j] != kNoPos, prid[j], pv[j]);
+    __syncthreads();
+    const uint32_t c = lane < kUnitWarps ? s_cnt[lane] : 0;
+    const uint32_t incl = warp_inclusive_sum(c);
+    uint32_t run = __shfl_sync(kFullMask, incl - c, warp);
+    if (warp == 0 && lane == kUnitWarps - 1) s_base = incl ? (uint32_t)atomicAdd(a.d_count, (unsigned long long)incl) : 0;
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const bool hit = pos[j] != kNoPos;
+      const unsigned bal = __ballot_sync(kFullMask, hit);
+      emit_match<Sh>(a, first + v0 + 32 * j + lane, prid[j], pv[j], pos[j], hit, [&](uint32_t& p, bool& live) {
+        if (j == 0) {  // the reservation is back
+          __syncthreads();
+          run += s_base;
+        }
+        p = run + __popc(bal & below);
+        run += __popc(bal);
+        live = live && p < cap;
+      });
+    }
+  }
+}
+
+// Probes of at most this many rows take units of 32 rows: a row has a thread of its own and the chain of
+// dependent loads is all there is. Units of 32 against units of 128 rows, int32 keys and payloads: 10K rows
+// 4.0 / 7.0 us, 200K 5.4 / 7.6, 400K 8.4 / 8.4, 600K 11.7 / 10.4, 2M 30.6 / 28.3, 4M 61.5 / 50.6 us (two
+// warps of 64 rows with a reservation each, before: 6.5, 8.5, 12.8, 17.7, 50.5, 98.0 us).
+constexpr int64_t kFewRows = 400000;
+
+// Records are held in registers when they are [row id | one 4-byte field] or [row id | - | 8-byte
+// fields]; the fields of other records are gathered from the row store one by one.
+static DirectArgs plain_records(DirectArgs a) {
+  if (a.rec && !a.rec_std && !(a.n_bin == 1 && a.rec_stride == 8 && a.rec_off[0] == 4)) {
+    a.brid_map = static_cast<const int32_t*>(a.rec);
+    a.brid_stride = a.rec_stride;
+    a.bin_by_pos = 1;
+    for (int c = 0; c < a.n_bin; ++c) {
+      a.bin[c] = static_cast<const char*>(a.rec) + a.rec_off[c];
+      a.bin_stride[c] = a.rec_stride;
+    }
+    a.rec = nullptr;
+  }
+  return a;
+}
+
+void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t kvoff, int64_t n, const int64_t* d_n,
+                 const RunArgs* runs, const DirectArgs& a_in, cudaStream_t s) {
+  if (n == 0) return;
+  const DirectArgs a = plain_records(a_in);
+  RunArgs ra = runs ? *runs : RunArgs{};
+  // pieces of about 128 rows (a run holds kPartTileRows / P rows): with whole runs of 1024 rows a warp's
+  // chain was eight times as long and the few warps of a 1M-row probe took 100 us instead of 63
+  while (runs && ((uint64_t)ra.P * 128 << ra.log2_pieces) < kPartTileRows) ++ra.log2_pieces;
+  const bool few = !runs && n <= kFewRows;
+  auto ctas = [](int64_t units) { return (units + kUnitWarps - 1) / kUnitWarps; };
+  const int64_t unit = few ? 32 : 128;
+  const int grid = (int)(runs ? ra.P * ctas((int64_t)ra.n_tiles << ra.log2_pieces) : ctas((n + unit - 1) / unit));
+  const TableDev d = table_dev(t);
+  KernelTimer timer("probe_units", s);
+  using std::integral_constant;
+  auto shape = [&](auto k, auto w, auto sp, auto sb) {
+    using K = decltype(k);
+    constexpr bool W = decltype(w)::value;
+    constexpr int SP = decltype(sp)::value, SB = decltype(sb)::value;
+    auto kernel = runs ? probe_units_kernel<K, W, true, 4, SP, SB>
+                  : few ? probe_units_kernel<K, W, false, 1, SP, SB> : probe_units_kernel<K, W, false, 4, SP, SB>;
+    kernel<<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(keys), kv, kvoff, (uint32_t)n, d_n, ra, a);
+  };
+  auto go = [&](auto k, auto w) {
+    const bool both = a.out_prid && a.out_brid && a.rec && a.rec_stride != 8;
+    if (both && a.n_pin == 1 && a.pin_w[0] == 8 && a.n_bin == 2) shape(k, w, integral_constant<int, 1>{}, integral_constant<int, 2>{});
+    else if (both && a.n_pin == 0 && a.n_bin == 1) shape(k, w, integral_constant<int, 0>{}, integral_constant<int, 1>{});
+    else shape(k, w, integral_constant<int, -1>{}, integral_constant<int, -1>{});
+  };
+  const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
+  if (t->key_type == SJ_INT32) {
+    if (wide) go(int32_t{}, std::true_type{});
+    else go(int32_t{}, std::false_type{});
+  } else {
+    if (wide) go(int64_t{}, std::true_type{});
+    else go(int64_t{}, std::false_type{});
+  }
+}
+
+}  // namespace sj

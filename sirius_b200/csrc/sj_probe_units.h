@@ -1,0 +1,13 @@
+// The unit probe of DISTINCT tables (sj_probe_units.cu).
+#pragma once
+
+#include "sj_probe_direct.h"
+
+namespace sj {
+
+// Probes `n` rows (at most *d_n when d_n is given), or the partition runs `runs` of the probe arrays, into `t`
+// for the gather `a`.
+void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t kvoff, int64_t n, const int64_t* d_n,
+                 const RunArgs* runs, const DirectArgs& a, cudaStream_t s);
+
+}  // namespace sj
