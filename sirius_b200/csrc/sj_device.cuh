@@ -388,6 +388,7 @@ struct GatherArgs {
   int32_t rec_stride;
   int16_t rec_off[kMaxPayload];   // byte offset of attached column c inside a record
   int16_t rec_voff[kMaxPayload];  // byte offset of its validity byte, -1 when it has no NULLs
+  uint32_t* matched;  // bit of every probe row with a match, set by the unit probe; or NULL
 };
 
 __device__ __forceinline__ uint64_t load_elem(const void* base, int64_t i, int w) {

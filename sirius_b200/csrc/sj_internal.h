@@ -183,12 +183,18 @@ struct GatherSpec {
   const sj_mut_column* out_probe_payload;
   const sj_mut_column* out_build_payload;
   int64_t capacity;
+  // LEFT / FULL: (probe rows + 31) / 32 zeroed words. Set to true when the probe sets bit i for every probe
+  // row i with a match; left alone when it does not.
+  uint32_t* matched = nullptr;
+  bool* matched_set = nullptr;
 };
 
 sj_status probe_count(const sj_table* t, const sj_column& probe, const Allocator& alloc,
                       cudaStream_t stream, int64_t* d_count);
 sj_status probe_gather(const sj_table* t, const sj_column& probe, const GatherSpec& g,
                        const Allocator& alloc, cudaStream_t stream, int64_t* d_count);
+
+sj_status probe_find(const sj_table* t, const sj_column& p, uint32_t* words, const Allocator& alloc, cudaStream_t s);
 
 sj_status validate_column(const sj_column* c, const char* what, bool key);
 

@@ -26,6 +26,7 @@
 #include "sj_internal.h"
 #include "sj_partition.cuh"
 #include "sj_probe_direct.h"
+#include "sj_probe_units.h"
 #include "sj_scan.cuh"
 
 namespace sj {
@@ -818,17 +819,22 @@ static int probe_partition_bits(const sj_table* t) {
   return std::min(b, t->pbits);
 }
 
+// Tile-local partition (one pass, no histogram) + the probe of its runs, when the unit probe serves the
+// output shape and the probe payloads are plain 4/8-byte columns without NULLs.
+static bool partition_is_local(const sj_table* t, const GatherArgs& g) {
+  bool local = probe_runs_ok(t, g) && g.n_pin <= 2;
+  for (int c = 0; c < g.n_pin; ++c)
+    local = local && !g.pin[c].valid && !g.pin[c].valid8 && (g.pin[c].width == 4 || g.pin[c].width == 8) &&
+            g.pin[c].stride == g.pin[c].width;
+  return local;
+}
+
 static sj_status probe_partitioned(const sj_table* t, const sj_column& p, GatherArgs g, const Allocator& alloc,
                                    cudaStream_t s) {
   const int64_t n = p.num_rows;
   const int pbits = probe_partition_bits(t);
   const int kw = t->key_type == SJ_INT32 ? 4 : 8;
-  // Tile-local partition (one pass, no histogram) + the run-walking probe, when the direct probe
-  // serves the output shape and the probe payloads are plain 4/8-byte columns without NULLs.
-  bool local = probe_runs_ok(t, g) && g.n_pin <= 2;
-  for (int c = 0; c < g.n_pin; ++c)
-    local = local && !g.pin[c].valid && !g.pin[c].valid8 && (g.pin[c].width == 4 || g.pin[c].width == 8) &&
-            g.pin[c].stride == g.pin[c].width;
+  const bool local = partition_is_local(t, g);
   const int64_t n_tiles = (n + kPartTileRows - 1) / kPartTileRows;
   const size_t run_bytes = (size_t)n_tiles * ((size_t)1 << pbits) * sizeof(int32_t);
   size_t bytes = align256((size_t)n * kw) + align256((size_t)n * 4) + 256 +
@@ -882,7 +888,47 @@ static sj_status probe_partitioned(const sj_table* t, const sj_column& p, Gather
   return SJ_OK;
 }
 
-// Probes of at least this many rows into a partitioned table take the partitioned path.
+// Which probe rows have a match, as one bit per row (SEMI, ANTI, MARK). A table whose slots outgrow L2 is
+// looked up in partition order when the probe touches each of its sectors twice or more: 64M probe rows into
+// 256 MB of slots in place 1,325 us (random DRAM sectors, 55 G/s); below that the partition pass costs more
+// than the random sectors. No scratch for it: looked up in place.
+sj_status probe_find(const sj_table* t, const sj_column& p, uint32_t* words, const Allocator& alloc, cudaStream_t s) {
+  SJ_TRY(check_probe(t, p));
+  const int64_t n = p.num_rows;
+  constexpr size_t kFitsL2 = (size_t)64 << 20;
+  if (t->pbits > 0 && t->slots_bytes > kFitsL2 && (size_t)n * kBucketBytes >= 2 * t->slots_bytes) {
+    int pbits = 1;
+    const size_t share = (size_t)(t->params.probe_partition_mb > 0 ? t->params.probe_partition_mb : 48) << 20;
+    while (pbits < t->pbits && (t->slots_bytes >> pbits) > share) ++pbits;
+    const int kw = t->key_type == SJ_INT32 ? 4 : 8;
+    const int64_t n_tiles = (n + kPartTileRows - 1) / kPartTileRows;
+    const size_t run_bytes = (size_t)n_tiles * ((size_t)1 << pbits) * sizeof(int32_t);
+    Scratch sc;
+    if (sc.get(alloc, align256((size_t)n * kw) + align256((size_t)n * 4) + 2 * align256(run_bytes) + 256, s) == SJ_OK) {
+      char* cur = reinterpret_cast<char*>(align256(reinterpret_cast<size_t>(sc.ptr)));
+      PartSrc ps{};
+      PartDst pd{};
+      ps.keys = p.data;
+      ps.kvalid = p.validity;
+      ps.kvoff = p.validity_offset;
+      ps.n = n;
+      pd.keys = cur;
+      pd.rid = reinterpret_cast<int32_t*>(cur + align256((size_t)n * kw));
+      int32_t* run_off = reinterpret_cast<int32_t*>(cur + align256((size_t)n * kw) + align256((size_t)n * 4));
+      int32_t* run_cnt = run_off + align256(run_bytes) / sizeof(int32_t);
+      SJ_TRY(local_partition(ps, t->key_type, pbits, pd, run_off, run_cnt, t->device, s));
+      SJ_CUDA_TRY(cudaMemsetAsync(words, 0, (size_t)((n + 31) / 32) * sizeof(uint32_t), s));
+      const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0};
+      find_units(t, pd.keys, nullptr, 0, n, &ra, pd.rid, words, s);
+      SJ_CUDA_TRY(cudaGetLastError());
+      return SJ_OK;
+    }
+    clear_error();
+  }
+  find_units(t, p.data, p.validity, p.validity_offset, n, nullptr, nullptr, words, s);
+  SJ_CUDA_TRY(cudaGetLastError());
+  return SJ_OK;
+}
 
 sj_status probe_gather(const sj_table* t, const sj_column& p, const GatherSpec& gs, const Allocator& alloc,
                        cudaStream_t s, int64_t* d_count) {
@@ -899,6 +945,14 @@ sj_status probe_gather(const sj_table* t, const sj_column& p, const GatherSpec& 
   if (p.num_rows == 0) return SJ_OK;
 
   if (t->layout == SJ_LAYOUT_DISTINCT) {
+    // the unit probe sets the matched bits: wherever it serves the gather and, when partitioned, walks runs
+    if (gs.matched && t->params.probe_kernel != SJ_PROBE_KERNEL_DIRECT_TMA && probe_runs_ok(t, g)) {
+      const bool split = t->pbits > 0 && p.num_rows >= kMinPartitionedProbe;
+      if (!split || partition_is_local(t, g)) {
+        g.matched = gs.matched;
+        *gs.matched_set = true;
+      }
+    }
     if (t->pbits > 0 && p.num_rows >= kMinPartitionedProbe) return probe_partitioned(t, p, g, alloc, s);
     if (!probe_direct(t, p, nullptr, g, s)) dispatch_distinct<false>(t, p, nullptr, g, s);
     SJ_CUDA_TRY(cudaGetLastError());

@@ -289,6 +289,7 @@ bool direct_args(const GatherArgs& g, DirectArgs& a) {
   a.prid_map = g.prid_map;
   a.capacity = g.capacity;
   a.d_count = g.d_count;
+  a.matched = g.matched;
   a.n_pin = g.n_pin;
   a.n_bin = g.n_bin;
   for (int c = 0; c < g.n_pin; ++c) {
@@ -353,7 +354,7 @@ bool probe_direct(const sj_table* t, const sj_column& p, const int64_t* d_n, con
   a.l2_last = pr.table_l2_priority == SJ_L2_EVICT_LAST;
   // AUTO takes plain loads: on the large 1:1 join the TMA ring's per-tile CTA barriers cost more than
   // the DRAM latency it hides (measured 1.96 vs 1.73 ms per 64M probe rows)
-  bool tma = pr.probe_kernel == SJ_PROBE_KERNEL_DIRECT_TMA && (!a.rec || a.rec_std);
+  bool tma = pr.probe_kernel == SJ_PROBE_KERNEL_DIRECT_TMA && (!a.rec || a.rec_std) && !a.matched;
   tma = tma && al16(p.data) && (!a.prid_map || al16(a.prid_map));
   for (int c = 0; c < a.n_pin; ++c) tma = tma && al16(a.pin[c]);
   if (tma) {

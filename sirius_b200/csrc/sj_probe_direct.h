@@ -30,6 +30,7 @@ struct DirectArgs {
   void* bout[kDirectMaxBuildPayload];
   int64_t capacity;
   unsigned long long* d_count;
+  uint32_t* matched;  // unit probe: bit of every probe row with a match (zero before if partitioned), or NULL
   int32_t l2_last;  // TMA-staged probe: table slot loads marked L2 evict_last
 };
 

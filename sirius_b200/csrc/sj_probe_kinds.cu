@@ -3,21 +3,21 @@
 // anti_join, hash_join::left_join / full_join, distinct_hash_join::left_join — and the MARK result of
 // resolve_mark_join_result, :1461-1525).
 //
-//   SEMI / ANTI  one pass: every probe row looks its key up (a NULL key finds nothing unless NULLs
-//                compare equal and the build has NULL keys) and the selected rows are compacted with
-//                their probe payloads. A warp stages the selected row ids in shared memory and
-//                reserves output once per flush of about 224 rows, then writes rows and payloads in
-//                contiguous runs: one atomicAdd per 32-row step on the one output counter serialised
-//                the pass (64M rows, 30 % absent: ANTI 2.60 ms, MARK — the same lookups without
-//                compaction — 0.85 ms).
-//   MARK         one pass, no compaction: mark byte and validity bit of every probe row. Unmatched
-//                rows are NULL when their key is NULL, or all of them when the build has a NULL key.
+//   SEMI / ANTI  two passes: the lookup (probe_find: a NULL key finds nothing unless NULLs compare equal
+//                and the build has NULL keys; in partition order where the table outgrows L2) leaves one
+//                bit per probe row, then the selected rows and their payloads are compacted in row order
+//                (64M x 16M rows, 30 % absent: SEMI 1,325 -> 1,115 us).
+//   MARK         the same bits, then mark byte and validity bit of every probe row. Unmatched rows are
+//                NULL when their key is NULL, or all of them when the build has a NULL key.
+//                When the allocator refuses the bits, all three run as one pass over the table in place,
+//                which needs no scratch: a warp stages the selected row ids in shared memory and reserves
+//                output once per flush of about 224 rows.
 //   LEFT         the INNER probe + gather (probe_gather, any table layout), then the unmatched probe
 //                rows appended after the INNER rows on the same counter with build row id
-//                SJ_NO_ROW: the rows whose bit is clear in a mask set from the INNER rows' probe row
-//                ids (or, when no probe row ids are written or the INNER rows overflowed the
-//                capacity, the ANTI lookup); validity of the NULL-padded build payloads is set by
-//                range.
+//                SJ_NO_ROW: the rows whose bit is clear in a mask that the unit probe sets as it looks
+//                the rows up, or that is set from the INNER rows' probe row ids (or, when those are not
+//                written or overflowed the capacity, the ANTI lookup); validity of the NULL-padded build
+//                payloads is set by range.
 //   FULL         LEFT, then the unmatched build rows: the build rows whose bit is clear in a mask
 //                set from the INNER rows' build row ids (NULL-key rows included). When no build row
 //                ids are written or the INNER rows overflowed the capacity: a pass that flags every
@@ -51,9 +51,9 @@ struct KindArgs {
   uint32_t* mark_valid;
   int32_t build_has_null;
   uint8_t* flags;  // kFlags: one byte per slot (+ the NULL group)
-  const uint32_t* matched;  // kUnmatched: bit i set when probe row i has an INNER row
-  const unsigned long long* inner_rows;  // kUnmatched: INNER rows; past `capacity` the bits are
-                                         // incomplete and the rows are looked up instead
+  const unsigned long long* inner_rows;  // kUnmatched, kFlags, select_rows: INNER rows that the match bits
+                                         // were set from; past `capacity` the bits are incomplete and the
+                                         // rows are looked up instead. NULL: the bits are complete
 };
 
 // Slot of key k in the table (k in range), or -1. Slots fill each bucket in order, so the walk stops
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kKindThreads) kind_probe_kernel(TableDev t, co
   __shared__ int32_t s_stage[kKindThreads / 32][kKindStage];
   int32_t* st = s_stage[threadIdx.x >> 5];
   uint32_t fill = 0;  // staged rows of this warp (warp-uniform)
-  const bool by_bits = MODE == kUnmatched && (int64_t)*a.inner_rows <= a.capacity;
+  if (MODE == kUnmatched && (int64_t)*a.inner_rows <= a.capacity) return;  // emitted by their bits
   // FULL flags pass: not needed when the build-row bits of the INNER rows are complete
   if (MODE == kFlags && a.inner_rows && (int64_t)*a.inner_rows <= a.capacity) return;
   // reserve the staged rows' output range with one atomicAdd and write them out in order
@@ -129,13 +129,8 @@ __global__ void __launch_bounds__(kKindThreads) kind_probe_kernel(TableDev t, co
     const int64_t i = i0 + lane;
     const bool live = i < n;
     int64_t s = -1;
-    const bool valid = live && (by_bits || bit_valid(kv, kvoff, i));
-    if (by_bits) {
-      // no lookup: the INNER rows already told which probe rows matched
-      if (live && (__ldg(a.matched + (i >> 5)) >> (i & 31) & 1u)) s = 0;
-    } else {
-      s = live ? lookup<K, WIDE>(t, __ldg(keys + i), valid) : -1;
-    }
+    const bool valid = live && bit_valid(kv, kvoff, i);
+    if (live) s = lookup<K, WIDE>(t, __ldg(keys + i), valid);
     const bool found = s >= 0;
     if (MODE == kMark) {
       if (live) a.mark[i] = found ? 1 : 0;
@@ -158,6 +153,108 @@ __global__ void __launch_bounds__(kKindThreads) kind_probe_kernel(TableDev t, co
   }
   if (MODE == kSemi || MODE == kAnti || MODE == kUnmatched)
     if (fill) flush();
+}
+
+// Emits the probe rows whose bit in `words` is set (WANT) or clear, with their probe payloads. A warp takes 1024
+// rows, one word per lane; a CTA reserves once for its 8192 rows, and the words' rows go to consecutive
+// positions, so rows, payload loads and stores stay in order. 64M rows, 70 % of them with an 8-byte payload:
+// 213 us (5.0 TB/s), 254 with one word at a time.
+constexpr int kSelectWarps = kKindThreads / 32;
+
+template <bool WANT>
+__global__ void __launch_bounds__(kKindThreads) select_rows_kernel(const uint32_t* __restrict__ words, uint32_t n, KindArgs a) {
+  if (a.inner_rows && (int64_t)*a.inner_rows > a.capacity) return;  // the bits are incomplete
+  __shared__ uint32_t s_cnt[kSelectWarps];
+  __shared__ unsigned long long s_base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const uint32_t word0 = (blockIdx.x * kSelectWarps + warp) * 32;
+  const uint32_t row0 = (word0 + lane) * 32;
+  uint32_t w = 0;
+  if (row0 < n) {
+    w = __ldg(words + word0 + lane);
+    if (!WANT) w = ~w;
+    if (n - row0 < 32) w &= (1u << (n - row0)) - 1u;
+  }
+  const uint32_t incl = warp_inclusive_sum(__popc(w));
+  if (lane == 31) s_cnt[warp] = incl;
+  __syncthreads();
+  const uint32_t c = lane < kSelectWarps ? s_cnt[lane] : 0;
+  const uint32_t all = warp_inclusive_sum(c);
+  const uint32_t mine = __shfl_sync(kFullMask, all - c, warp);
+  if (warp == 0 && lane == kSelectWarps - 1) s_base = all ? atomicAdd(a.d_count, (unsigned long long)all) : 0ull;
+  __syncthreads();
+  const int64_t base = (int64_t)s_base + mine;
+  const uint32_t at = incl - __popc(w);
+  constexpr int B = 8;  // words at a time: their first payload loads are in flight together
+  const PayloadIn in = a.pin[0];
+  const bool one = a.n_pin > 0 && !a.pout[0].valid && (in.width == 8 || in.width == 4);
+  for (int q0 = 0; q0 < 32; q0 += B) {
+    uint64_t v[B];
+    int64_t p[B];
+    uint32_t sel = 0;
+#pragma unroll
+    for (int h = 0; h < B; ++h) {
+      const uint32_t wq = __shfl_sync(kFullMask, w, q0 + h);
+      p[h] = base + __shfl_sync(kFullMask, at, q0 + h) + __popc(wq & below);
+      v[h] = 0;
+      if (!(wq >> lane & 1u) || p[h] >= a.capacity) continue;
+      sel |= 1u << h;
+      const uint32_t i = (word0 + q0 + h) * 32 + lane;
+      if (one)
+        v[h] = in.width == 8 ? (uint64_t)__ldcs(static_cast<const unsigned long long*>(in.data) + i)
+                             : (uint64_t)__ldcs(static_cast<const unsigned int*>(in.data) + i);
+    }
+#pragma unroll
+    for (int h = 0; h < B; ++h) {
+      if (!(sel >> h & 1u)) continue;
+      const uint32_t i = (word0 + q0 + h) * 32 + lane;
+      if (a.out_prid) __stcs(a.out_prid + p[h], (int32_t)i);
+      if (a.out_brid) __stcs(a.out_brid + p[h], kNoRow);
+      if (one) {
+        if (in.width == 8) __stcs(static_cast<unsigned long long*>(a.pout[0].data) + p[h], (unsigned long long)v[h]);
+        else __stcs(static_cast<unsigned int*>(a.pout[0].data) + p[h], (unsigned int)v[h]);
+      }
+      for (int k = one ? 1 : 0; k < a.n_pin; ++k) {
+        store_elem_cs(a.pout[k].data, p[h], a.pin[k].width, pl_load(a.pin[k], i));
+        if (a.pout[k].valid && payload_valid(a.pin[k], i)) set_out_bit(a.pout[k].valid, p[h]);
+      }
+    }
+  }
+}
+
+// MARK from the match bits: one byte per row, and the validity words (a row without a match is NULL when its
+// key is, or when the build has a NULL key). One thread per word.
+__global__ void __launch_bounds__(kKindThreads) mark_rows_kernel(const uint32_t* __restrict__ words, const uint32_t* __restrict__ kv,
+                                                                 int64_t kvoff, int64_t n, KindArgs a) {
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, row0 = q * 32;
+  if (row0 >= n) return;
+  const uint32_t w = __ldg(words + q);
+  const int rows = (int)(n - row0 < 32 ? n - row0 : 32);
+  uint8_t* out = a.mark + row0;
+  if (rows == 32 && ((uintptr_t)out & 15) == 0) {
+    uint32_t b[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t x = w >> (4 * i) & 0xfu;
+      b[i] = (x & 1u) | (x & 2u) << 7 | (x & 4u) << 14 | (x & 8u) << 21;
+    }
+    reinterpret_cast<uint4*>(out)[0] = make_uint4(b[0], b[1], b[2], b[3]);
+    reinterpret_cast<uint4*>(out)[1] = make_uint4(b[4], b[5], b[6], b[7]);
+  } else {
+    for (int i = 0; i < rows; ++i) out[i] = w >> i & 1u;
+  }
+  if (!a.mark_valid) return;
+  uint32_t valid = w;
+  if (!a.build_has_null) {
+    uint32_t known = kFullMask;
+    if (kv) {
+      known = 0;
+      for (int i = 0; i < rows; ++i) known |= (uint32_t)bit_valid(kv, kvoff, row0 + i) << i;
+    }
+    valid |= known;
+  }
+  a.mark_valid[q] = rows == 32 ? valid : valid & ((1u << rows) - 1u);
 }
 
 struct BuildEmitArgs {
@@ -360,6 +457,13 @@ static void launch_kind(const sj_table* t, const sj_column& p, const KindArgs& a
   }
 }
 
+template <bool WANT>
+static void launch_select(const uint32_t* words, int64_t n, const KindArgs& a, cudaStream_t s) {
+  KernelTimer timer("select_rows", s);
+  const int64_t per_cta = (int64_t)kSelectWarps * 1024;
+  select_rows_kernel<WANT><<<(int)((n + per_cta - 1) / per_cta), kKindThreads, 0, s>>>(words, (uint32_t)n, a);
+}
+
 static sj_status probe_payloads(const sj_column& p, const GatherSpec& gs, KindArgs& a) {
   if (gs.n_probe_payload < 0 || gs.n_probe_payload > kMaxPayload)
     return set_error(SJ_ERR_INVALID, "at most 8 payload columns per side");
@@ -388,6 +492,13 @@ static sj_status zero_validity(const sj_mut_column* outs, int n, int64_t capacit
   return SJ_OK;
 }
 
+// Scratch for one bit per probe row. Refused: false, and the join takes the pass that needs none.
+static bool match_bits(int64_t n, const Allocator& alloc, cudaStream_t s, Scratch& bits) {
+  if (bits.get(alloc, (size_t)((n + 31) / 32) * sizeof(uint32_t), s) == SJ_OK) return true;
+  clear_error();
+  return false;
+}
+
 sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const GatherSpec& gs, uint8_t* out_mark,
                      uint32_t* out_mark_valid, const Allocator& alloc, cudaStream_t s, int64_t* d_count) {
   if (kind == SJ_JOIN_INNER) return probe_gather(t, p, gs, alloc, s, d_count);
@@ -408,7 +519,16 @@ sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const 
     a.mark_valid = out_mark_valid;
     a.build_has_null = t->null_rows > 0;
     set_count_kernel<<<1, 1, 0, s>>>(d_count, p.num_rows);
-    if (p.num_rows > 0) launch_kind<kMark>(t, p, a, s);
+    Scratch bits;
+    if (p.num_rows > 0 && match_bits(p.num_rows, alloc, s, bits)) {
+      SJ_TRY(probe_find(t, p, bits.as<uint32_t>(), alloc, s));
+      const int64_t words = (p.num_rows + 31) / 32;
+      KernelTimer timer("mark_rows", s);
+      mark_rows_kernel<<<(int)((words + kKindThreads - 1) / kKindThreads), kKindThreads, 0, s>>>(
+          bits.as<uint32_t>(), p.validity, p.validity_offset, p.num_rows, a);
+    } else if (p.num_rows > 0) {
+      launch_kind<kMark>(t, p, a, s);
+    }
     SJ_CUDA_TRY(cudaGetLastError());
     return SJ_OK;
   }
@@ -417,7 +537,12 @@ sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const 
     a.out_prid = gs.out_probe_rid;
     SJ_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(int64_t), s));
     SJ_TRY(zero_validity(gs.out_probe_payload, gs.n_probe_payload, gs.capacity, s));
-    if (p.num_rows > 0) {
+    Scratch bits;
+    if (p.num_rows > 0 && match_bits(p.num_rows, alloc, s, bits)) {
+      SJ_TRY(probe_find(t, p, bits.as<uint32_t>(), alloc, s));
+      if (kind == SJ_JOIN_SEMI) launch_select<true>(bits.as<uint32_t>(), p.num_rows, a, s);
+      else launch_select<false>(bits.as<uint32_t>(), p.num_rows, a, s);
+    } else if (p.num_rows > 0) {
       if (kind == SJ_JOIN_SEMI) launch_kind<kSemi>(t, p, a, s);
       else launch_kind<kAnti>(t, p, a, s);
     }
@@ -445,27 +570,35 @@ sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const 
   SJ_TRY(marks.get(alloc, 2 * sizeof(unsigned long long), s));
   unsigned long long* m = marks.as<unsigned long long>();
 
-  // 1. INNER rows
-  SJ_TRY(probe_gather(t, p, gs, alloc, s, d_count));
+  // 1. INNER rows, and where the unit probe serves them, one bit per probe row with a match
+  Scratch mbits;
+  const size_t mbytes = (size_t)((p.num_rows + 31) / 32) * sizeof(uint32_t);
+  bool by_probe = false;
+  GatherSpec inner = gs;
+  if (p.num_rows > 0) {
+    SJ_TRY(mbits.get(alloc, mbytes, s));
+    SJ_CUDA_TRY(cudaMemsetAsync(mbits.ptr, 0, mbytes, s));
+    inner.matched = mbits.as<uint32_t>();
+    inner.matched_set = &by_probe;
+  }
+  SJ_TRY(probe_gather(t, p, inner, alloc, s, d_count));
   SJ_CUDA_TRY(cudaMemcpyAsync(m, d_count, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
-  // 2. unmatched probe rows, appended: the probe rows no INNER row names (one bit per probe row, set
-  // from the INNER rows' probe row ids; 0.94 ms for a second lookup of 64M rows before), or a second
-  // lookup when the call writes no probe row ids
+  // 2. unmatched probe rows, appended: the rows whose bit is clear. Where the probe did not set the bits they
+  // are set from the INNER rows' probe row ids; if those overflowed the capacity (known on the device) or are
+  // not written, the rows are looked up again
   a.out_prid = gs.out_probe_rid;
   a.out_brid = gs.out_build_rid;
-  Scratch mbits;
   if (p.num_rows > 0) {
-    if (gs.out_probe_rid && gs.capacity > 0) {
-      const size_t words = (size_t)((p.num_rows + 31) / 32);
-      SJ_TRY(mbits.get(alloc, words * sizeof(uint32_t), s));
-      SJ_CUDA_TRY(cudaMemsetAsync(mbits.ptr, 0, words * sizeof(uint32_t), s));
+    if (by_probe) {
+      launch_select<false>(mbits.as<uint32_t>(), p.num_rows, a, s);
+    } else if (gs.out_probe_rid && gs.capacity > 0) {
       {
         KernelTimer timer("matched_bits", s);
         matched_bits_kernel<<<kind_grid(t, std::min<int64_t>(gs.capacity, p.num_rows)), 256, 0, s>>>(
             gs.out_probe_rid, m, gs.capacity, mbits.as<uint32_t>());
       }
-      a.matched = mbits.as<uint32_t>();
       a.inner_rows = m;
+      launch_select<false>(mbits.as<uint32_t>(), p.num_rows, a, s);
       launch_kind<kUnmatched>(t, p, a, s);
     } else {
       launch_kind<kAnti>(t, p, a, s);

@@ -155,12 +155,123 @@ struct WaitRows {
   uint32_t bucket[32 * S];  // then the row's position
 };
 
+// Table positions of rows first + v0 + 32 j + lane (keys k[j]) of the warp's unit, kNoPos where there is none.
+template <typename K, bool WIDE, bool RUNS, int S>
+__device__ __forceinline__ void unit_lookup(const TableDev& t, const K (&k)[S], const uint32_t* __restrict__ kv, int64_t kvoff,
+                                            uint32_t first, uint32_t v0, uint32_t rows, WaitRows<S>& wait, uint32_t (&pos)[S]) {
+  using Ops = SectorOps<WIDE>;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const uint32_t rid_mask = (1u << t.rbits) - 1u;
+  uint32_t n_wait = 0;
+  uint32_t waits = 0;  // byte j: 1 + place in the list of the lane's row j, or 0
+#pragma unroll
+  for (int j = 0; j < S; ++j) {
+    const uint32_t v = v0 + 32 * j + lane;
+    SectorKey key;
+    uint32_t b, q = 0;
+    pos[j] = kNoPos;
+    bool cont = false;
+    if (sector_key<K, WIDE>(t, k[j], key, b) && v < rows && (RUNS || bit_valid(kv, kvoff, first + v))) {
+      const Sector s = load_sector(t.slots, b);
+      uint32_t p;
+      if (Ops::find(s, key, rid_mask, p, q)) pos[j] = p;
+      else cont = t.segmask != 0 && !Ops::open(s);
+    }
+    const unsigned bal = __ballot_sync(kFullMask, cont);
+    if (bal) {
+      if (cont) {
+        const uint32_t e = n_wait + __popc(bal & below);
+        wait.key[e] = key;
+        wait.bucket[e] = next_bucket(b, t.segmask);
+        waits |= (e + 1) << (8 * j);
+      }
+      n_wait += __popc(bal);
+    }
+  }
+  if (n_wait) {
+    __syncwarp();
+    for (uint32_t e0 = 0; e0 < n_wait; e0 += 32) {
+      const uint32_t e = e0 + lane;
+      bool act = e < n_wait;
+      SectorKey key{};
+      uint32_t b = 0, res = kNoPos;
+      if (act) {
+        key = wait.key[e];
+        b = wait.bucket[e];
+      }
+      for (uint32_t step = 0; step < t.segmask && __any_sync(kFullMask, act); ++step) {
+        if (act) {
+          const Sector s = load_sector(t.slots, b);
+          uint32_t q = 0, p;
+          const bool f = Ops::find(s, key, rid_mask, p, q);
+          if (f) res = p;
+          act = !f && !Ops::open(s);
+          b = next_bucket(b, t.segmask);
+        }
+      }
+      if (e < n_wait) wait.bucket[e] = res;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < S; ++j)
+      if (waits >> (8 * j) & 0xffu) pos[j] = wait.bucket[(waits >> (8 * j) & 0xffu) - 1];
+  }
+}
+
+// Sets the bits of the rows row0 + lane that `found` names: a whole word when the rows are in their own order,
+// else one bit for each partitioned row's row id. (Collected per tile in shared memory and flushed in lines, the
+// bits of 64M rows took 605-770 us with the lookup against 570: what shared memory takes from L1 and from the
+// warps per SM costs more than the atomics.)
+template <bool RUNS>
+__device__ __forceinline__ void mark_found(uint32_t* words, const int32_t* prid_map, uint32_t row0, bool any, unsigned found) {
+  const int lane = threadIdx.x & 31;
+  if constexpr (RUNS) {
+    if (found >> lane & 1u) {
+      const uint32_t r = (uint32_t)__ldg(prid_map + row0 + lane);
+      atomicOr(words + (r >> 5), 1u << (r & 31));
+    }
+  } else {
+    if (lane == 0 && any) words[row0 >> 5] = found;
+  }
+}
+
+// The lookup alone: bit i of `words` = probe row i has a match. NULL rows match the NULL group if it has rows.
+template <typename K, bool WIDE, bool RUNS>
+__global__ void __launch_bounds__(kUnitThreads, 8) find_units_kernel(TableDev t, const K* __restrict__ keys,
+                                                                     const uint32_t* __restrict__ kv, int64_t kvoff,
+                                                                     uint32_t n, RunArgs ra,
+                                                                     const int32_t* __restrict__ prid_map, uint32_t* words) {
+  constexpr int S = 4;
+  __shared__ WaitRows<S> s_wait[kUnitWarps];
+  const int lane = threadIdx.x & 31;
+  const Units u = cta_units<RUNS>(ra);
+  uint32_t first, rows;
+  unit_rows<RUNS, S>(ra, u, n, first, rows);
+  const bool null_found = !RUNS && t.null_group >= 0 && __ldg(t.grp_off + t.null_group + 1) > __ldg(t.grp_off + t.null_group);
+  for (uint32_t v0 = 0; v0 < rows; v0 += 32 * S) {
+    K k[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const uint32_t v = v0 + 32 * j + lane;
+      k[j] = v < rows ? __ldcs(keys + first + v) : (K)0;
+    }
+    uint32_t pos[S];
+    unit_lookup<K, WIDE, RUNS, S>(t, k, kv, kvoff, first, v0, rows, s_wait[threadIdx.x >> 5], pos);
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const uint32_t v = v0 + 32 * j + lane;
+      const bool found = pos[j] != kNoPos || (null_found && v < rows && !bit_valid(kv, kvoff, first + v));
+      mark_found<RUNS>(words, prid_map, first + v0 + 32 * j, v0 + 32 * j < rows, __ballot_sync(kFullMask, found));
+    }
+  }
+}
+
 template <typename K, bool WIDE, bool RUNS, int S, int SP, int SB>
 __global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kernel(TableDev t, const K* __restrict__ keys,
                                                                       const uint32_t* __restrict__ kv, int64_t kvoff,
                                                                       uint32_t n, const int64_t* d_n, RunArgs ra,
                                                                       DirectArgs a) {
-  using Ops = SectorOps<WIDE>;
   using Sh = Shape<SP, SB>;
   if (!RUNS && d_n) n = min(n, (uint32_t)*d_n);
   __shared__ WaitRows<S> s_wait[kUnitWarps];
@@ -169,7 +280,6 @@ __global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kern
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
   WaitRows<S>& wait = s_wait[warp];
-  const uint32_t rid_mask = (1u << t.rbits) - 1u;
   const uint32_t cap = (uint32_t)(a.capacity < (int64_t)0x7fffffff ? a.capacity : (int64_t)0x7fffffff);
   const Units u = cta_units<RUNS>(ra);
   uint32_t first, rows;
@@ -181,63 +291,15 @@ __global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kern
       const uint32_t v = v0 + 32 * j + lane;
       k[j] = v < rows ? __ldcs(keys + first + v) : (K)0;
     }
-    uint32_t pos[S], n_wait = 0;
-    uint32_t waits = 0;  // byte j: 1 + place in the list of the lane's row j, or 0
-#pragma unroll
-    for (int j = 0; j < S; ++j) {
-      const uint32_t v = v0 + 32 * j + lane;
-      SectorKey key;
-      uint32_t b, q = 0;
-      pos[j] = kNoPos;
-      bool cont = false;
-      if (sector_key<K, WIDE>(t, k[j], key, b) && v < rows && (RUNS || bit_valid(kv, kvoff, first + v))) {
-        const Sector s = load_sector(t.slots, b);
-        uint32_t p;
-        if (Ops::find(s, key, rid_mask, p, q)) pos[j] = p;
-        else cont = t.segmask != 0 && !Ops::open(s);
-      }
-      const unsigned bal = __ballot_sync(kFullMask, cont);
-      if (bal) {
-        if (cont) {
-          const uint32_t e = n_wait + __popc(bal & below);
-          wait.key[e] = key;
-          wait.bucket[e] = next_bucket(b, t.segmask);
-          waits |= (e + 1) << (8 * j);
-        }
-        n_wait += __popc(bal);
-      }
-    }
-    if (n_wait) {
-      __syncwarp();
-      for (uint32_t e0 = 0; e0 < n_wait; e0 += 32) {
-        const uint32_t e = e0 + lane;
-        bool act = e < n_wait;
-        SectorKey key{};
-        uint32_t b = 0, res = kNoPos;
-        if (act) {
-          key = wait.key[e];
-          b = wait.bucket[e];
-        }
-        for (uint32_t step = 0; step < t.segmask && __any_sync(kFullMask, act); ++step) {
-          if (act) {
-            const Sector s = load_sector(t.slots, b);
-            uint32_t q = 0, p;
-            const bool f = Ops::find(s, key, rid_mask, p, q);
-            if (f) res = p;
-            act = !f && !Ops::open(s);
-            b = next_bucket(b, t.segmask);
-          }
-        }
-        if (e < n_wait) wait.bucket[e] = res;
-      }
-      __syncwarp();
-#pragma unroll
-      for (int j = 0; j < S; ++j)
-        if (waits >> (8 * j) & 0xffu) pos[j] = wait.bucket[(waits >> (8 * j) & 0xffu) - 1];
-    }
+    uint32_t pos[S];
+    unit_lookup<K, WIDE, RUNS, S>(t, k, kv, kvoff, first, v0, rows, wait, pos);
     uint32_t cnt = 0;
 #pragma unroll
-    for (int j = 0; j < S; ++j) cnt += __popc(__ballot_sync(kFullMask, pos[j] != kNoPos));
+    for (int j = 0; j < S; ++j) {
+      const unsigned bal = __ballot_sync(kFullMask, pos[j] != kNoPos);
+      cnt += __popc(bal);
+      if (a.matched) mark_found<RUNS>(a.matched, a.prid_map, first + v0 + 32 * j, v0 + 32 * j < rows, bal);
+    }
     if (lane == 0) s_cnt[warp] = cnt;
     int32_t prid[S];
     uint64_t pv[S];
@@ -287,18 +349,26 @@ static DirectArgs plain_records(DirectArgs a) {
   return a;
 }
 
+// Runs cut into pieces of about 128 rows (a run holds kPartTileRows / P rows): with whole runs of 1024 rows a
+// warp's chain was eight times as long and the few warps of a 1M-row probe took 100 us instead of 63.
+static RunArgs unit_pieces(RunArgs ra) {
+  ra.log2_pieces = 0;
+  while (((uint64_t)ra.P * 128 << ra.log2_pieces) < kPartTileRows) ++ra.log2_pieces;
+  return ra;
+}
+
+static int unit_grid(int64_t n, int unit, const RunArgs* ra) {
+  auto ctas = [](int64_t units) { return (units + kUnitWarps - 1) / kUnitWarps; };
+  return (int)(ra ? ra->P * ctas((int64_t)ra->n_tiles << ra->log2_pieces) : ctas((n + unit - 1) / unit));
+}
+
 void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t kvoff, int64_t n, const int64_t* d_n,
                  const RunArgs* runs, const DirectArgs& a_in, cudaStream_t s) {
   if (n == 0) return;
   const DirectArgs a = plain_records(a_in);
-  RunArgs ra = runs ? *runs : RunArgs{};
-  // pieces of about 128 rows (a run holds kPartTileRows / P rows): with whole runs of 1024 rows a warp's
-  // chain was eight times as long and the few warps of a 1M-row probe took 100 us instead of 63
-  while (runs && ((uint64_t)ra.P * 128 << ra.log2_pieces) < kPartTileRows) ++ra.log2_pieces;
+  const RunArgs ra = runs ? unit_pieces(*runs) : RunArgs{};
   const bool few = !runs && n <= kFewRows;
-  auto ctas = [](int64_t units) { return (units + kUnitWarps - 1) / kUnitWarps; };
-  const int64_t unit = few ? 32 : 128;
-  const int grid = (int)(runs ? ra.P * ctas((int64_t)ra.n_tiles << ra.log2_pieces) : ctas((n + unit - 1) / unit));
+  const int grid = unit_grid(n, few ? 32 : 128, runs ? &ra : nullptr);
   const TableDev d = table_dev(t);
   KernelTimer timer("probe_units", s);
   using std::integral_constant;
@@ -315,6 +385,29 @@ void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_
     if (both && a.n_pin == 1 && a.pin_w[0] == 8 && a.n_bin == 2) shape(k, w, integral_constant<int, 1>{}, integral_constant<int, 2>{});
     else if (both && a.n_pin == 0 && a.n_bin == 1) shape(k, w, integral_constant<int, 0>{}, integral_constant<int, 1>{});
     else shape(k, w, integral_constant<int, -1>{}, integral_constant<int, -1>{});
+  };
+  const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
+  if (t->key_type == SJ_INT32) {
+    if (wide) go(int32_t{}, std::true_type{});
+    else go(int32_t{}, std::false_type{});
+  } else {
+    if (wide) go(int64_t{}, std::true_type{});
+    else go(int64_t{}, std::false_type{});
+  }
+}
+
+void find_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t kvoff, int64_t n, const RunArgs* runs,
+                const int32_t* prid_map, uint32_t* words, cudaStream_t s) {
+  if (n == 0) return;
+  const RunArgs ra = runs ? unit_pieces(*runs) : RunArgs{};
+  const int grid = unit_grid(n, 128, runs ? &ra : nullptr);
+  const TableDev d = table_dev(t);
+  KernelTimer timer("find_units", s);
+  auto go = [&](auto k, auto w) {
+    using K = decltype(k);
+    constexpr bool W = decltype(w)::value;
+    auto kernel = runs ? find_units_kernel<K, W, true> : find_units_kernel<K, W, false>;
+    kernel<<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(keys), kv, kvoff, (uint32_t)n, ra, prid_map, words);
   };
   const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
   if (t->key_type == SJ_INT32) {
