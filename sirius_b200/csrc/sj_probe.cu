@@ -21,6 +21,7 @@
 //     output position per step (load-balanced search over the offsets staged in shared memory),
 //     so a probe key matching 10^6 build rows is spread over the whole GPU instead of one thread.
 #include <algorithm>
+#include <type_traits>
 
 #include "sj_device.cuh"
 #include "sj_internal.h"
@@ -317,130 +318,25 @@ __global__ void __launch_bounds__(kProbeThreads, 4) probe_distinct_kernel(TableD
 }
 
 // ------------------------------------------------------------------------------------------------
-// GROUPED pass A: find each probe row's group; compact (row, start, size); sum the output size.
-// A warp owns 32 * kMatchR consecutive probe rows per tile, lane l rows base + 32 j + l, so every
-// key load is one coalesced warp access; a bucket is tested as a whole (one slot per distinct
-// key); the rows with matches of row group j are ranked with one ballot and written at
-// base + (earlier groups) + popc(ballot_j & lanes below), one atomicAdd per warp tile.
-// ------------------------------------------------------------------------------------------------
-constexpr int kMatchR = 4;
-
-template <typename K, bool WIDE, bool COMPACT>
-__global__ void __launch_bounds__(kProbeThreads, 4) grouped_match_kernel(TableDev t, const K* __restrict__ keys,
-                                                                          const uint32_t* __restrict__ kv,
-                                                                          int64_t kvoff, int64_t n, int32_t* m_row,
-                                                                          int32_t* m_start, int32_t* m_cnt,
-                                                                          unsigned long long* d_nent,
-                                                                          unsigned long long* d_total) {
-  using Ops = SlotOps<WIDE>;
-  constexpr int R = kMatchR;
-  const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << lane) - 1u;
-  const int64_t wtiles = (n + 32 * R - 1) / (32 * R);
-  const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const uint64_t kmask = ~((1ull << t.rbits) - 1);
-  unsigned long long total = 0;
-  for (int64_t wt = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); wt < wtiles; wt += wstride) {
-    const int64_t r0 = wt * 32 * R + lane;
-    K k[R];
-    uint32_t act = 0;
-    int32_t slot[R];
-#pragma unroll
-    for (int j = 0; j < R; ++j) {
-      const int64_t r = r0 + 32 * j;
-      k[j] = r < n ? __ldcs(keys + r) : (K)0;
-      slot[j] = -1;
-    }
-#pragma unroll
-    for (int j = 0; j < R; ++j) {
-      const int64_t r = r0 + 32 * j;
-      if (r >= n) continue;
-      if (!bit_valid(kv, kvoff, r)) {
-        if (t.null_group >= 0) slot[j] = t.null_group;  // NULLs equal: the NULL group
-      } else if (in_range(t, k[j])) {
-        act |= 1u << j;
-      }
-    }
-    uint32_t b[R];
-    uint64_t ks[R];
-#pragma unroll
-    for (int j = 0; j < R; ++j) {
-      const uint64_t kb = key_u64<K>(k[j]);
-      b[j] = home_bucket(t, kb);
-      ks[j] = Ops::probe_key((uint64_t)(long long)k[j] - (uint64_t)t.kmin, kb, t.rbits);
-    }
-    for (uint32_t step = 0; act && step <= t.segmask; ++step) {
-      Bucket bk[R];
-#pragma unroll
-      for (int j = 0; j < R; ++j)
-        if (act >> j & 1u) bk[j] = load_bucket<true>(t.slots, b[j]);
-#pragma unroll
-      for (int j = 0; j < R; ++j) {
-        if (!(act >> j & 1u)) continue;
-        int q;
-        const bool m = Ops::match_slot(bk[j], ks[j], kmask, q);
-        if (m) slot[j] = (int32_t)(b[j] * Ops::kSlots + q);
-        if (m || Ops::open(bk[j])) act &= ~(1u << j);
-        else b[j] = next_bucket(b[j], t.segmask);
-      }
-    }
-    int32_t start[R], cnt[R];
-    uint32_t hit = 0;
-#pragma unroll
-    for (int j = 0; j < R; ++j) {
-      start[j] = cnt[j] = 0;
-      if (slot[j] >= 0) {
-        start[j] = __ldg(t.grp_off + slot[j]);
-        cnt[j] = __ldg(t.grp_off + slot[j] + 1) - start[j];
-        if (cnt[j] > 0) hit |= 1u << j;
-        total += (unsigned long long)cnt[j];
-      }
-    }
-    if (COMPACT) {
-      unsigned bal[R];
-      uint32_t tot = 0;
-#pragma unroll
-      for (int j = 0; j < R; ++j) {
-        bal[j] = __ballot_sync(kFullMask, (hit >> j) & 1u);
-        tot += __popc(bal[j]);
-      }
-      if (tot) {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(d_nent, (unsigned long long)tot);
-        base = __shfl_sync(kFullMask, base, 0);
-#pragma unroll
-        for (int j = 0; j < R; ++j) {
-          if (hit >> j & 1u) {
-            const unsigned long long p = base + __popc(bal[j] & below);
-            m_row[p] = (int32_t)(r0 + 32 * j);
-            m_start[p] = start[j];
-            m_cnt[p] = cnt[j];
-          }
-          base += __popc(bal[j]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) total += __shfl_down_sync(kFullMask, total, d);
-  if (lane == 0 && total) atomicAdd(d_total, total);
-}
-
-// ------------------------------------------------------------------------------------------------
 // GROUPED expand: output position j -> (entry e with m_off[e] <= j < m_off[e+1]) -> one row.
 //
-// Every warp works alone (no CTA barrier): it owns a contiguous range of 256-output tiles and, per
-// tile, stages the entries the tile touches (at most 257: every entry has at least one output) in
-// its own shared-memory area, finds each output's entry there, loads the build rows and stores.
-// Lane l handles outputs j0 + 32m + l (m < 8), so each store is one coalesced warp access. A
-// warp's first entry comes from a 32-ary search of m_off (5 steps for 32M entries); every later
-// tile starts at the entry the previous tile ended in.
+// Every warp works alone (no CTA barrier): it owns a contiguous range of 256-output tiles and, per tile,
+// stages the entries the tile touches (at most 256, 32 at a time until one starts behind the tile) as one
+// 8-byte word each — probe row, and what to add to an output's place in the tile to get its group member —
+// and one bit per output where an entry starts. An output's entry is then the number of starts up to it:
+// one word, one popc, one 8-byte load from shared memory, whatever the groups' sizes. Lane l handles outputs
+// j0 + 32m + l (m < 8), so each store is one coalesced warp access. A warp's first entry comes from a 32-ary
+// search of m_off (5 steps for 32M entries); every later tile starts at the entry the previous tile ended in,
+// and its first entries are loaded while the tile before is written. 32M Zipf probe rows into 8M, 1.1e8 outputs
+// of 12 bytes: 427 us (511 before: 257 entries of 16 bytes staged for every 256 outputs, 92 instructions per
+// output, now about 48). It waits for records and entries (8 loads per lane in flight, 32 warps per SM); fewer
+// loads and more warps took 479 (4, 40 warps) and 551 us (2, 48 warps).
 // ------------------------------------------------------------------------------------------------
 constexpr int kExpandThreads = 256;
 constexpr int kExpandWarps = kExpandThreads / 32;
 constexpr int kExpandItems = 8;
 constexpr int kExpandOut = 32 * kExpandItems;  // outputs per warp tile
-constexpr int kExpandEnt = kExpandOut + 1;     // entries a tile can touch
+constexpr int kExpandRun = 8;                  // consecutive tiles of a warp
 
 // Largest e in [0, n) with off[e] <= j (off[0] <= j assumed), found by the whole warp: each step
 // compares 32 evenly spaced candidates and keeps the gap between the last one at or below j and
@@ -470,171 +366,186 @@ __device__ __forceinline__ int64_t warp_upper_index(const int64_t* off, int64_t 
 // one payload of RS / 2 bytes at offset RS / 2 (no validity), no probe payloads; one load per row.
 // RS = 0: the shape is read from `g` at run time.
 template <int RS>
-__global__ void __launch_bounds__(kExpandThreads, 4) expand_kernel(const int32_t* __restrict__ m_row,
-                                                                const int32_t* __restrict__ m_start,
+__global__ void __launch_bounds__(kExpandThreads, RS == 16 ? 3 : 4) expand_kernel(const int2* __restrict__ m_ent,
                                                                 const int64_t* __restrict__ m_off,
                                                                 const unsigned long long* d_nent,
                                                                 const int32_t* __restrict__ grp_rid,
                                                                 GatherArgs g) {
-  __shared__ int64_t s_off_all[kExpandWarps][kExpandEnt];
-  __shared__ int32_t s_row_all[kExpandWarps][kExpandEnt];
-  __shared__ int32_t s_start_all[kExpandWarps][kExpandEnt];
+  __shared__ int2 s_ent_all[kExpandWarps][kExpandOut + 32];  // {probe row, group start - offset in the tile}
+  __shared__ uint32_t s_start_all[kExpandWarps][kExpandItems];  // bit l of word m: an entry starts at 32 m + l > 0
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  int64_t* s_off = s_off_all[warp];
-  int32_t* s_row = s_row_all[warp];
-  int32_t* s_start = s_start_all[warp];
+  int2* s_ent = s_ent_all[warp];
+  uint32_t* s_starts = s_start_all[warp];
   const int64_t nent = (int64_t)*d_nent;
   if (nent == 0) return;
   const int64_t M = __ldg(m_off + nent);
   const int64_t cap = M < g.capacity ? M : g.capacity;
   const int64_t ntile = (cap + kExpandOut - 1) / kExpandOut;
   const int64_t nwarps = (int64_t)gridDim.x * kExpandWarps;
-  const int64_t per_warp = (ntile + nwarps - 1) / nwarps;
-  const int64_t t_lo = ((int64_t)blockIdx.x * kExpandWarps + warp) * per_warp;
-  const int64_t t_hi = t_lo + per_warp < ntile ? t_lo + per_warp : ntile;
-  if (t_lo >= t_hi) return;
-  int64_t e0 = warp_upper_index(m_off, nent, t_lo * kExpandOut);
-  for (int64_t tile = t_lo; tile < t_hi; ++tile) {
-    const int64_t j0 = tile * kExpandOut;
-    const int64_t j1 = j0 + kExpandOut < cap ? j0 + kExpandOut : cap;
-    const int ne = (int)((nent - e0) < kExpandEnt ? (nent - e0) : kExpandEnt);
-    for (int i = lane; i < ne; i += 32) {
-      s_off[i] = __ldg(m_off + e0 + i);
-      s_row[i] = __ldg(m_row + e0 + i);
-      s_start[i] = __ldg(m_start + e0 + i);
-    }
-    __syncwarp();
-    // 1. entries (shared memory only): eb = the entry of the warp's first position of item m; the
-    //    next 31 entry starts are read one per lane and OR-ed into a mask of lane offsets, so a
-    //    lane's entry is eb plus the starts at or below it
-    int32_t row[kExpandItems], gi[kExpandItems];
-    int eb = 0;
-#pragma unroll
-    for (int m = 0; m < kExpandItems; ++m) {
-      const int64_t jb = j0 + 32 * m;
-      const int64_t j = jb + lane;
-      row[m] = 0;
-      gi[m] = -1;
-      if (jb >= j1) continue;  // warp-uniform
-      const int nb = eb + 1 + lane;
-      const int64_t rel = (lane < 31 && nb < ne) ? s_off[nb] - jb : 64;
-      const unsigned starts = __reduce_or_sync(kFullMask, rel < 32 ? (1u << rel) : 0u);
-      const unsigned upto = lane == 31 ? kFullMask : ((2u << lane) - 1u);
-      const int e = eb + __popc(starts & upto);
-      if (j < j1) {
-        row[m] = s_row[e];
-        gi[m] = s_start[e] + (int32_t)(j - s_off[e]);
+  for (int64_t t_lo = ((int64_t)blockIdx.x * kExpandWarps + warp) * kExpandRun; t_lo < ntile; t_lo += nwarps * kExpandRun) {
+    const int64_t t_hi = t_lo + kExpandRun < ntile ? t_lo + kExpandRun : ntile;
+    int64_t e0 = warp_upper_index(m_off, nent, t_lo * kExpandOut);
+    // the tile's first 32 entries, loaded while the tile before is written
+    int64_t off = 0;
+    int2 ent = make_int2(0, 0);
+    auto fetch = [&]() {
+      const bool in = e0 + lane < nent;
+      off = in ? __ldg(m_off + e0 + lane) : INT64_MAX;
+      if (in) ent = __ldg(m_ent + e0 + lane);
+    };
+    fetch();
+    for (int64_t tile = t_lo; tile < t_hi; ++tile) {
+      const int64_t j0 = tile * kExpandOut;
+      const int64_t j1 = j0 + kExpandOut < cap ? j0 + kExpandOut : cap;
+      if (lane < kExpandItems) s_starts[lane] = 0;
+      __syncwarp();
+      auto stage = [&](int i) {
+        const bool in = off < j1;
+        const int rel = in ? (int)(off - j0) : 1;  // a group has at most 2^31 rows
+        if (in) {
+          s_ent[i + lane] = make_int2(ent.x, ent.y - rel);
+          if (rel > 0) atomicOr(&s_starts[rel >> 5], 1u << (rel & 31));
+        }
+        return rel;
+      };
+      // one or two entries start at or before the tile
+      int eb = __popc(__ballot_sync(kFullMask, stage(0) <= 0)) - 1;
+      for (int i = 32; i < kExpandOut + 32 && __all_sync(kFullMask, off < j1); i += 32) {
+        const int64_t e = e0 + i + lane;
+        off = e < nent ? __ldg(m_off + e) : INT64_MAX;
+        if (e < nent) ent = __ldg(m_ent + e);
+        stage(i);
       }
-      // the entry of position jb + 32: lane 31's entry, or the next one if it starts right there
-      const int e31 = __shfl_sync(kFullMask, e, 31);
-      eb = e31 + ((e31 + 1 < ne && s_off[e31 + 1] == jb + 32) ? 1 : 0);
-    }
-    // 2. group members (table positions)
-    int32_t pos[kExpandItems];
+      __syncwarp();
+      // 1. entries: the starts up to each output, counted from the tile's first entry
+      const unsigned upto = kFullMask >> (31 - lane);
+      if constexpr (RS > 0) {
+        // one record load per output, and stores at fixed distances from the tile's first output
+        using V = std::conditional_t<RS == 8, uint2, uint4>;
+        const int n_out = (int)(j1 - j0);
+        int32_t row[kExpandItems];
+        V v[kExpandItems];
 #pragma unroll
-    for (int m = 0; m < kExpandItems; ++m) pos[m] = gi[m] < 0 ? 0 : grp_rid ? __ldg(grp_rid + gi[m]) : gi[m];
-    // 3. build side: one row-store record per item, or row id (+ payloads by row id / position)
-    if constexpr (RS == 8 || RS == 16) {
-      uint32_t rid[kExpandItems];
-      uint64_t fv[kExpandItems];
+        for (int m = 0; m < kExpandItems; ++m) {
+          const uint32_t starts = s_starts[m];
+          const int r = 32 * m + lane;
+          if (r < n_out) {
+            const int2 x = s_ent[eb + __popc(starts & upto)];
+            row[m] = x.x;
+            v[m] = __ldg(static_cast<const V*>(g.rec) + (uint32_t)(x.y + r));
+          }
+          eb += __popc(starts);
+        }
+        e0 += eb;  // the entry of the tile's last output
+        if (tile + 1 < t_hi) fetch();
+        int32_t* op = g.out_prid ? g.out_prid + j0 + lane : nullptr;
+        int32_t* ob = g.out_brid ? g.out_brid + j0 + lane : nullptr;
+        using P = std::conditional_t<RS == 8, unsigned int, unsigned long long>;
+        P* oc = static_cast<P*>(g.bout[0].data) + j0 + lane;
 #pragma unroll
-      for (int m = 0; m < kExpandItems; ++m) {
-        rid[m] = 0;
-        fv[m] = 0;
-        if (gi[m] < 0) continue;
-        const char* rp = static_cast<const char*>(g.rec) + (int64_t)pos[m] * RS;
-        if constexpr (RS == 8) {
-          const uint2 x = __ldg(reinterpret_cast<const uint2*>(rp));
-          rid[m] = x.x;
-          fv[m] = x.y;
+        for (int m = 0; m < kExpandItems; ++m) {
+          if (32 * m + lane >= n_out) continue;
+          if (op) __stcs(op + 32 * m, row[m]);
+          if (ob) __stcs(ob + 32 * m, (int32_t)v[m].x);
+          if constexpr (RS == 8) __stcs(oc + 32 * m, v[m].y);
+          else __stcs(oc + 32 * m, (unsigned long long)v[m].w << 32 | v[m].z);
+        }
+      } else {
+        int32_t row[kExpandItems], gi[kExpandItems];
+#pragma unroll
+        for (int m = 0; m < kExpandItems; ++m) {
+          const uint32_t starts = s_starts[m];
+          const int r = 32 * m + lane;
+          row[m] = 0;
+          gi[m] = -1;
+          if (j0 + r < j1) {
+            const int2 x = s_ent[eb + __popc(starts & upto)];
+            row[m] = x.x;
+            gi[m] = x.y + r;
+          }
+          eb += __popc(starts);
+        }
+        e0 += eb;
+        if (tile + 1 < t_hi) fetch();
+        // 2. group members (table positions)
+        int32_t pos[kExpandItems];
+#pragma unroll
+        for (int m = 0; m < kExpandItems; ++m) pos[m] = gi[m] < 0 ? 0 : grp_rid ? __ldg(grp_rid + gi[m]) : gi[m];
+        // 3. build side: one row-store record per item, or row id (+ payloads by row id / position)
+        if (g.rec) {
+          constexpr int kHalf = kExpandItems / 2;  // 4 records (up to 32 registers) in flight at a time
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            Record r[kHalf];
+#pragma unroll
+            for (int q = 0; q < kHalf; ++q) {
+              const int m = h * kHalf + q;
+              if (gi[m] >= 0)
+                r[q] = load_record(static_cast<const char*>(g.rec) + (int64_t)pos[m] * g.rec_stride, g.rec_stride);
+            }
+#pragma unroll
+            for (int q = 0; q < kHalf; ++q) {
+              const int m = h * kHalf + q;
+              const int64_t j = j0 + 32 * m + lane;
+              const bool live = gi[m] >= 0;
+              if (live && g.out_prid) __stcs(g.out_prid + j, row[m]);
+              if (live && g.out_brid) __stcs(g.out_brid + j, (int32_t)r[q].w[0]);
+              for (int c = 0; c < g.n_bin; ++c) {
+                const int w = g.bin[c].width;
+                if (live) store_elem_cs(g.bout[c].data, j, w, record_field(r[q], g.rec_off[c], w));
+                if (g.rec_voff[c] >= 0) {
+                  const unsigned word = __ballot_sync(kFullMask, live && record_field(r[q], g.rec_voff[c], 1) != 0);
+                  if (lane == 0 && j - lane < j1) g.bout[c].valid[(j - lane) >> 5] = word;
+                }
+              }
+            }
+          }
         } else {
-          const uint4 x = __ldg(reinterpret_cast<const uint4*>(rp));
-          rid[m] = x.x;
-          fv[m] = ((uint64_t)x.w << 32) | x.z;
+          int32_t rid[kExpandItems];
+#pragma unroll
+          for (int m = 0; m < kExpandItems; ++m) rid[m] = gi[m] >= 0 ? brid_of(g, pos[m]) : 0;
+#pragma unroll
+          for (int m = 0; m < kExpandItems; ++m) {
+            const int64_t j = j0 + 32 * m + lane;
+            const bool live = gi[m] >= 0;
+            if (live && g.out_prid) __stcs(g.out_prid + j, row[m]);
+            if (live && g.out_brid) __stcs(g.out_brid + j, rid[m]);
+            for (int c = 0; c < g.n_bin; ++c) {
+              const PayloadIn in = g.bin[c];
+              const int32_t idx = g.bin_by_pos ? pos[m] : rid[m];
+              bool v = false;
+              if (live) {
+                store_elem_cs(g.bout[c].data, j, in.width, pl_load(in, idx));
+                v = payload_valid(in, idx);
+              }
+              if (has_validity(in)) {
+                const unsigned word = __ballot_sync(kFullMask, v);
+                if (lane == 0 && j - lane < j1) g.bout[c].valid[(j - lane) >> 5] = word;
+              }
+            }
+          }
         }
-      }
+        // 4. probe payloads (by probe row)
+        for (int c = 0; c < g.n_pin; ++c) {
+          const PayloadIn in = g.pin[c];
+          uint64_t v[kExpandItems];
 #pragma unroll
-      for (int m = 0; m < kExpandItems; ++m) {
-        if (gi[m] < 0) continue;
-        const int64_t j = j0 + 32 * m + lane;
-        if (g.out_prid) __stcs(g.out_prid + j, row[m]);
-        if (g.out_brid) __stcs(g.out_brid + j, (int32_t)rid[m]);
-        if constexpr (RS == 8) __stcs(static_cast<unsigned int*>(g.bout[0].data) + j, (unsigned int)fv[m]);
-        else __stcs(static_cast<unsigned long long*>(g.bout[0].data) + j, (unsigned long long)fv[m]);
-      }
-    } else if (g.rec) {
-      constexpr int kHalf = kExpandItems / 2;  // 4 records (up to 32 registers) in flight at a time
+          for (int m = 0; m < kExpandItems; ++m) v[m] = gi[m] >= 0 ? pl_load(in, row[m]) : 0;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        Record r[kHalf];
-#pragma unroll
-        for (int q = 0; q < kHalf; ++q) {
-          const int m = h * kHalf + q;
-          if (gi[m] >= 0)
-            r[q] = load_record(static_cast<const char*>(g.rec) + (int64_t)pos[m] * g.rec_stride, g.rec_stride);
-        }
-#pragma unroll
-        for (int q = 0; q < kHalf; ++q) {
-          const int m = h * kHalf + q;
-          const int64_t j = j0 + 32 * m + lane;
-          const bool live = gi[m] >= 0;
-          if (live && g.out_prid) __stcs(g.out_prid + j, row[m]);
-          if (live && g.out_brid) __stcs(g.out_brid + j, (int32_t)r[q].w[0]);
-          for (int c = 0; c < g.n_bin; ++c) {
-            const int w = g.bin[c].width;
-            if (live) store_elem_cs(g.bout[c].data, j, w, record_field(r[q], g.rec_off[c], w));
-            if (g.rec_voff[c] >= 0) {
-              const unsigned word = __ballot_sync(kFullMask, live && record_field(r[q], g.rec_voff[c], 1) != 0);
-              if (lane == 0 && j - lane < j1) g.bout[c].valid[(j - lane) >> 5] = word;
+          for (int m = 0; m < kExpandItems; ++m) {
+            const int64_t j = j0 + 32 * m + lane;
+            const bool live = gi[m] >= 0;
+            if (live) store_elem_cs(g.pout[c].data, j, in.width, v[m]);
+            if (has_validity(in)) {
+              const unsigned word = __ballot_sync(kFullMask, live && payload_valid(in, row[m]));
+              if (lane == 0 && j - lane < j1) g.pout[c].valid[(j - lane) >> 5] = word;
             }
           }
         }
       }
-    } else {
-      int32_t rid[kExpandItems];
-#pragma unroll
-      for (int m = 0; m < kExpandItems; ++m) rid[m] = gi[m] >= 0 ? brid_of(g, pos[m]) : 0;
-#pragma unroll
-      for (int m = 0; m < kExpandItems; ++m) {
-        const int64_t j = j0 + 32 * m + lane;
-        const bool live = gi[m] >= 0;
-        if (live && g.out_prid) __stcs(g.out_prid + j, row[m]);
-        if (live && g.out_brid) __stcs(g.out_brid + j, rid[m]);
-        for (int c = 0; c < g.n_bin; ++c) {
-          const PayloadIn in = g.bin[c];
-          const int32_t idx = g.bin_by_pos ? pos[m] : rid[m];
-          bool v = false;
-          if (live) {
-            store_elem_cs(g.bout[c].data, j, in.width, pl_load(in, idx));
-            v = payload_valid(in, idx);
-          }
-          if (has_validity(in)) {
-            const unsigned word = __ballot_sync(kFullMask, v);
-            if (lane == 0 && j - lane < j1) g.bout[c].valid[(j - lane) >> 5] = word;
-          }
-        }
-      }
+      __syncwarp();  // every lane is done with this tile's staged entries
     }
-    // 4. probe payloads (by probe row)
-    for (int c = 0; c < (RS > 0 ? 0 : g.n_pin); ++c) {
-      const PayloadIn in = g.pin[c];
-      uint64_t v[kExpandItems];
-#pragma unroll
-      for (int m = 0; m < kExpandItems; ++m) v[m] = gi[m] >= 0 ? pl_load(in, row[m]) : 0;
-#pragma unroll
-      for (int m = 0; m < kExpandItems; ++m) {
-        const int64_t j = j0 + 32 * m + lane;
-        const bool live = gi[m] >= 0;
-        if (live) store_elem_cs(g.pout[c].data, j, in.width, v[m]);
-        if (has_validity(in)) {
-          const unsigned word = __ballot_sync(kFullMask, live && payload_valid(in, row[m]));
-          if (lane == 0 && j - lane < j1) g.pout[c].valid[(j - lane) >> 5] = word;
-        }
-      }
-    }
-    e0 += eb;      // the entry of position j0 + 256: where the next tile starts
-    __syncwarp();  // every lane is done with this tile's staged entries
   }
 }
 
@@ -683,34 +594,6 @@ static void dispatch_distinct(const sj_table* t, const sj_column& p, const int64
 #undef SJ_D
 }
 
-template <typename K, bool WIDE, bool COMPACT>
-static void launch_match(const sj_table* t, const sj_column& p, int32_t* m_row, int32_t* m_start, int32_t* m_cnt,
-                         unsigned long long* d_nent, unsigned long long* d_total, cudaStream_t s) {
-  const int block = kProbeThreads;
-  KernelTimer timer(COMPACT ? "grouped_match" : "grouped_count", s);
-  const int64_t wtiles = (p.num_rows + 32 * kMatchR - 1) / (32 * kMatchR);
-  const int64_t cap = (int64_t)sm_count(t->device) * std::max(1, t->params.ctas_per_sm);
-  const int grid = (int)std::max<int64_t>(1, std::min(cap, (wtiles + kWarpsPerCta - 1) / kWarpsPerCta));
-  grouped_match_kernel<K, WIDE, COMPACT><<<grid, block, 0, s>>>(
-      table_dev(t), static_cast<const K*>(p.data), p.validity, p.validity_offset, p.num_rows, m_row, m_start,
-      m_cnt, d_nent, d_total);
-}
-
-template <bool COMPACT>
-static void dispatch_match(const sj_table* t, const sj_column& p, int32_t* m_row, int32_t* m_start, int32_t* m_cnt,
-                           unsigned long long* d_nent, unsigned long long* d_total, cudaStream_t s) {
-  const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
-#define SJ_M(K, W) launch_match<K, W, COMPACT>(t, p, m_row, m_start, m_cnt, d_nent, d_total, s)
-  if (t->key_type == SJ_INT32) {
-    if (wide) SJ_M(int32_t, true);
-    else SJ_M(int32_t, false);
-  } else {
-    if (wide) SJ_M(int64_t, true);
-    else SJ_M(int64_t, false);
-  }
-#undef SJ_M
-}
-
 static sj_status check_probe(const sj_table* t, const sj_column& p) {
   SJ_TRY(validate_column(&p, "probe key", true));
   if (p.type != t->key_type) return set_error(SJ_ERR_INVALID, "probe key type differs from the build key type");
@@ -730,7 +613,7 @@ sj_status probe_count(const sj_table* t, const sj_column& p, const Allocator& al
     g.d_count = dc;
     dispatch_distinct<true>(t, p, nullptr, g, s);
   } else {
-    dispatch_match<false>(t, p, nullptr, nullptr, nullptr, nullptr, dc, s);
+    match_units(t, p, nullptr, nullptr, nullptr, dc, s);
   }
   SJ_CUDA_TRY(cudaGetLastError());
   return SJ_OK;
@@ -965,14 +848,13 @@ sj_status probe_gather(const sj_table* t, const sj_column& p, const GatherSpec& 
   const size_t b_tmp = kScanBlocks * sizeof(int64_t);
   SJ_TRY(sc.get(alloc, 3 * b_row + b_off + b_tmp + 256, s));
   char* base = sc.as<char>();
-  int32_t* m_row = reinterpret_cast<int32_t*>(base);
-  int32_t* m_start = reinterpret_cast<int32_t*>(base + b_row);
+  int2* m_ent = reinterpret_cast<int2*>(base);  // {probe row, group start}
   int32_t* m_cnt = reinterpret_cast<int32_t*>(base + 2 * b_row);
   int64_t* m_off = reinterpret_cast<int64_t*>(base + 3 * b_row);
   int64_t* tmp = reinterpret_cast<int64_t*>(base + 3 * b_row + b_off);
   unsigned long long* d_nent = reinterpret_cast<unsigned long long*>(base + 3 * b_row + b_off + b_tmp);
   SJ_CUDA_TRY(cudaMemsetAsync(d_nent, 0, sizeof(unsigned long long), s));
-  dispatch_match<true>(t, p, m_row, m_start, m_cnt, d_nent, g.d_count, s);
+  match_units(t, p, m_ent, m_cnt, d_nent, g.d_count, s);
   {
     KernelTimer timer("scan", s);
     device_exclusive_scan<int32_t, int64_t>(m_cnt, m_off, d_nent, 0, tmp, s);
@@ -989,7 +871,7 @@ sj_status probe_gather(const sj_table* t, const sj_column& p, const GatherSpec& 
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kExpandThreads, 0);
   const int grid = sm_count(t->device) * std::max(1, per_sm);
   KernelTimer timer("expand", s);
-  kernel<<<grid, kExpandThreads, 0, s>>>(m_row, m_start, m_off, d_nent, t->grp_rid, g);
+  kernel<<<grid, kExpandThreads, 0, s>>>(m_ent, m_off, d_nent, t->grp_rid, g);
   SJ_CUDA_TRY(cudaGetLastError());
   return SJ_OK;
 }

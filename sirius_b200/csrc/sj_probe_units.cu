@@ -155,8 +155,9 @@ struct WaitRows {
   uint32_t bucket[32 * S];  // then the row's position
 };
 
-// Table positions of rows first + v0 + 32 j + lane (keys k[j]) of the warp's unit, kNoPos where there is none.
-template <typename K, bool WIDE, bool RUNS, int S>
+// Table positions (SLOT: slots) of rows first + v0 + 32 j + lane (keys k[j]) of the warp's unit, kNoPos where
+// there is none.
+template <typename K, bool WIDE, bool RUNS, int S, bool SLOT = false>
 __device__ __forceinline__ void unit_lookup(const TableDev& t, const K (&k)[S], const uint32_t* __restrict__ kv, int64_t kvoff,
                                             uint32_t first, uint32_t v0, uint32_t rows, WaitRows<S>& wait, uint32_t (&pos)[S]) {
   using Ops = SectorOps<WIDE>;
@@ -175,7 +176,7 @@ __device__ __forceinline__ void unit_lookup(const TableDev& t, const K (&k)[S], 
     if (sector_key<K, WIDE>(t, k[j], key, b) && v < rows && (RUNS || bit_valid(kv, kvoff, first + v))) {
       const Sector s = load_sector(t.slots, b);
       uint32_t p;
-      if (Ops::find(s, key, rid_mask, p, q)) pos[j] = p;
+      if (SLOT ? Ops::find_slot(s, key, rid_mask, q) : Ops::find(s, key, rid_mask, p, q)) pos[j] = SLOT ? b * Ops::kSlots + q : p;
       else cont = t.segmask != 0 && !Ops::open(s);
     }
     const unsigned bal = __ballot_sync(kFullMask, cont);
@@ -204,8 +205,8 @@ __device__ __forceinline__ void unit_lookup(const TableDev& t, const K (&k)[S], 
         if (act) {
           const Sector s = load_sector(t.slots, b);
           uint32_t q = 0, p;
-          const bool f = Ops::find(s, key, rid_mask, p, q);
-          if (f) res = p;
+          const bool f = SLOT ? Ops::find_slot(s, key, rid_mask, q) : Ops::find(s, key, rid_mask, p, q);
+          if (f) res = SLOT ? b * Ops::kSlots + q : p;
           act = !f && !Ops::open(s);
           b = next_bucket(b, t.segmask);
         }
@@ -333,6 +334,82 @@ __global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kern
 // warps of 64 rows with a reservation each, before: 6.5, 8.5, 12.8, 17.7, 50.5, 98.0 us).
 constexpr int64_t kFewRows = 400000;
 
+// GROUPED tables: each probe row's group. COMPACT: appends (row, group start, group size) of the rows with
+// matches; always: adds the matches up. One reservation per CTA (1024 rows): with one per warp of 128 rows the
+// entry counter alone took 176 us of a 32M-row probe (one same-address atomic per 0.67 ns).
+template <typename K, bool WIDE, bool COMPACT>
+__global__ void __launch_bounds__(kUnitThreads, 6) match_units_kernel(TableDev t, const K* __restrict__ keys,
+                                                                      const uint32_t* __restrict__ kv, int64_t kvoff,
+                                                                      uint32_t n, int2* m_ent, int32_t* m_cnt,
+                                                                      unsigned long long* d_nent,
+                                                                      unsigned long long* d_total) {
+  constexpr int S = 4;
+  __shared__ WaitRows<S> s_wait[kUnitWarps];
+  __shared__ uint32_t s_ent[kUnitWarps];
+  __shared__ unsigned long long s_sum[kUnitWarps], s_base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const Units u = cta_units<false>(RunArgs{});
+  uint32_t first, rows;
+  unit_rows<false, S>(RunArgs{}, u, n, first, rows);
+  K k[S];
+#pragma unroll
+  for (int j = 0; j < S; ++j) {
+    const uint32_t v = 32 * j + lane;
+    k[j] = v < rows ? __ldcs(keys + first + v) : (K)0;
+  }
+  uint32_t slot[S];
+  unit_lookup<K, WIDE, false, S, true>(t, k, kv, kvoff, first, 0, rows, s_wait[warp], slot);
+  int32_t start[S], cnt[S];
+  unsigned long long sum = 0;
+  uint32_t ents = 0;
+#pragma unroll
+  for (int j = 0; j < S; ++j) {
+    const uint32_t v = 32 * j + lane;
+    if (t.null_group >= 0 && v < rows && !bit_valid(kv, kvoff, first + v)) slot[j] = (uint32_t)t.null_group;
+    start[j] = cnt[j] = 0;
+    if (slot[j] != kNoPos) {
+      start[j] = __ldg(t.grp_off + slot[j]);
+      cnt[j] = __ldg(t.grp_off + slot[j] + 1) - start[j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < S; ++j) {
+    sum += (unsigned long long)cnt[j];
+    ents += __popc(__ballot_sync(kFullMask, cnt[j] > 0));
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) sum += __shfl_down_sync(kFullMask, sum, d);
+  if (lane == 0) {
+    s_ent[warp] = ents;
+    s_sum[warp] = sum;
+  }
+  __syncthreads();
+  const uint32_t c = lane < kUnitWarps ? s_ent[lane] : 0;
+  const uint32_t incl = warp_inclusive_sum(c);
+  if (warp == 0) {
+    unsigned long long all = lane < kUnitWarps ? s_sum[lane] : 0;
+#pragma unroll
+    for (int d = kUnitWarps / 2; d > 0; d >>= 1) all += __shfl_down_sync(kFullMask, all, d);
+    if (lane == 0 && all) atomicAdd(d_total, all);
+    if (COMPACT && lane == kUnitWarps - 1) s_base = incl ? atomicAdd(d_nent, (unsigned long long)incl) : 0ull;
+  }
+  if constexpr (COMPACT) {
+    uint32_t run = __shfl_sync(kFullMask, incl - c, warp);
+    __syncthreads();
+    run += (uint32_t)s_base;
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const unsigned bal = __ballot_sync(kFullMask, cnt[j] > 0);
+      const uint32_t e = run + __popc(bal & below);
+      run += __popc(bal);
+      if (cnt[j] <= 0) continue;
+      m_ent[e] = make_int2((int32_t)(first + 32 * j + lane), start[j]);
+      m_cnt[e] = cnt[j];
+    }
+  }
+}
+
 // Records are held in registers when they are [row id | one 4-byte field] or [row id | - | 8-byte
 // fields]; the fields of other records are gathered from the row store one by one.
 static DirectArgs plain_records(DirectArgs a) {
@@ -408,6 +485,30 @@ void find_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t
     constexpr bool W = decltype(w)::value;
     auto kernel = runs ? find_units_kernel<K, W, true> : find_units_kernel<K, W, false>;
     kernel<<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(keys), kv, kvoff, (uint32_t)n, ra, prid_map, words);
+  };
+  const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
+  if (t->key_type == SJ_INT32) {
+    if (wide) go(int32_t{}, std::true_type{});
+    else go(int32_t{}, std::false_type{});
+  } else {
+    if (wide) go(int64_t{}, std::true_type{});
+    else go(int64_t{}, std::false_type{});
+  }
+}
+
+void match_units(const sj_table* t, const sj_column& p, int2* m_ent, int32_t* m_cnt, unsigned long long* d_nent,
+                 unsigned long long* d_total, cudaStream_t s) {
+  if (p.num_rows == 0) return;
+  const bool compact = m_ent != nullptr;
+  const int grid = unit_grid(p.num_rows, 128, nullptr);
+  const TableDev d = table_dev(t);
+  KernelTimer timer(compact ? "grouped_match" : "grouped_count", s);
+  auto go = [&](auto k, auto w) {
+    using K = decltype(k);
+    constexpr bool W = decltype(w)::value;
+    auto kernel = compact ? match_units_kernel<K, W, true> : match_units_kernel<K, W, false>;
+    kernel<<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(p.data), p.validity, p.validity_offset,
+                                         (uint32_t)p.num_rows, m_ent, m_cnt, d_nent, d_total);
   };
   const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
   if (t->key_type == SJ_INT32) {

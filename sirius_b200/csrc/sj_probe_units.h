@@ -15,4 +15,9 @@ void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_
 void find_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t kvoff, int64_t n, const RunArgs* runs,
                 const int32_t* prid_map, uint32_t* words, cudaStream_t s);
 
+// GROUPED table: adds the matches of all probe rows to *d_total and, when m_ent is given, appends {probe row, group
+// start} and the group size of the rows with matches to m_ent / m_cnt at *d_nent.
+void match_units(const sj_table* t, const sj_column& p, int2* m_ent, int32_t* m_cnt, unsigned long long* d_nent,
+                 unsigned long long* d_total, cudaStream_t s);
+
 }  // namespace sj
