@@ -749,7 +749,8 @@ sj_status partition_columns(const void* keys, int key_type, int64_t n, int pbits
                             int device, cudaStream_t s, const int64_t** d_total_out, const int64_t** d_offs_out,
                             int* grid_out) {
   if (pbits < 0 || pbits > kMaxPartBits) return set_error(SJ_ERR_INVALID, "partition bits out of range");
-  const int G = sm_count(device) * kColCtasPerSm;  // one chunk per CTA, all resident
+  // one chunk per CTA, all resident, and none for less than a tile (25K rows: 7 CTAs, not 296)
+  const int G = (int)std::max<int64_t>(1, std::min<int64_t>((n + kColTile - 1) / kColTile, (int64_t)sm_count(device) * kColCtasPerSm));
   const int P = 1 << pbits;
   const size_t PG = (size_t)P * G;
   char* base = static_cast<char*>(scratch);
