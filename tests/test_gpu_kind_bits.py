@@ -1,5 +1,5 @@
-"""SEMI / ANTI / MARK / LEFT by match bits: row counts at the edges of words (32), units (128) and select CTAs (8192
-rows); a table that is looked up in partition order, with NULL keys and int32 and wide slots; capacities at, above
+"""SEMI / ANTI / MARK / LEFT by match bits: row counts at the edges of words (32), units (128), select CTAs (8192
+rows) and of the sizes that take two passes; a table that is looked up in partition order, with NULL keys and int32 and wide slots; capacities at, above
 and below the row count; every refusal of an allocator."""
 import ctypes
 
@@ -40,7 +40,8 @@ def _check(cuda, bk, pk, pv, pp, capacity=None, **kw):
             assert np.array_equal(got[:out.count].cpu().numpy(), c[rid])
 
 
-@pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129, 1023, 1025, 8191, 8192, 8193, 100_001])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129, 1023, 1025, 8191, 8192, 8193, 100_001,
+                               (8 << 20) - 1, 8 << 20, (8 << 20) + 8193])
 @pytest.mark.parametrize("types", [(), (np.int64,), (np.int8, np.int32), (np.float32, np.int16)])
 def test_row_count_edges(cuda, n, types):
     rng = np.random.default_rng(n + len(types))
@@ -66,7 +67,7 @@ def test_refused_scratch_takes_the_pass_without(cuda, kind):
     """An allocator that refuses everything after the build: the join still runs, with the same rows."""
     rng = np.random.default_rng(8)
     bk = dev_t(rng.permutation(40_000)[:20_000].astype(np.int64), cuda)
-    pk = dev_t(rng.integers(0, 40_000, 300_000).astype(np.int64), cuda)
+    pk = dev_t(rng.integers(0, 40_000, 9_000_001).astype(np.int64), cuda)
     with J.HashTable(bk) as t:
         want = t.probe_join(kind, pk)
         A, F = L.SjAlloc._fields_[1][1], L.SjAlloc._fields_[2][1]
