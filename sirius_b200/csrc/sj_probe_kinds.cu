@@ -494,9 +494,9 @@ static sj_status zero_validity(const sj_mut_column* outs, int n, int64_t capacit
 
 // Scratch for one bit per probe row. False: the join takes the one pass that needs none, because the allocator
 // refuses, or because the probe is small: a second launch and an allocation cost more than the better lookup gains
-// (SEMI of 14K rows 46 / 69 us, ANTI of 1.9M rows 72 / 83, MARK of 4.4M rows 116 / 120, of 19M rows 191 / 166,
-// one pass / two passes).
-constexpr int64_t kMinMatchBits = 8 << 20;
+// (SEMI of 14K rows 46 / 69 us, ANTI of 1.9M rows 72 / 83, of 8.5M rows 124 / 130, MARK of 19M rows 191 / 166, one
+// pass / two passes).
+constexpr int64_t kMinMatchBits = 16 << 20;
 static bool match_bits(int64_t n, const Allocator& alloc, cudaStream_t s, Scratch& bits) {
   if (n < kMinMatchBits) return false;
   if (bits.get(alloc, (size_t)((n + 31) / 32) * sizeof(uint32_t), s) == SJ_OK) return true;

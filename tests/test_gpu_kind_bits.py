@@ -1,6 +1,6 @@
 """SEMI / ANTI / MARK / LEFT by match bits: row counts at the edges of words (32), units (128), select CTAs (8192
-rows) and of the sizes that take two passes; a table that is looked up in partition order, with NULL keys and int32 and wide slots; capacities at, above
-and below the row count; every refusal of an allocator."""
+rows) and of the sizes that take two passes; a table that is looked up in partition order, with NULL keys and int32
+and wide slots; an allocator that refuses the bits."""
 import ctypes
 
 import numpy as np
@@ -41,7 +41,7 @@ def _check(cuda, bk, pk, pv, pp, capacity=None, **kw):
 
 
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129, 1023, 1025, 8191, 8192, 8193, 100_001,
-                               (8 << 20) - 1, 8 << 20, (8 << 20) + 8193])
+                               (16 << 20) - 1, 16 << 20, (16 << 20) + 8193])
 @pytest.mark.parametrize("types", [(), (np.int64,), (np.int8, np.int32), (np.float32, np.int16)])
 def test_row_count_edges(cuda, n, types):
     rng = np.random.default_rng(n + len(types))
@@ -57,7 +57,7 @@ def test_lookup_in_partition_order(cuda, dtype, wide):
     rng = np.random.default_rng(3)
     nb = (2 << 20) + 5 if wide else (5 << 20)
     bk = rng.permutation(3 * nb)[:nb].astype(dtype)
-    n = 10_000_019
+    n = 16_800_019
     pk = rng.integers(0, 3 * nb, n).astype(dtype)
     _check(cuda, bk, pk, rng.random(n) > 0.03, [rng.integers(0, 100, n).astype(np.int32)], force_wide=wide, load_factor=0.4)
 
@@ -67,7 +67,7 @@ def test_refused_scratch_takes_the_pass_without(cuda, kind):
     """An allocator that refuses everything after the build: the join still runs, with the same rows."""
     rng = np.random.default_rng(8)
     bk = dev_t(rng.permutation(40_000)[:20_000].astype(np.int64), cuda)
-    pk = dev_t(rng.integers(0, 40_000, 9_000_001).astype(np.int64), cuda)
+    pk = dev_t(rng.integers(0, 40_000, 17_000_001).astype(np.int64), cuda)
     with J.HashTable(bk) as t:
         want = t.probe_join(kind, pk)
         A, F = L.SjAlloc._fields_[1][1], L.SjAlloc._fields_[2][1]
