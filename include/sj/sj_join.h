@@ -309,7 +309,8 @@ typedef enum sj_join_kind {
  *          (bitmask, may be NULL only when no row can be NULL) marks NULL the unmatched rows whose
  *          probe key is NULL, or every unmatched row when the build side has a NULL key (the IN rule
  *          of resolve_mark_join_result; the table must use SJ_NULLS_UNEQUAL). *d_count = probe rows.
- * Rows beyond `capacity` are not written (*d_count still counts them). Stream-ordered. */
+ * Rows beyond `capacity` are not written (*d_count still counts them). Stream-ordered. Scratch comes from
+ * `alloc`; SEMI, ANTI and MARK run without any when it is refused. */
 SJ_EXPORT sj_status sj_probe_join(const sj_table* table, sj_join_kind kind, const sj_column* probe_keys,
                                   int32_t num_keys, const sj_column* probe_payload, int32_t num_probe_payload,
                                   const sj_column* build_payload, int32_t num_build_payload, int32_t* out_probe_rid,

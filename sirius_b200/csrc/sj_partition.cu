@@ -574,11 +574,11 @@ sj_status radix_partition(const PartSrc& src, int key_type, int pbits, const Par
 // partition runs with consecutive threads on consecutive positions. The loads of the next column (or
 // of the next tile's keys) are in registers before a column is written, so reads overlap writes. The
 // key column, when the caller wants it reordered too, is staged from the registers it was hashed in.
-// 4096-row tiles: a run holds 4096 / P rows, twice the length of the 2048-row tiles above. 64M int64
-// keys and one int64 column into 64 partitions: 1,114 us with row ids and a key copy written by
-// part_scatter_fast_kernel, 502 us here (4.3 TB/s of 2.1 GB; while it took 514 us, other shapes of
-// threads x rows x CTAs per SM took 542 (256x8x4), 541 (512x4x3), 524 (256x16x2), 526 us (1024x4x2)). It is bound by its write fronts, P per CTA, that
-// advance by one run of a tile at a time.
+// 4096-row tiles: a run holds 4096 / P rows, twice the length of the 2048-row tiles above. 64M int64 keys
+// and one int64 column into 64 partitions: 1,114 us with row ids and a key copy written by
+// part_scatter_fast_kernel, 502 us here (4.3 TB/s of 2.1 GB). While it took 514 us, other shapes of threads
+// x rows x CTAs per SM took 542 (256x8x4), 541 (512x4x3), 524 (256x16x2) and 526 us (1024x4x2). It is bound
+// by its write fronts, P per CTA, that advance by one run of a tile at a time.
 // ------------------------------------------------------------------------------------------------
 constexpr int kColThreads = 512;
 constexpr int kColRows = 8;      // rows per thread

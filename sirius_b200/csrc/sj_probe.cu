@@ -4,7 +4,8 @@
 // gather_join_output (:1299-1359): the output row (probe rid, build rid, probe payloads, build
 // payloads) is written once, by the kernel that found the match.
 //
-// DISTINCT tables (one slot per build row, unique keys) take a single pass:
+// DISTINCT tables (one slot per build row, unique keys) take a single pass, the unit probe
+// (sj_probe_units.cu) where it serves the output, else the staged kernel here:
 //   - every thread owns KPT = 4 consecutive probe rows and reads their keys with 128-bit
 //     streaming loads (ld.global.cs: the probe stream must not evict the table from L2);
 //   - keys outside [key_min, key_max] or NULL are rejected without touching the table;
@@ -13,13 +14,12 @@
 //   - matches are compacted warp-aggregated: __shfl_up prefix of the per-lane hit counts and one
 //     atomicAdd per warp reserves the warp's output range;
 //   - payloads are gathered straight into the reserved positions (build columns by row id).
-// GROUPED tables (duplicated keys, or NULLs equal) take count -> scan -> expand:
-//   - pass A finds each probe row's group and appends (probe row, group start, group size) to a
-//     compacted match list (warp-aggregated), summing the output size M;
+// GROUPED tables (duplicated keys, or NULLs equal) take match -> scan -> expand:
+//   - match_units (sj_probe_units.cu) finds each probe row's group and appends {probe row, group start} and
+//     the group size to a compacted match list, summing the output size M;
 //   - an exclusive scan turns group sizes into output offsets;
-//   - the expand kernel gives every CTA a contiguous range of output tiles and each thread one
-//     output position per step (load-balanced search over the offsets staged in shared memory),
-//     so a probe key matching 10^6 build rows is spread over the whole GPU instead of one thread.
+//   - the expand kernel gives every warp tiles of 256 consecutive outputs and finds each output's entry, so
+//     a probe key matching 10^6 build rows is spread over the whole GPU instead of one thread.
 #include <algorithm>
 #include <type_traits>
 
