@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kExpandThreads, RS == 16 ? 3 : 4) expand_kerne
   if (nent == 0) return;
   const int64_t M = __ldg(m_off + nent);
   const int64_t cap = M < g.capacity ? M : g.capacity;
-  const uint32_t ntile = (uint32_t)((cap + kExpandOut - 1) / kExpandOut);  // the outputs fit the device
+  const uint32_t ntile = (uint32_t)((cap + kExpandOut - 1) / kExpandOut);  // some output is written: it fits the device
   const uint32_t nwarps = gridDim.x * kExpandWarps;
   // every warp gets tiles first (1.2M outputs: 69 us with 8 tiles for each of 600 warps, 16 with one or two each)
   const uint32_t run = ntile >= nwarps * kExpandRun ? kExpandRun : 1 + ntile / nwarps;
@@ -840,6 +840,13 @@ sj_status probe_gather(const sj_table* t, const sj_column& p, const GatherSpec& 
     }
     if (t->pbits > 0 && p.num_rows >= kMinPartitionedProbe) return probe_partitioned(t, p, g, alloc, s);
     if (!probe_direct(t, p, nullptr, g, s)) dispatch_distinct<false>(t, p, nullptr, g, s);
+    SJ_CUDA_TRY(cudaGetLastError());
+    return SJ_OK;
+  }
+  if (!g.out_prid && !g.out_brid && g.n_pin == 0 && g.n_bin == 0) {
+    // nothing to write: the count alone. The expand numbers tiles in 32 bits, enough for outputs that are in
+    // memory; without any, the matches up to `capacity` may be 2^40 and more.
+    match_units(t, p, nullptr, nullptr, nullptr, g.d_count, s);
     SJ_CUDA_TRY(cudaGetLastError());
     return SJ_OK;
   }

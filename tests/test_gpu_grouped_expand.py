@@ -60,3 +60,23 @@ def test_group_sizes(cuda, sizes, types, n_probe, absent, null_frac):
 @pytest.mark.parametrize("capacity", [1, 31, 255, 256, 257, 2047, 2049, 5000])
 def test_capacity_cuts_a_tile(cuda, capacity):
     _run(cuda, SIZES["small"](np.random.default_rng(2)), 1500, (np.int32,), 7, capacity)
+
+
+def test_no_outputs_is_a_count(cuda):
+    """Row ids and payloads all left out, any capacity: the matches are counted and nothing is expanded."""
+    rng = np.random.default_rng(4)
+    bk, pk = rng.integers(0, 500, 20_000), rng.integers(0, 1000, 30_000)
+    dk, dc = dev_t(pk, cuda), torch.zeros(1, dtype=torch.int64, device=cuda)
+    keys, nk, _ = J._keys(dk)
+    with J.HashTable(dev_t(bk, cuda), layout=L.SJ_LAYOUT_GROUPED) as t:
+        L.timing_collect()
+        L.timing_enable(True)
+        try:
+            L.check(L.load().sj_probe_gather(t.handle, keys, nk, None, 0, None, 0, None, None, None, None, 1 << 62, None,
+                                             None, dc.data_ptr()), "sj_probe_gather")
+            torch.cuda.synchronize()
+            names = [name for name, _ in L.timing_collect()]
+        finally:
+            L.timing_enable(False)
+    assert int(dc.item()) == int(np.bincount(bk, minlength=1000)[pk].sum())
+    assert "expand" not in names and names, names
