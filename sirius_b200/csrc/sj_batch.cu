@@ -633,13 +633,20 @@ static sj_status reset_batch(sj_batch_plan* P, cudaStream_t s) {
   return SJ_OK;
 }
 
+// The limit is one value for the whole process: the largest block's, not this plan's, which another thread's plan
+// of smaller blocks could lower before this one's launch.
+template <typename Kernel>
+static void allow_stage_smem(Kernel* kernel) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem(8, 512));
+}
+
 static int resident_ctas(sj_batch_plan* P) {
   int per_sm = 0;
   const int block = P->params.block_size;
   dispatch_kg(P->key_type, P->params.group_width, P->shape, [&](auto k, auto g, auto sh) {
     auto* kern = batch_persistent_kernel<decltype(k), decltype(g)::value, decltype(sh)::value>;
     const size_t smem = (decltype(g)::value == 1 ? stage_smem(decltype(sh)::value, block) : 0);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_stage_smem(kern);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem);
   });
   per_sm = std::max(1, std::min(per_sm, P->params.ctas_per_sm));
@@ -821,9 +828,7 @@ SJ_EXPORT sj_status sj_batch_plan_launch_per_join(sj_batch_plan* P, sj_stream_t 
   const int block = P->params.block_size;
   const int cap = sm_count(P->device) * P->params.ctas_per_sm;
   dispatch_kg(P->key_type, P->params.group_width, P->shape, [&](auto k, auto g, auto sh) {
-    const size_t smem = (decltype(g)::value == 1 ? stage_smem(decltype(sh)::value, block) : 0);
-    cudaFuncSetAttribute(batch_probe_one_kernel<decltype(k), decltype(g)::value, decltype(sh)::value>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_stage_smem(batch_probe_one_kernel<decltype(k), decltype(g)::value, decltype(sh)::value>);
   });
   KernelTimer timer("batch_per_join", s);
   for (int32_t j = 0; j < P->n_joins; ++j) {

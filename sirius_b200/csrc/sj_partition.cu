@@ -129,6 +129,22 @@ static ScatterSmem scatter_smem(int pbits, int kw, const PartSrc& s) {
   return m;
 }
 
+// The dynamic shared memory limit of a kernel is one value for the whole process, so each kernel gets the most that
+// any call asks of it: with the call's own size, a thread that partitions into fewer parts lowered the limit
+// between another thread's set and its launch.
+static sj_status allow_smem(const void* kernel, size_t most) {
+  SJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  return SJ_OK;
+}
+
+static size_t most_scatter_smem() {
+  PartSrc s{};
+  s.n_pay = kMaxPayload;
+  static const uint32_t some = 0;
+  for (int c = 0; c < kMaxPayload; ++c) s.pay[c] = column_payload(nullptr, &some, 0, 8);
+  return scatter_smem(kMaxPartBits, 8, s).total;
+}
+
 template <typename K>
 __global__ void __launch_bounds__(kPartThreads) part_scatter_kernel(PartSrc s, int pbits, int64_t chunk,
                                                                     const int64_t* __restrict__ off, PartDst d,
@@ -458,7 +474,7 @@ static sj_status launch_fast_scatter(const PartSrc& src, int pbits, int64_t chun
                                      const PartDst& dst, int G, cudaStream_t s) {
   const FastSmem m = fast_smem(pbits, sizeof(K), src.n_pay);
   auto go = [&](auto kernel) -> sj_status {
-    SJ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m.total));
+    SJ_TRY(allow_smem((const void*)kernel, fast_smem(kMaxPartBits, 8, kFastMaxPay).total));
     KernelTimer timer("partition_scatter", s);
     kernel<<<G, kPartThreads, m.total, s>>>(src, pbits, chunk, offs, dst, m);
     return SJ_OK;
@@ -489,13 +505,13 @@ static int scatter_per_sm(const PartSrc& src, int key_type, int pbits, bool fast
       k = src.n_pay == 0 ? (const void*)part_scatter_fast_kernel<int64_t, 0>
           : src.n_pay == 1 ? (const void*)part_scatter_fast_kernel<int64_t, 1>
                            : (const void*)part_scatter_fast_kernel<int64_t, 2>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m.total);
+    allow_smem(k, fast_smem(kMaxPartBits, 8, kFastMaxPay).total);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k, kPartThreads, m.total);
   } else {
     const ScatterSmem m = scatter_smem(pbits, key_type == SJ_INT32 ? 4 : 8, src);
     const void* k = key_type == SJ_INT32 ? (const void*)part_scatter_kernel<int32_t>
                                          : (const void*)part_scatter_kernel<int64_t>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m.total);
+    allow_smem(k, most_scatter_smem());
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k, kPartThreads, m.total);
   }
   cudaGetLastError();
@@ -549,13 +565,11 @@ sj_status radix_partition(const PartSrc& src, int key_type, int pbits, const Par
   }
   const ScatterSmem m = scatter_smem(pbits, key_type == SJ_INT32 ? 4 : 8, src);
   if (key_type == SJ_INT32) {
-    SJ_CUDA_TRY(cudaFuncSetAttribute(part_scatter_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)m.total));
+    SJ_TRY(allow_smem((const void*)part_scatter_kernel<int32_t>, most_scatter_smem()));
     KernelTimer timer("partition_scatter", s);
     part_scatter_kernel<int32_t><<<G, kPartThreads, m.total, s>>>(src, pbits, chunk, offs, dst, m);
   } else {
-    SJ_CUDA_TRY(cudaFuncSetAttribute(part_scatter_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)m.total));
+    SJ_TRY(allow_smem((const void*)part_scatter_kernel<int64_t>, most_scatter_smem()));
     KernelTimer timer("partition_scatter", s);
     part_scatter_kernel<int64_t><<<G, kPartThreads, m.total, s>>>(src, pbits, chunk, offs, dst, m);
   }
@@ -777,7 +791,7 @@ sj_status partition_columns(const void* keys, int key_type, int64_t n, int pbits
   auto go = [&](auto k) -> sj_status {
     using K = decltype(k);
     const size_t smem = columns_smem(pbits);
-    SJ_CUDA_TRY(cudaFuncSetAttribute(part_columns_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SJ_TRY(allow_smem((const void*)part_columns_kernel<K>, columns_smem(kMaxPartBits)));
     KernelTimer timer("partition_scatter", s);
     part_columns_kernel<K><<<G, kColThreads, smem, s>>>(static_cast<const K*>(keys), key_pairs, (uint32_t)n, pbits, (uint32_t)chunk, offs, cols);
     return SJ_OK;

@@ -1,6 +1,9 @@
 """The partition operator's column scatter at the edges of its 4096-row tiles: row counts around a tile and
 around one chunk per CTA, the key column first, last and absent among 0..8 columns of every width, NULLs,
-columns that do not start on a row pair's alignment, and no rows."""
+columns that do not start on a row pair's alignment, no rows,
+and threads with different part counts (their shared memory differs)."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -46,3 +49,27 @@ def test_column_scatter_edges(cuda, n, key_at, n_cols, shift):
         assert np.array_equal(o.cpu().numpy(), h[at])
         if v is not None:
             assert np.array_equal(O.unpack_validity(vo.cpu().numpy().view(np.uint32), n), v[at])
+
+
+@pytest.mark.parametrize("null_keys", [False, True])
+def test_threads_with_different_part_counts(cuda, null_keys):
+    n = 20_000
+    keys = torch.arange(n, dtype=torch.int64, device=cuda)
+    key = [(keys, torch.full(((n + 31) // 32,), -1, dtype=torch.int32, device=cuda))] if null_keys else keys
+    errors, streams = [], [torch.cuda.Stream(device=cuda) for _ in range(3)]
+    torch.cuda.synchronize()
+
+    def work(parts, stream):
+        try:
+            with torch.cuda.stream(stream):
+                for _ in range(400):
+                    off = J.hash_partition(key, [keys], parts, stream=stream)[2]
+                assert int(off[-1].item()) == n
+        except Exception as e:
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=a) for a in zip((1024, 2, 64), streams)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
