@@ -57,9 +57,11 @@ struct Scratch {
     bytes = n < 16 ? 16 : n;
     return a.allocate(&ptr, bytes, s);
   }
-  ~Scratch() {
+  void drop() {
     if (ptr) alloc->release(ptr, bytes, stream);
+    ptr = nullptr;
   }
+  ~Scratch() { drop(); }
   template <typename T>
   T* as() const {
     return static_cast<T*>(ptr);

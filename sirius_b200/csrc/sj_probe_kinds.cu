@@ -580,13 +580,29 @@ sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const 
   const size_t mbytes = (size_t)((p.num_rows + 31) / 32) * sizeof(uint32_t);
   bool by_probe = false;
   GatherSpec inner = gs;
-  if (p.num_rows > 0) {
+  // The bits are optional here, and the INNER probe's own scratch, taken after them and given back before the
+  // next step, has the better claim: a budget that holds either but not both must do.
+  auto get_bits = [&]() -> sj_status {
     SJ_TRY(mbits.get(alloc, mbytes, s));
     SJ_CUDA_TRY(cudaMemsetAsync(mbits.ptr, 0, mbytes, s));
-    inner.matched = mbits.as<uint32_t>();
-    inner.matched_set = &by_probe;
+    return SJ_OK;
+  };
+  if (p.num_rows > 0) {
+    if (sj_status e = get_bits(); e == SJ_OK) {
+      inner.matched = mbits.as<uint32_t>();
+      inner.matched_set = &by_probe;
+    } else if (e != SJ_ERR_OOM) {
+      return e;
+    }
   }
-  SJ_TRY(probe_gather(t, p, inner, alloc, s, d_count));
+  sj_status probed = probe_gather(t, p, inner, alloc, s, d_count);
+  if (probed == SJ_ERR_OOM && mbits.ptr) {
+    mbits.drop();
+    by_probe = false;
+    probed = probe_gather(t, p, gs, alloc, s, d_count);
+  }
+  SJ_TRY(probed);
+  clear_error();  // of an allocation that was refused and then done without
   SJ_CUDA_TRY(cudaMemcpyAsync(m, d_count, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
   // 2. unmatched probe rows, appended: the rows whose bit is clear. Where the probe did not set the bits they
   // are set from the INNER rows' probe row ids; if those overflowed the capacity (known on the device) or are
@@ -597,6 +613,7 @@ sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const 
     if (by_probe) {
       launch_select<false>(mbits.as<uint32_t>(), p.num_rows, a, s);
     } else if (gs.out_probe_rid && gs.capacity > 0) {
+      if (!mbits.ptr) SJ_TRY(get_bits());
       {
         KernelTimer timer("matched_bits", s);
         matched_bits_kernel<<<kind_grid(t, std::min<int64_t>(gs.capacity, p.num_rows)), 256, 0, s>>>(
@@ -609,6 +626,7 @@ sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const 
       launch_kind<kAnti>(t, p, a, s);
     }
   }
+  mbits.drop();
   SJ_CUDA_TRY(cudaMemcpyAsync(m + 1, d_count, sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
 
   // 3. FULL: unmatched build rows. With build row ids written: the build rows no INNER row names

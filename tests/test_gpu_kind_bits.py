@@ -62,6 +62,74 @@ def test_lookup_in_partition_order(cuda, dtype, wide):
     _check(cuda, bk, pk, rng.random(n) > 0.03, [rng.integers(0, 100, n).astype(np.int32)], force_wide=wide, load_factor=0.4)
 
 
+class Budget:
+    """An allocator over torch tensors that refuses what would take more than `limit` bytes at a time."""
+
+    def __init__(self, cuda, limit=1 << 62):
+        self.limit, self.live, self.peak, held = limit, 0, 0, {}
+
+        def alloc(ctx, size, stream):
+            if self.live + size > self.limit:
+                return None
+            t = torch.empty(max(1, size), dtype=torch.uint8, device=cuda)
+            held[t.data_ptr()] = (t, size)
+            self.live += size
+            self.peak = max(self.peak, self.live)
+            return t.data_ptr()
+
+        def free(ctx, p, size, stream):
+            self.live -= held.pop(p)[1]
+        self._calls = L.SjAlloc._fields_[1][1](alloc), L.SjAlloc._fields_[2][1](free)
+        self.c = L.SjAlloc(None, *self._calls)
+
+
+def _join_under(budget, t, kind, pk, n_out, rids=True):
+    """(status, count, probe row ids, build row ids) of a join whose scratch comes from `budget`."""
+    rid = [torch.empty(max(1, n_out), dtype=torch.int32, device=pk.device) for _ in range(2)]
+    dc = torch.zeros(1, dtype=torch.int64, device=pk.device)
+    keys, nk, _ = J._keys(pk)
+    p = [r.data_ptr() if rids else None for r in rid]
+    st = L.load().sj_probe_join(t.handle, kind, keys, nk, None, 0, None, 0, *p, None, None, n_out, None, None,
+                                ctypes.byref(budget.c), None, dc.data_ptr())
+    torch.cuda.synchronize()
+    return st, int(dc.item()), rid[0], rid[1]
+
+
+@pytest.mark.parametrize("kind", [L.SJ_JOIN_LEFT, L.SJ_JOIN_FULL])
+@pytest.mark.parametrize("layout", [L.SJ_LAYOUT_DISTINCT, L.SJ_LAYOUT_GROUPED])
+@pytest.mark.parametrize("pbits", [-1, 3])
+def test_outer_joins_need_no_more_than_the_larger_of_their_parts(cuda, kind, layout, pbits):
+    """The match bits are not worth a refusal: with room for the INNER probe's scratch or the bits, not both."""
+    rng = np.random.default_rng(2)
+    bk = rng.permutation(300_000)[:200_000].astype(np.int64)
+    pk = dev_t(rng.integers(0, 300_000, 1_000_000).astype(np.int64), cuda)
+    bits = 1_000_000 // 8
+    with J.HashTable(dev_t(bk, cuda), layout=layout, partition_bits=pbits) as t:
+        inner = Budget(cuda)
+        dc = torch.zeros(1, dtype=torch.int64, device=cuda)
+        out = torch.empty(1_000_000, dtype=torch.int32, device=cuda)
+        keys, nk, _ = J._keys(pk)
+        L.check(L.load().sj_probe_gather(t.handle, keys, nk, None, 0, None, 0, out.data_ptr(), None, None, None,
+                                         1_000_000, ctypes.byref(inner.c), None, dc.data_ptr()), "sj_probe_gather")
+        torch.cuda.synchronize()
+        n_out = 1_000_000 + (200_000 if kind == L.SJ_JOIN_FULL else 0)
+        st, want, p, b = _join_under(Budget(cuda), t, kind, pk, n_out)
+        assert st == L.SJ_OK and want == 1_000_000 + (
+            200_000 - len(np.intersect1d(bk, pk.cpu().numpy())) if kind == L.SJ_JOIN_FULL else 0)
+        rows = O.canonical(p[:want].cpu().numpy(), b[:want].cpu().numpy())
+        # the two counters of the call, and for FULL its flag bytes (one per slot) and build-row bits
+        later = (int(t.info().num_slots) + 1 + 200_000 // 8 + 64 if kind == L.SJ_JOIN_FULL else 0)
+        budget = Budget(cuda, 16 + max(inner.peak, bits + later))
+        st, got, p, b = _join_under(budget, t, kind, pk, n_out)
+        assert st == L.SJ_OK, (st, L.load().sj_last_error())
+        assert got == want
+        for x, y in zip(rows, O.canonical(p[:got].cpu().numpy(), b[:got].cpu().numpy())):
+            assert np.array_equal(x, y)
+        # no row ids wanted: no bits are needed either
+        st, got, _, _ = _join_under(Budget(cuda, 16 + max(inner.peak, later)), t, kind, pk, n_out, rids=False)
+        assert st == L.SJ_OK and got == want
+
+
 @pytest.mark.parametrize("kind", [L.SJ_JOIN_SEMI, L.SJ_JOIN_ANTI, L.SJ_JOIN_MARK])
 def test_refused_scratch_takes_the_pass_without(cuda, kind):
     """An allocator that refuses everything after the build: the join still runs, with the same rows."""
