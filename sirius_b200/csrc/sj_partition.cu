@@ -807,9 +807,12 @@ sj_status partition_columns(const void* keys, int key_type, int64_t n, int pbits
 // ------------------------------------------------------------------------------------------------
 // Tile-local partition (the probe side): every tile of kColTile rows is sorted by partition and written
 // back to its own rows, one column at a time through the staging buffer, in 16-byte pieces; its runs go to
-// run_off / run_cnt[p * tiles + tile]. NULL-key rows are dropped. No histogram, no scan, no write fronts.
-// 64M int64 keys and one 8-byte payload, 16 partitions: 490 us, as long as 2048-row tiles staged whole
-// (479 us), but the probe reads runs twice as long (unit probe 1,361 -> 1,300 us).
+// run_off / run_cnt[p * tiles + tile]. Rows that match nothing, those with a NULL key or one outside [kmin, kmax],
+// are dropped: they are not written and the probe does not read them. No histogram, no scan, no write fronts.
+// 64M int64 keys and one 8-byte payload, 16 partitions: 446 us, and the probe reads runs twice as long as with
+// 2048-row tiles staged whole (479 us; unit probe 1,361 -> 1,300 us). A row's partition, then its slot, then the
+// mark of a row that was dropped share a register: with a mask and a slot of their own 16 bytes spilled, and the test
+// of the range took 465 us instead of 446 (454 without the test).
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void stage_copy(const unsigned char* stage, void* dst, size_t at, uint32_t bytes) {
   uint4* d = reinterpret_cast<uint4*>(static_cast<char*>(dst) + at);
@@ -821,8 +824,9 @@ template <typename K>
 __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(const K* __restrict__ keys, bool key_pairs,
                                                                                 const uint32_t* __restrict__ kvalid,
                                                                                 int64_t kvoff, uint32_t n, int pbits,
-                                                                                uint32_t n_tiles, K* okeys, int32_t* orid,
-                                                                                PartColumns cols, int32_t* run_off,
+                                                                                uint32_t n_tiles, std::make_unsigned_t<K> kmin,
+                                                                                std::make_unsigned_t<K> span, K* okeys,
+                                                                                int32_t* orid, PartColumns cols, int32_t* run_off,
                                                                                 int32_t* run_cnt) {
   using U = std::conditional_t<sizeof(K) == 8, unsigned long long, unsigned int>;
   __shared__ __align__(16) unsigned char stage[kColTile * 8];
@@ -838,14 +842,14 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(
   for (; tile < n_tiles; tile += gridDim.x) {
     const uint32_t t0 = tile * kColTile;
     const int tile_n = (int)min(n - t0, (uint32_t)kColTile);
-    // 1. rank every valid row within its partition
-    uint32_t pr[kColRows];  // partition << 16 | rank
-    uint32_t live = 0;
+    // 1. rank every row that may match within its partition
+    uint32_t pr[kColRows];  // partition << 16 | rank, ~0 for the others
 #pragma unroll
     for (int j = 0; j < kColRows; ++j) {
       const int r = col_row(j, tid);
-      if (r >= tile_n || !bit_valid(kvalid, kvoff, (int64_t)t0 + r)) continue;
-      live |= 1u << j;
+      pr[j] = 0xffffffffu;
+      const bool in = (std::make_unsigned_t<K>)((std::make_unsigned_t<K>)v[j] - kmin) <= span;
+      if (!(in & (r < tile_n)) || !bit_valid(kvalid, kvoff, (int64_t)t0 + r)) continue;
       const uint32_t p = (uint32_t)partition_of(key_u64<K>((K)v[j]), pbits);
       pr[j] = p << 16 | atomicAdd(&tcnt[p], 1u);
     }
@@ -880,13 +884,11 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(
     }
     __syncthreads();
     // 3. the keys, the payloads, the row ids
-    uint16_t slot[kColRows];
 #pragma unroll
     for (int j = 0; j < kColRows; ++j) {
-      slot[j] = 0;
-      if (!(live >> j & 1u)) continue;
-      slot[j] = (uint16_t)(tbase[pr[j] >> 16] + (pr[j] & 0xffffu));
-      reinterpret_cast<K*>(stage)[slot[j]] = (K)v[j];
+      if (pr[j] == 0xffffffffu) continue;
+      pr[j] = tbase[pr[j] >> 16] + (pr[j] & 0xffffu);  // the sorted slot
+      reinterpret_cast<K*>(stage)[pr[j]] = (K)v[j];
     }
     __syncthreads();
     auto next = [&](int q) {
@@ -901,11 +903,11 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(
       if (w == 8) {
 #pragma unroll
         for (int j = 0; j < kColRows; ++j)
-          if (live >> j & 1u) reinterpret_cast<uint64_t*>(stage)[slot[j]] = v[j];
+          if (pr[j] < kColTile) reinterpret_cast<uint64_t*>(stage)[pr[j]] = v[j];
       } else {
 #pragma unroll
         for (int j = 0; j < kColRows; ++j)
-          if (live >> j & 1u) reinterpret_cast<uint32_t*>(stage)[slot[j]] = (uint32_t)v[j];
+          if (pr[j] < kColTile) reinterpret_cast<uint32_t*>(stage)[pr[j]] = (uint32_t)v[j];
       }
       __syncthreads();
       next(q + 1);
@@ -914,7 +916,7 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(
     }
 #pragma unroll
     for (int j = 0; j < kColRows; ++j)
-      if (live >> j & 1u) reinterpret_cast<uint32_t*>(stage)[slot[j]] = t0 + col_row(j, tid);
+      if (pr[j] < kColTile) reinterpret_cast<uint32_t*>(stage)[pr[j]] = t0 + col_row(j, tid);
     __syncthreads();
     stage_copy(stage, orid, (size_t)t0 * 4, valid * 4);
     __syncthreads();
@@ -922,8 +924,8 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(
 }
 
 // The outputs start on 16 bytes and have room for whole 16-byte pieces.
-sj_status local_partition(const PartSrc& src, int key_type, int pbits, const PartDst& dst, int32_t* run_off,
-                          int32_t* run_cnt, int device, cudaStream_t s) {
+sj_status local_partition(const PartSrc& src, int key_type, int pbits, int64_t kmin, int64_t kmax, const PartDst& dst,
+                          int32_t* run_off, int32_t* run_cnt, int device, cudaStream_t s) {
   if (!partition_plain_shape(src, dst)) return set_error(SJ_ERR_INVALID, "tile-local partition needs the plain shape");
   if (src.n == 0) return SJ_OK;
   static_assert(kColTile == kPartTileRows, "tile of the run tables");
@@ -935,9 +937,10 @@ sj_status local_partition(const PartSrc& src, int key_type, int pbits, const Par
                                   (int16_t)((uintptr_t)src.pay[c].data % (2 * src.pay[c].width) == 0)};
   auto go = [&](auto k) {
     using K = decltype(k);
+    using UK = std::make_unsigned_t<K>;
     KernelTimer timer("partition_scatter", s);
     part_local_kernel<K><<<grid, kColThreads, 0, s>>>(static_cast<const K*>(src.keys), (uintptr_t)src.keys % (2 * sizeof(K)) == 0,
-                                                      src.kvalid, src.kvoff, (uint32_t)src.n, pbits, tiles,
+                                                      src.kvalid, src.kvoff, (uint32_t)src.n, pbits, tiles, (UK)kmin, (UK)((UK)kmax - (UK)kmin),
                                                       static_cast<K*>(dst.keys), dst.rid, cols, run_off, run_cnt);
   };
   if (key_type == SJ_INT32) go(int32_t{});

@@ -750,9 +750,10 @@ static sj_status probe_partitioned(const sj_table* t, const sj_column& p, Gather
     pd.valid8[c] = g.pin[c].valid ? reinterpret_cast<uint8_t*>(carve((size_t)n)) : nullptr;
   }
   if (local) {
+    const TableDev range = table_dev(t);
     int32_t* run_off = reinterpret_cast<int32_t*>(carve(run_bytes));
     int32_t* run_cnt = reinterpret_cast<int32_t*>(carve(run_bytes));
-    SJ_TRY(local_partition(ps, t->key_type, pbits, pd, run_off, run_cnt, t->device, s));
+    SJ_TRY(local_partition(ps, t->key_type, pbits, range.kmin, range.kmax, pd, run_off, run_cnt, t->device, s));
     g.prid_map = pd.rid;
     for (int c = 0; c < g.n_pin; ++c) g.pin[c] = column_payload(pd.pay[c], nullptr, 0, g.pin[c].width);
     const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0};
@@ -791,6 +792,7 @@ sj_status probe_find(const sj_table* t, const sj_column& p, uint32_t* words, con
     Scratch sc;
     if (sc.get(alloc, align256((size_t)n * kw) + align256((size_t)n * 4) + 2 * align256(run_bytes) + 256, s) == SJ_OK) {
       char* cur = reinterpret_cast<char*>(align256(reinterpret_cast<size_t>(sc.ptr)));
+      const TableDev range = table_dev(t);
       PartSrc ps{};
       PartDst pd{};
       ps.keys = p.data;
@@ -801,7 +803,7 @@ sj_status probe_find(const sj_table* t, const sj_column& p, uint32_t* words, con
       pd.rid = reinterpret_cast<int32_t*>(cur + align256((size_t)n * kw));
       int32_t* run_off = reinterpret_cast<int32_t*>(cur + align256((size_t)n * kw) + align256((size_t)n * 4));
       int32_t* run_cnt = run_off + align256(run_bytes) / sizeof(int32_t);
-      SJ_TRY(local_partition(ps, t->key_type, pbits, pd, run_off, run_cnt, t->device, s));
+      SJ_TRY(local_partition(ps, t->key_type, pbits, range.kmin, range.kmax, pd, run_off, run_cnt, t->device, s));
       SJ_CUDA_TRY(cudaMemsetAsync(words, 0, (size_t)((n + 31) / 32) * sizeof(uint32_t), s));
       const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0};
       find_units(t, pd.keys, nullptr, 0, n, &ra, pd.rid, words, s);

@@ -157,7 +157,7 @@ struct WaitRows {
 };
 
 // Table positions (SLOT: slots) of rows first + v0 + 32 j + lane (keys k[j]) of the warp's unit, kNoPos where
-// there is none.
+// there is none. RUNS: the partition has dropped NULL keys and those outside the build's key range.
 template <typename K, bool WIDE, bool RUNS, int S, bool SLOT = false>
 __device__ __forceinline__ void unit_lookup(const TableDev& t, const K (&k)[S], const uint32_t* __restrict__ kv, int64_t kvoff,
                                             uint32_t first, uint32_t v0, uint32_t rows, WaitRows<S>& wait, uint32_t (&pos)[S]) {
@@ -174,7 +174,8 @@ __device__ __forceinline__ void unit_lookup(const TableDev& t, const K (&k)[S], 
     uint32_t b, q = 0;
     pos[j] = kNoPos;
     bool cont = false;
-    if (sector_key<K, WIDE>(t, k[j], key, b) && v < rows && (RUNS || bit_valid(kv, kvoff, first + v))) {
+    const bool in = sector_key<K, WIDE>(t, k[j], key, b);
+    if (v < rows && (RUNS || (in && bit_valid(kv, kvoff, first + v)))) {
       const Sector s = load_sector(t.slots, b);
       uint32_t p;
       if (SLOT ? Ops::find_slot(s, key, rid_mask, q) : Ops::find(s, key, rid_mask, p, q)) pos[j] = SLOT ? b * Ops::kSlots + q : p;

@@ -11,7 +11,7 @@ void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_
                  const RunArgs* runs, const DirectArgs& a, cudaStream_t s);
 
 // Bit i of `words` ((n + 31) / 32 of them): probe row i has a match in `t` (any layout). With `runs`, `keys` and
-// `prid_map` are the partitioned arrays, NULL-key rows are not in them, and `words` must be zero before.
+// `prid_map` are the partitioned arrays, rows that cannot match are not in them, and `words` must be zero before.
 void find_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t kvoff, int64_t n, const RunArgs* runs,
                 const int32_t* prid_map, uint32_t* words, cudaStream_t s);
 

@@ -52,13 +52,16 @@ def test_row_count_edges(cuda, n, types):
 
 
 @pytest.mark.parametrize("dtype,wide", [(np.int32, False), (np.int64, False), (np.int64, True)])
-def test_lookup_in_partition_order(cuda, dtype, wide):
-    """More than 64 MB of slots, and a probe that touches each sector twice or more."""
+@pytest.mark.parametrize("far", [0.0, 0.4])
+def test_lookup_in_partition_order(cuda, dtype, wide, far):
+    """More than 64 MB of slots, and a probe that touches each sector twice or more; `far` of the rows' keys lie
+    outside the build's range, on both sides, and take no part in the partition."""
     rng = np.random.default_rng(3)
     nb = (2 << 20) + 5 if wide else (5 << 20)
     bk = rng.permutation(3 * nb)[:nb].astype(dtype)
     n = 16_800_019
     pk = rng.integers(0, 3 * nb, n).astype(dtype)
+    pk = np.where(rng.random(n) < far, np.where(pk % 2, -1 - pk, 3 * nb + pk), pk).astype(dtype)
     _check(cuda, bk, pk, rng.random(n) > 0.03, [rng.integers(0, 100, n).astype(np.int32)], force_wide=wide, load_factor=0.4)
 
 

@@ -8,6 +8,7 @@ import torch
 
 from jhelp import assert_same_rows, dev_t, dev_valid, oracle_join
 from oracle import oracle as O
+from sirius_b200 import _lib as L
 from sirius_b200 import datagen as D
 from sirius_b200 import join as J
 
@@ -50,6 +51,31 @@ def test_partition_runs(cuda, n, pbits, wide):
     pv = O.pack_validity(rng.random(n) > 0.05)
     bp = [rng.integers(0, 1 << 40, nb).astype(np.int64)]
     _join(cuda, bk, pk, bp, [], pv, partition_bits=pbits, force_wide=wide, probe_partition_mb=1)
+
+
+@pytest.mark.parametrize("dtype", [np.int32, np.int64])
+@pytest.mark.parametrize("full", [False, True])
+@pytest.mark.parametrize("far", [0.4, 1.0])
+def test_partition_runs_without_keys_outside_the_range(cuda, dtype, full, far):
+    """The partition drops what lies outside the build's key range, the type's ends among it; with a build that holds
+    both ends of the type nothing lies outside."""
+    rng = np.random.default_rng(9)
+    info, nb, n = np.iinfo(dtype), 30_000, 200_003
+    bk = (rng.permutation(3 * nb)[:nb] - nb).astype(dtype)
+    if full:
+        bk[:2] = info.min, info.max
+    pk = rng.integers(-nb, 2 * nb, n).astype(dtype)
+    ends = np.array([info.min, info.min + 1, bk.min() - (not full), bk.max() + (not full), info.max - 1, info.max])
+    pk = np.where(rng.random(n) < far, rng.choice(ends.astype(dtype), n), pk)
+    pv = O.pack_validity(rng.random(n) > 0.05)
+    rows = _join(cuda, bk, pk, [rng.integers(0, 9, nb).astype(np.int64)], [rng.integers(0, 9, n).astype(np.int32)], pv,
+                 partition_bits=4)
+    assert (rows > 0) == (full or far < 1)
+    with J.HashTable(dev_t(bk, cuda), partition_bits=4) as t:
+        left = t.probe_join(L.SJ_JOIN_LEFT, dev_t(pk, cuda), dev_valid(pv, cuda))
+    prid, brid = left.probe_rid[:left.count].cpu().numpy(), left.build_rid[:left.count].cpu().numpy()
+    assert np.array_equal(np.sort(prid), np.arange(n)) and (brid >= 0).sum() == rows
+    assert np.array_equal(bk[brid[brid >= 0]], pk[prid[brid >= 0]])
 
 
 @pytest.mark.parametrize("wide", [False, True])
