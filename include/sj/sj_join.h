@@ -310,7 +310,10 @@ typedef enum sj_join_kind {
  *          probe key is NULL, or every unmatched row when the build side has a NULL key (the IN rule
  *          of resolve_mark_join_result; the table must use SJ_NULLS_UNEQUAL). *d_count = probe rows.
  * Rows beyond `capacity` are not written (*d_count still counts them). Stream-ordered. Scratch comes from
- * `alloc`; SEMI, ANTI and MARK run without any when it is refused. */
+ * `alloc`. SEMI, ANTI and MARK of a single key column of the table's type need none: they take some where
+ * slots of 256 MB or more meet tens of millions of probe rows, and do without it when it is refused or while
+ * `stream` is being captured. Composite keys are packed, and a key column of the other integer type is
+ * converted, into scratch that every kind needs. */
 SJ_EXPORT sj_status sj_probe_join(const sj_table* table, sj_join_kind kind, const sj_column* probe_keys,
                                   int32_t num_keys, const sj_column* probe_payload, int32_t num_probe_payload,
                                   const sj_column* build_payload, int32_t num_build_payload, int32_t* out_probe_rid,

@@ -196,7 +196,18 @@ sj_status probe_count(const sj_table* t, const sj_column& probe, const Allocator
 sj_status probe_gather(const sj_table* t, const sj_column& probe, const GatherSpec& g,
                        const Allocator& alloc, cudaStream_t stream, int64_t* d_count);
 
-sj_status probe_find(const sj_table* t, const sj_column& p, uint32_t* words, const Allocator& alloc, cudaStream_t s);
+// A decision that the device takes: of kSampleRows sampled probe rows (sj_units.cuh), *rows have a key in the build's
+// range. The lookup in partition order runs when there are `need` or more, the one in place otherwise; the kernels of
+// the other return at once. rows NULL: no choice, the kernel runs.
+struct RangeGate {
+  const uint32_t* rows = nullptr;
+  uint32_t need = 0;
+};
+
+// Looks the probe rows up in partition order where that may pay off, else *words stays NULL. `bits` then holds, and
+// *words points at, one bit per row with a match, if *gate is open.
+sj_status find_in_order(const sj_table* t, const sj_column& p, const Allocator& alloc, cudaStream_t s, Scratch& bits,
+                        const uint32_t** words, RangeGate* gate);
 
 sj_status validate_column(const sj_column* c, const char* what, bool key);
 

@@ -20,6 +20,7 @@
 
 #include "sj_partition.cuh"
 #include "sj_scan.cuh"
+#include "sj_units.cuh"
 
 namespace sj {
 
@@ -807,7 +808,7 @@ sj_status partition_columns(const void* keys, int key_type, int64_t n, int pbits
 // ------------------------------------------------------------------------------------------------
 // Tile-local partition (the probe side): every tile of kColTile rows is sorted by partition and written
 // back to its own rows, one column at a time through the staging buffer, in 16-byte pieces; its runs go to
-// run_off / run_cnt[p * tiles + tile]. Rows that match nothing, those with a NULL key or one outside [kmin, kmax],
+// runs.off / runs.cnt[p * tiles + tile]. Rows that match nothing, those with a NULL key or one outside [kmin, kmax],
 // are dropped: they are not written and the probe does not read them. No histogram, no scan, no write fronts.
 // 64M int64 keys and one 8-byte payload, 16 partitions: 446 us, and the probe reads runs twice as long as with
 // 2048-row tiles staged whole (479 us; unit probe 1,361 -> 1,300 us). A row's partition, then its slot, then the
@@ -826,8 +827,9 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(
                                                                                 int64_t kvoff, uint32_t n, int pbits,
                                                                                 uint32_t n_tiles, std::make_unsigned_t<K> kmin,
                                                                                 std::make_unsigned_t<K> span, K* okeys,
-                                                                                int32_t* orid, PartColumns cols, int32_t* run_off,
-                                                                                int32_t* run_cnt) {
+                                                                                int32_t* orid, PartColumns cols,
+                                                                                LocalRuns runs) {
+  if (!gate_open(runs.gate)) return;
   using U = std::conditional_t<sizeof(K) == 8, unsigned long long, unsigned int>;
   __shared__ __align__(16) unsigned char stage[kColTile * 8];
   __shared__ uint32_t s_wsum[kColThreads / 32], tcnt[1 << kMaxPartBits], tbase[1 << kMaxPartBits];
@@ -842,6 +844,7 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(
   for (; tile < n_tiles; tile += gridDim.x) {
     const uint32_t t0 = tile * kColTile;
     const int tile_n = (int)min(n - t0, (uint32_t)kColTile);
+    if (runs.zero_bits && tid * 32 < tile_n) runs.zero_bits[t0 / 32 + tid] = 0;
     // 1. rank every row that may match within its partition
     uint32_t pr[kColRows];  // partition << 16 | rank, ~0 for the others
 #pragma unroll
@@ -877,8 +880,8 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(
       if (p < P) {
         tbase[p] = run;
         tcnt[p] = 0;
-        run_off[(size_t)p * n_tiles + tile] = (int32_t)(t0 + run);
-        run_cnt[(size_t)p * n_tiles + tile] = (int32_t)c[q];
+        runs.off[(size_t)p * n_tiles + tile] = (int32_t)(t0 + run);
+        runs.cnt[(size_t)p * n_tiles + tile] = (int32_t)c[q];
       }
       run += c[q];
     }
@@ -925,7 +928,7 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_local_kernel(
 
 // The outputs start on 16 bytes and have room for whole 16-byte pieces.
 sj_status local_partition(const PartSrc& src, int key_type, int pbits, int64_t kmin, int64_t kmax, const PartDst& dst,
-                          int32_t* run_off, int32_t* run_cnt, int device, cudaStream_t s) {
+                          const LocalRuns& runs, int device, cudaStream_t s) {
   if (!partition_plain_shape(src, dst)) return set_error(SJ_ERR_INVALID, "tile-local partition needs the plain shape");
   if (src.n == 0) return SJ_OK;
   static_assert(kColTile == kPartTileRows, "tile of the run tables");
@@ -941,7 +944,7 @@ sj_status local_partition(const PartSrc& src, int key_type, int pbits, int64_t k
     KernelTimer timer("partition_scatter", s);
     part_local_kernel<K><<<grid, kColThreads, 0, s>>>(static_cast<const K*>(src.keys), (uintptr_t)src.keys % (2 * sizeof(K)) == 0,
                                                       src.kvalid, src.kvoff, (uint32_t)src.n, pbits, tiles, (UK)kmin, (UK)((UK)kmax - (UK)kmin),
-                                                      static_cast<K*>(dst.keys), dst.rid, cols, run_off, run_cnt);
+                                                      static_cast<K*>(dst.keys), dst.rid, cols, runs);
   };
   if (key_type == SJ_INT32) go(int32_t{});
   else go(int64_t{});

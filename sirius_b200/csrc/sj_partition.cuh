@@ -29,12 +29,18 @@ struct PartDst {
 
 size_t partition_scratch_bytes(int pbits, int device);
 // Tile-local variant (one pass, no histogram): each tile of kPartTileRows rows is sorted by partition
-// in place; run_off / run_cnt[p * tiles + tile] give partition p's rows of every tile. Only for
+// in place; off / cnt[p * tiles + tile] give partition p's rows of every tile. Only for
 // plain outputs with at most 2 payloads of 4/8 bytes without NULLs. Rows with a NULL key or a key outside
-// [kmin, kmax] (the table's range) are dropped.
+// [kmin, kmax] (the table's range) are dropped. zero_bits: NULL, or one bit per row to clear on the way.
 constexpr int kPartTileRows = 4096;
+struct LocalRuns {
+  int32_t* off;
+  int32_t* cnt;
+  uint32_t* zero_bits = nullptr;
+  RangeGate gate;
+};
 sj_status local_partition(const PartSrc& src, int key_type, int pbits, int64_t kmin, int64_t kmax, const PartDst& dst,
-                          int32_t* run_off, int32_t* run_cnt, int device, cudaStream_t s);
+                          const LocalRuns& runs, int device, cudaStream_t s);
 bool partition_plain_shape(const PartSrc& src, const PartDst& dst);
 
 sj_status radix_partition(const PartSrc& src, int key_type, int pbits, const PartDst& dst, void* scratch,

@@ -29,6 +29,7 @@
 #include "sj_probe_direct.h"
 #include "sj_probe_units.h"
 #include "sj_scan.cuh"
+#include "sj_units.cuh"
 
 namespace sj {
 
@@ -753,7 +754,7 @@ static sj_status probe_partitioned(const sj_table* t, const sj_column& p, Gather
     const TableDev range = table_dev(t);
     int32_t* run_off = reinterpret_cast<int32_t*>(carve(run_bytes));
     int32_t* run_cnt = reinterpret_cast<int32_t*>(carve(run_bytes));
-    SJ_TRY(local_partition(ps, t->key_type, pbits, range.kmin, range.kmax, pd, run_off, run_cnt, t->device, s));
+    SJ_TRY(local_partition(ps, t->key_type, pbits, range.kmin, range.kmax, pd, LocalRuns{run_off, run_cnt}, t->device, s));
     g.prid_map = pd.rid;
     for (int c = 0; c < g.n_pin; ++c) g.pin[c] = column_payload(pd.pay[c], nullptr, 0, g.pin[c].width);
     const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0};
@@ -774,46 +775,80 @@ static sj_status probe_partitioned(const sj_table* t, const sj_column& p, Gather
   return SJ_OK;
 }
 
-// Which probe rows have a match, as one bit per row (SEMI, ANTI, MARK). A table whose slots outgrow L2 is
-// looked up in partition order when the probe touches each of its sectors twice or more: 64M probe rows into
-// 256 MB of slots in place 1,325 us (random DRAM sectors, 55 G/s); below that the partition pass costs more
-// than the random sectors. No scratch for it: looked up in place.
-sj_status probe_find(const sj_table* t, const sj_column& p, uint32_t* words, const Allocator& alloc, cudaStream_t s) {
+// How many of kSampleRows evenly spaced probe rows have a key in the build's range.
+template <typename K>
+__global__ void __launch_bounds__(256) sample_range_kernel(TableDev t, const K* __restrict__ keys, const uint32_t* kv,
+                                                           int64_t kvoff, int64_t n, uint32_t* in_range_rows) {
+  const int64_t i = (int64_t)(blockIdx.x * blockDim.x + threadIdx.x) * n / kSampleRows;
+  const int in = __syncthreads_count(in_range(t, __ldg(keys + i)) && bit_valid(kv, kvoff, i));
+  if (threadIdx.x == 0 && in) atomicAdd(in_range_rows, (uint32_t)in);
+}
+
+// Which probe rows have a match, as one bit per row (SEMI, ANTI, MARK), in partition order. Against the lookup in
+// place (kind_units_kernel), us for SEMI of int64 keys, 70 % of the rows with a match and the others in the range:
+//   slots      16M rows        64M rows      64M, half of them out of range
+//   128 MB   237 / 326       782 / 1,024         (in place / in partition order)
+//   256 MB   312 / 334     1,102 / 1,035       713 / 790
+//   512 MB   375 / 355     1,347 / 1,072       784 / 815
+//   1 GB                   1,484 / 1,124       843 / 850
+// So: slots of 256 MB or more, 32M rows or more that touch each sector about once or more, and a key in the build's
+// range for 3/4 of the rows (1/2 from 512 MB on). The last only the device knows: a sample decides there, and what
+// runs in vain then takes about 40 us. In place, too, when the scratch is refused, and in a capture, whose graph would go on to use
+// memory that the caller's allocator has got back.
+sj_status find_in_order(const sj_table* t, const sj_column& p, const Allocator& alloc, cudaStream_t s, Scratch& bits,
+                        const uint32_t** words, RangeGate* gate) {
   SJ_TRY(check_probe(t, p));
   const int64_t n = p.num_rows;
-  constexpr size_t kFitsL2 = (size_t)64 << 20;
-  if (t->pbits > 0 && t->slots_bytes > kFitsL2 && (size_t)n * kBucketBytes >= 2 * t->slots_bytes) {
-    int pbits = 1;
-    const size_t share = (size_t)(t->params.probe_partition_mb > 0 ? t->params.probe_partition_mb : 48) << 20;
-    while (pbits < t->pbits && (t->slots_bytes >> pbits) > share) ++pbits;
-    const int kw = t->key_type == SJ_INT32 ? 4 : 8;
-    const int64_t n_tiles = (n + kPartTileRows - 1) / kPartTileRows;
-    const size_t run_bytes = (size_t)n_tiles * ((size_t)1 << pbits) * sizeof(int32_t);
-    Scratch sc;
-    if (sc.get(alloc, align256((size_t)n * kw) + align256((size_t)n * 4) + 2 * align256(run_bytes) + 256, s) == SJ_OK) {
-      char* cur = reinterpret_cast<char*>(align256(reinterpret_cast<size_t>(sc.ptr)));
-      const TableDev range = table_dev(t);
-      PartSrc ps{};
-      PartDst pd{};
-      ps.keys = p.data;
-      ps.kvalid = p.validity;
-      ps.kvoff = p.validity_offset;
-      ps.n = n;
-      pd.keys = cur;
-      pd.rid = reinterpret_cast<int32_t*>(cur + align256((size_t)n * kw));
-      int32_t* run_off = reinterpret_cast<int32_t*>(cur + align256((size_t)n * kw) + align256((size_t)n * 4));
-      int32_t* run_cnt = run_off + align256(run_bytes) / sizeof(int32_t);
-      SJ_TRY(local_partition(ps, t->key_type, pbits, range.kmin, range.kmax, pd, run_off, run_cnt, t->device, s));
-      SJ_CUDA_TRY(cudaMemsetAsync(words, 0, (size_t)((n + 31) / 32) * sizeof(uint32_t), s));
-      const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0};
-      find_units(t, pd.keys, nullptr, 0, n, &ra, pd.rid, words, s);
-      SJ_CUDA_TRY(cudaGetLastError());
-      return SJ_OK;
-    }
-    clear_error();
+  constexpr int64_t kLeast = (int64_t)256 << 20;
+  const int64_t slots = (int64_t)t->slots_bytes, sectors = n * kBucketBytes;
+  if (t->pbits == 0 || slots < kLeast || sectors < std::max(slots, 4 * kLeast)) return SJ_OK;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) {
+    cudaGetLastError();
+    return SJ_OK;
   }
-  find_units(t, p.data, p.validity, p.validity_offset, n, nullptr, nullptr, words, s);
+  if (capture != cudaStreamCaptureStatusNone) return SJ_OK;
+  int pbits = 1;
+  const size_t share = (size_t)(t->params.probe_partition_mb > 0 ? t->params.probe_partition_mb : 48) << 20;
+  while (pbits < t->pbits && (t->slots_bytes >> pbits) > share) ++pbits;
+  const int kw = t->key_type == SJ_INT32 ? 4 : 8;
+  const int64_t n_tiles = (n + kPartTileRows - 1) / kPartTileRows;
+  const size_t run_bytes = (size_t)n_tiles * ((size_t)1 << pbits) * sizeof(int32_t);
+  const size_t bit_bytes = 16 + (size_t)((n + 31) / 32) * sizeof(uint32_t);
+  Scratch sc;
+  if (bits.get(alloc, bit_bytes, s) != SJ_OK ||
+      sc.get(alloc, align256((size_t)n * kw) + align256((size_t)n * 4) + 2 * align256(run_bytes) + 256, s) != SJ_OK) {
+    clear_error();
+    return SJ_OK;
+  }
+  uint32_t* count = bits.as<uint32_t>();
+  SJ_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(uint32_t), s));
+  uint32_t* set = count + 4;
+  const TableDev d = table_dev(t);
+  KernelTimer timer("sample_range", s);
+  if (t->key_type == SJ_INT32)
+    sample_range_kernel<int32_t><<<kSampleRows / 256, 256, 0, s>>>(d, static_cast<const int32_t*>(p.data), p.validity,
+                                                                   p.validity_offset, n, count);
+  else
+    sample_range_kernel<int64_t><<<kSampleRows / 256, 256, 0, s>>>(d, static_cast<const int64_t*>(p.data), p.validity,
+                                                                   p.validity_offset, n, count);
+  char* cur = reinterpret_cast<char*>(align256(reinterpret_cast<size_t>(sc.ptr)));
+  PartSrc ps{};
+  PartDst pd{};
+  ps.keys = p.data;
+  ps.kvalid = p.validity;
+  ps.kvoff = p.validity_offset;
+  ps.n = n;
+  pd.keys = cur;
+  pd.rid = reinterpret_cast<int32_t*>(cur + align256((size_t)n * kw));
+  int32_t* run_off = reinterpret_cast<int32_t*>(cur + align256((size_t)n * kw) + align256((size_t)n * 4));
+  int32_t* run_cnt = run_off + align256(run_bytes) / sizeof(int32_t);
+  *gate = RangeGate{count, slots < 2 * kLeast ? kSampleRows / 4 * 3 : kSampleRows / 2};
+  SJ_TRY(local_partition(ps, t->key_type, pbits, d.kmin, d.kmax, pd, LocalRuns{run_off, run_cnt, set, *gate}, t->device, s));
+  const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0};
+  find_units(t, pd.keys, n, ra, pd.rid, set, *gate, s);
   SJ_CUDA_TRY(cudaGetLastError());
+  *words = set;
   return SJ_OK;
 }
 

@@ -74,9 +74,8 @@ struct SectorOps<true> {
 
 // Key of a probe row; false when it lies outside the build's key range.
 template <typename K, bool WIDE>
-__device__ __forceinline__ bool sector_key(const TableDev& t, K k, SectorKey& out, uint32_t& bucket) {
+__device__ __forceinline__ bool sector_key(const TableDev& t, K k, SectorKey& out) {
   const uint64_t kb = key_u64<K>(k);
-  bucket = home_bucket(t, kb);
   bool in;
   uint64_t kn;
   if constexpr (sizeof(K) == 4) {

@@ -3,15 +3,13 @@
 // anti_join, hash_join::left_join / full_join, distinct_hash_join::left_join — and the MARK result of
 // resolve_mark_join_result, :1461-1525).
 //
-//   SEMI / ANTI  two passes: the lookup (probe_find: a NULL key finds nothing unless NULLs compare equal
-//                and the build has NULL keys; in partition order where the table outgrows L2) leaves one
-//                bit per probe row, then the selected rows and their payloads are compacted in row order
-//                (64M x 16M rows, 30 % absent: SEMI 1,325 -> 1,115 us).
-//   MARK         the same bits, then mark byte and validity bit of every probe row. Unmatched rows are
+//   SEMI / ANTI  one pass over the probe rows: a lookup in place, and the selected rows compacted with their probe
+//                payloads (kind_units_kernel; a NULL key finds nothing unless NULLs compare equal and the build
+//                has NULL keys). No scratch. Where slots of 256 MB and more meet enough rows, the lookup runs in
+//                partition order instead (find_in_order, sj_probe.cu) and leaves one bit per probe row, and the
+//                rows are selected by them; that takes scratch, and without it the one pass remains.
+//   MARK         the same lookups: mark byte and validity bit of every probe row. Unmatched rows are
 //                NULL when their key is NULL, or all of them when the build has a NULL key.
-//                When the allocator refuses the bits, all three run as one pass over the table in place,
-//                which needs no scratch: a warp stages the selected row ids in shared memory and reserves
-//                output once per flush of about 224 rows.
 //   LEFT         the INNER probe + gather (probe_gather, any table layout), then the unmatched probe
 //                rows appended after the INNER rows on the same counter with build row id
 //                SJ_NO_ROW: the rows whose bit is clear in a mask that the unit probe sets as it looks
@@ -28,6 +26,8 @@
 
 #include "sj_device.cuh"
 #include "sj_internal.h"
+#include "sj_probe_units.h"
+#include "sj_units.cuh"
 
 namespace sj {
 
@@ -37,7 +37,7 @@ constexpr int kKindThreads = 256;
 constexpr int kKindStage = 256;  // staged row ids per warp (SEMI / ANTI rows, FULL's unmatched build rows)
 constexpr int32_t kNoRow = (int32_t)0x80000000;
 
-enum KindMode { kSemi = 0, kAnti = 1, kMark = 2, kFlags = 3, kUnmatched = 4 };
+enum KindMode { kSemi = 0, kAnti = 1, kMark = 2, kFlags = 3 };
 
 struct KindArgs {
   int32_t* out_prid;
@@ -51,124 +51,220 @@ struct KindArgs {
   uint32_t* mark_valid;
   int32_t build_has_null;
   uint8_t* flags;  // kFlags: one byte per slot (+ the NULL group)
-  const unsigned long long* inner_rows;  // kUnmatched, kFlags, select_rows: INNER rows that the match bits
+  const unsigned long long* inner_rows;  // kAnti, kFlags, select_rows: INNER rows that the match bits
                                          // were set from; past `capacity` the bits are incomplete and the
                                          // rows are looked up instead. NULL: the bits are complete
+  RangeGate gate;  // closed: looked up in place
 };
 
-// Slot of key k in the table (k in range), or -1. Slots fill each bucket in order, so the walk stops
-// after the first bucket that has an EMPTY slot.
-template <typename K, bool WIDE>
-__device__ __forceinline__ int64_t find_slot(const TableDev& t, K k) {
-  using Ops = SlotOps<WIDE>;
-  const uint64_t kb = key_u64<K>(k);
-  uint32_t b = home_bucket(t, kb);
-  const uint64_t kmask = ~((1ull << t.rbits) - 1);
-  const uint64_t ks = Ops::probe_key((uint64_t)(long long)k - (uint64_t)t.kmin, kb, t.rbits);
-  for (uint32_t step = 0; step <= t.segmask; ++step) {
-    const Bucket bk = load_bucket<true>(t.slots, b);
-    bool open = false;
+// Rows written by the warps of a CTA to consecutive output positions: one reservation for all of them. `cnt`: the
+// warp's rows; `part`, in shared memory, keeps the warps' counts. Returns the warp's first position.
+__device__ __forceinline__ unsigned long long cta_reserve(uint32_t cnt, uint32_t (&part)[kUnitWarps],
+                                                          unsigned long long& base, unsigned long long* d_count) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) part[warp] = cnt;
+  __syncthreads();
+  const uint32_t c = lane < kUnitWarps ? part[lane] : 0;
+  const uint32_t incl = warp_inclusive_sum(c);
+  const uint32_t mine = __shfl_sync(kFullMask, incl - c, warp);
+  if (warp == 0 && lane == kUnitWarps - 1) base = incl ? atomicAdd(d_count, (unsigned long long)incl) : 0ull;
+  __syncthreads();
+  return base + mine;
+}
+
+// Rows that fit behind position `base`.
+__device__ __forceinline__ uint32_t rows_left(int64_t capacity, int64_t base) {
+  const int64_t left = capacity - base;
+  return left <= 0 ? 0u : left > 0x7fffffff ? 0x7fffffffu : (uint32_t)left;
+}
+
+// Validity bits of the lanes with `on`, whose rows went to consecutive positions. Called by the whole warp.
+__device__ __forceinline__ void set_out_bits(uint32_t* valid, uint32_t pos, bool on, bool bit) {
+  const unsigned any = __ballot_sync(kFullMask, on);
+  if (!any) return;
+  const uint32_t word0 = __shfl_sync(kFullMask, pos, __ffs(any) - 1) >> 5;
+  const bool low = (pos >> 5) == word0;
+  const uint32_t b = on && bit ? 1u << (pos & 31) : 0u;
+  const uint32_t w0 = __reduce_or_sync(kFullMask, low ? b : 0u), w1 = __reduce_or_sync(kFullMask, low ? 0u : b);
+  if ((threadIdx.x & 31) == 0) {
+    if (w0) atomicOr(valid + word0, w0);
+    if (w1) atomicOr(valid + word0 + 1, w1);
+  }
+}
+
+// Payload values of N probe rows of the lane, and their stores: all loads of a column are in flight together.
+template <int N>
+__device__ __forceinline__ void load_rows(const PayloadIn& in, const uint32_t (&row)[N], uint32_t sel, uint64_t (&v)[N]) {
+  auto go = [&](auto x) {
+    using T = decltype(x);
 #pragma unroll
-    for (int q = 0; q < Ops::kSlots; ++q) {
-      if (Ops::match_s(bk, q, ks, kmask)) return (int64_t)b * Ops::kSlots + q;
-      open |= Ops::empty(bk, q);
-    }
-    if (open) return -1;
-    b = next_bucket(b, t.segmask);
-  }
-  return -1;
-}
-
-__device__ __forceinline__ bool group_nonempty(const TableDev& t, int64_t s) {
-  return t.grp_off == nullptr || __ldg(t.grp_off + s + 1) > __ldg(t.grp_off + s);
-}
-
-// The slot (group) a probe row matches, or -1.
-template <typename K, bool WIDE>
-__device__ __forceinline__ int64_t lookup(const TableDev& t, K k, bool valid) {
-  if (!valid) return t.null_group >= 0 && group_nonempty(t, t.null_group) ? (int64_t)t.null_group : -1;
-  if (!in_range(t, k)) return -1;
-  const int64_t s = find_slot<K, WIDE>(t, k);
-  return s >= 0 && group_nonempty(t, s) ? s : -1;
-}
-
-template <typename K, bool WIDE, int MODE>
-__global__ void __launch_bounds__(kKindThreads) kind_probe_kernel(TableDev t, const K* __restrict__ keys,
-                                                                  const uint32_t* __restrict__ kv, int64_t kvoff,
-                                                                  int64_t n, KindArgs a) {
-  const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << lane) - 1u;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  __shared__ int32_t s_stage[kKindThreads / 32][kKindStage];
-  int32_t* st = s_stage[threadIdx.x >> 5];
-  uint32_t fill = 0;  // staged rows of this warp (warp-uniform)
-  if (MODE == kUnmatched && (int64_t)*a.inner_rows <= a.capacity) return;  // emitted by their bits
-  // FULL flags pass: not needed when the build-row bits of the INNER rows are complete
-  if (MODE == kFlags && a.inner_rows && (int64_t)*a.inner_rows <= a.capacity) return;
-  // reserve the staged rows' output range with one atomicAdd and write them out in order
-  auto flush = [&]() {
-    __syncwarp();
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(a.d_count, (unsigned long long)fill);
-    base = __shfl_sync(kFullMask, base, 0);
-    for (uint32_t e = lane; e < fill; e += 32) {
-      const int64_t p = (int64_t)base + e;
-      if (p >= a.capacity) break;
-      const int64_t i = st[e];
-      if (a.out_prid) a.out_prid[p] = (int32_t)i;
-      if (a.out_brid) a.out_brid[p] = kNoRow;
-      for (int c = 0; c < a.n_pin; ++c) {
-        store_elem(a.pout[c].data, p, a.pin[c].width, pl_load(a.pin[c], i));
-        if (a.pout[c].valid && payload_valid(a.pin[c], i)) set_out_bit(a.pout[c].valid, p);
-      }
-    }
-    __syncwarp();
-    fill = 0;
+    for (int j = 0; j < N; ++j) v[j] = (sel >> j & 1u) ? (uint64_t)__ldcs(static_cast<const T*>(in.data) + row[j]) : 0ull;
   };
-  for (int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll; i0 < n; i0 += stride) {
-    const int64_t i = i0 + lane;
-    const bool live = i < n;
-    int64_t s = -1;
-    const bool valid = live && bit_valid(kv, kvoff, i);
-    if (live) s = lookup<K, WIDE>(t, __ldg(keys + i), valid);
-    const bool found = s >= 0;
-    if (MODE == kMark) {
-      if (live) a.mark[i] = found ? 1 : 0;
-      if (a.mark_valid) {
-        const unsigned w = __ballot_sync(kFullMask, live && (found || (!a.build_has_null && valid)));
-        if (lane == 0) a.mark_valid[i0 >> 5] = w;
-      }
-      continue;
-    }
-    if (MODE == kFlags) {
-      if (found) a.flags[s] = 1;
-      continue;
-    }
-    const bool sel = live && (MODE == kSemi ? found : !found);  // kAnti / kUnmatched: the rest
-    const unsigned bal = __ballot_sync(kFullMask, sel);
-    if (!bal) continue;
-    if (sel) st[fill + __popc(bal & below)] = (int32_t)i;
-    fill += __popc(bal);
-    if (fill > (uint32_t)(kKindStage - 32)) flush();  // the next step could not fit
+  switch (in.width) {
+    case 8: return go((unsigned long long)0);
+    case 4: return go((unsigned int)0);
+    case 2: return go((unsigned short)0);
+    default: return go((unsigned char)0);
   }
-  if (MODE == kSemi || MODE == kAnti || MODE == kUnmatched)
-    if (fill) flush();
+}
+template <int N>
+__device__ __forceinline__ void store_rows(void* out, int width, int64_t base, const uint32_t (&at)[N], uint32_t sel,
+                                           const uint64_t (&v)[N]) {
+  auto go = [&](auto x) {
+    using T = decltype(x);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (sel >> j & 1u) __stcs(static_cast<T*>(out) + base + at[j], (T)v[j]);
+  };
+  switch (width) {
+    case 8: return go((unsigned long long)0);
+    case 4: return go((unsigned int)0);
+    case 2: return go((unsigned short)0);
+    default: return go((unsigned char)0);
+  }
+}
+
+// Writes the lane's rows row[j] (bit j of `sel`) to the positions base + at[j]: row ids and probe payloads. The j-th
+// rows of a warp go to consecutive positions.
+template <int N>
+__device__ __forceinline__ void emit_rows(const KindArgs& a, const uint32_t (&row)[N], int64_t base, const uint32_t (&at)[N],
+                                          uint32_t sel) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if (!(sel >> j & 1u)) continue;
+    if (a.out_prid) __stcs(a.out_prid + base + at[j], (int32_t)row[j]);
+    if (a.out_brid) __stcs(a.out_brid + base + at[j], kNoRow);
+  }
+  for (int c = 0; c < a.n_pin; ++c) {
+    uint64_t v[N];
+    load_rows<N>(a.pin[c], row, sel, v);
+    store_rows<N>(a.pout[c].data, a.pin[c].width, base, at, sel, v);
+    if (!a.pout[c].valid) continue;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const bool on = sel >> j & 1u;
+      set_out_bits(a.pout[c].valid + (base >> 5), (uint32_t)(base & 31) + at[j], on, on && payload_valid(a.pin[c], row[j]));
+    }
+  }
+}
+
+// Mark bytes of 32 * S rows from `row0` on, word j of `found` for 32 of them: four bytes per lane where the rows are
+// whole and the bytes aligned.
+template <int S>
+__device__ __forceinline__ void mark_bytes(uint8_t* mark, const unsigned (&found)[S], uint32_t rows) {
+  const int lane = threadIdx.x & 31;
+  if (rows == 32u * S && ((uintptr_t)mark & 3) == 0) {
+    unsigned w = found[0];
+#pragma unroll
+    for (int j = 1; j < S; ++j) w = lane >> 3 == j ? found[j] : w;
+    const uint32_t x = w >> (4 * (lane & 7)) & 0xfu;
+    if (lane < 8 * S) reinterpret_cast<uint32_t*>(mark)[lane] = (x & 1u) | (x & 2u) << 7 | (x & 4u) << 14 | (x & 8u) << 21;
+  } else {
+#pragma unroll
+    for (int j = 0; j < S; ++j)
+      if (32u * j + lane < rows) mark[32 * j + lane] = found[j] >> lane & 1u;
+  }
+}
+
+// SEMI, ANTI (and the unmatched probe rows of LEFT and FULL), MARK, and FULL's flags of matched slots in one pass, the
+// table looked up in place, in units of 32 * S rows: no scratch and no bits. A CTA reserves once for its rows and
+// writes them in order, payload column after payload column.
+// It is bound by instructions while the table is in L2, so 64 warps per SM and short code: us for 64M int64 keys into
+// 4M / 16M keys, 80 % in the build: SEMI with an 8-byte payload 653 / 1,277, MARK 452 / 1,130 (one 64-bit lookup per
+// lane and 32-row step, matches staged per warp: 901 / 1,390 and 727 / 1,261; match bits, then a pass over them: 686
+// and 477 / -). With 48 warps: 706 / 1,250 and 512 / 1,069. NULLS: the probe keys have NULLs (apart, since the test for
+// the bitmask alone took 38 of 387 us of a MARK). Where all of a unit lies outside the build's range nothing is looked
+// up (64M rows, SEMI 277 -> 127 us); MARK, for which it cost 4 %, does not ask. BLOCKS: consecutive blocks of units per
+// CTA, for a launch that may have nothing to do (64K CTAs that return at once take 37 us).
+template <typename K, bool WIDE, int MODE, int S, bool NULLS, int BLOCKS>
+__global__ void __launch_bounds__(kUnitThreads, 8) kind_units_kernel(TableDev t, const K* __restrict__ keys,
+                                                                     const uint32_t* __restrict__ kv_in, int64_t kvoff,
+                                                                     uint32_t n, KindArgs a) {
+  __shared__ WaitRows<S> s_wait[kUnitWarps];
+  __shared__ uint32_t s_cnt[kUnitWarps];
+  __shared__ unsigned long long s_base;
+  // the match bits are complete: the rows are emitted, the build rows found by them
+  if ((MODE == kAnti || MODE == kFlags) && a.inner_rows && (int64_t)*a.inner_rows <= a.capacity) return;
+  if (BLOCKS > 1 && gate_open(a.gate)) return;  // looked up in partition order
+  const uint32_t* kv = NULLS ? kv_in : nullptr;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool null_found = NULLS && t.null_group >= 0 && __ldg(t.grp_off + t.null_group + 1) > __ldg(t.grp_off + t.null_group);
+  for (uint32_t block = 0; block < BLOCKS; ++block) {
+    uint32_t first, rows;
+    unit_rows<false, S>(RunArgs{}, Units{0, (blockIdx.x * BLOCKS + block) * kUnitWarps}, n, first, rows);
+    K k[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) k[j] = 32 * j + lane < rows ? __ldcs(keys + first + 32 * j + lane) : (K)0;
+    uint32_t pos[S];
+    bool any = true;
+    if constexpr (MODE == kSemi || MODE == kAnti) {  // where the whole unit lies outside the build's range, that is all there is to do
+      any = false;
+#pragma unroll
+      for (int j = 0; j < S; ++j) {
+        SectorKey key;
+        any |= sector_key<K, WIDE>(t, k[j], key);
+        pos[j] = kNoPos;
+      }
+      any = __any_sync(kFullMask, any);
+    }
+    if (any) unit_lookup<K, WIDE, false, S, MODE == kFlags>(t, k, kv, kvoff, first, 0, rows, s_wait[warp], pos);
+    unsigned found[S], known[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const uint32_t v = 32 * j + lane;
+      const bool null = NULLS && v < rows && (null_found || MODE == kMark) && !bit_valid(kv, kvoff, first + v);
+      if (MODE == kFlags) {
+        if (null) pos[j] = (uint32_t)t.null_group;
+        if (pos[j] != kNoPos) a.flags[pos[j]] = 1;
+        continue;
+      }
+      found[j] = __ballot_sync(kFullMask, pos[j] != kNoPos || (null && null_found));
+      if (MODE == kMark) known[j] = NULLS ? ~__ballot_sync(kFullMask, null) : kFullMask;
+      if (MODE == kAnti) found[j] = __ballot_sync(kFullMask, v < rows) & ~found[j];
+    }
+    if (MODE == kMark && rows > 0) {
+      mark_bytes<S>(a.mark + first, found, rows);
+      if (a.mark_valid && 32u * lane < rows) {
+        unsigned w = 0;
+#pragma unroll
+        for (int j = 0; j < S; ++j) w = lane == j ? found[j] | (a.build_has_null ? 0u : known[j]) : w;
+        const uint32_t left = rows - 32 * lane;
+        a.mark_valid[(first >> 5) + lane] = left >= 32 ? w : w & ((1u << left) - 1u);
+      }
+    }
+    if constexpr (MODE == kSemi || MODE == kAnti) {
+      uint32_t cnt = 0;
+#pragma unroll
+      for (int j = 0; j < S; ++j) cnt += __popc(found[j]);
+      const int64_t base = (int64_t)cta_reserve(cnt, s_cnt, s_base, a.d_count);
+      if (cnt == 0) continue;
+      const uint32_t room = rows_left(a.capacity, base);
+      uint32_t row[S], at[S], run = 0, sel = 0;
+#pragma unroll
+      for (int j = 0; j < S; ++j) {
+        row[j] = first + 32 * j + lane;
+        at[j] = run + __popc(found[j] & ((1u << lane) - 1u));
+        run += __popc(found[j]);
+        if ((found[j] >> lane & 1u) && at[j] < room) sel |= 1u << j;
+      }
+      emit_rows<S>(a, row, base, at, sel);
+    }
+  }
 }
 
 // Emits the probe rows whose bit in `words` is set (WANT) or clear, with their probe payloads. A warp takes 1024
 // rows, one word per lane; a CTA reserves once for its 8192 rows, and the words' rows go to consecutive
 // positions, so rows, payload loads and stores stay in order. 64M rows, 70 % of them with an 8-byte payload:
 // 213 us (5.0 TB/s), 254 with one word at a time.
-constexpr int kSelectWarps = kKindThreads / 32;
-
 template <bool WANT>
-__global__ void __launch_bounds__(kKindThreads) select_rows_kernel(const uint32_t* __restrict__ words, uint32_t n, KindArgs a) {
-  if (a.inner_rows && (int64_t)*a.inner_rows > a.capacity) return;  // the bits are incomplete
-  __shared__ uint32_t s_cnt[kSelectWarps];
+__global__ void __launch_bounds__(kUnitThreads) select_rows_kernel(const uint32_t* __restrict__ words, uint32_t n, KindArgs a) {
+  __shared__ uint32_t s_cnt[kUnitWarps];
   __shared__ unsigned long long s_base;
+  if (a.inner_rows && (int64_t)*a.inner_rows > a.capacity) return;  // the bits are incomplete
+  if (!gate_open(a.gate)) return;                                   // not set: looked up in place
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
-  const uint32_t word0 = (blockIdx.x * kSelectWarps + warp) * 32;
+  const uint32_t word0 = (blockIdx.x * kUnitWarps + warp) * 32;
   const uint32_t row0 = (word0 + lane) * 32;
   uint32_t w = 0;
   if (row0 < n) {
@@ -177,49 +273,20 @@ __global__ void __launch_bounds__(kKindThreads) select_rows_kernel(const uint32_
     if (n - row0 < 32) w &= (1u << (n - row0)) - 1u;
   }
   const uint32_t incl = warp_inclusive_sum(__popc(w));
-  if (lane == 31) s_cnt[warp] = incl;
-  __syncthreads();
-  const uint32_t c = lane < kSelectWarps ? s_cnt[lane] : 0;
-  const uint32_t all = warp_inclusive_sum(c);
-  const uint32_t mine = __shfl_sync(kFullMask, all - c, warp);
-  if (warp == 0 && lane == kSelectWarps - 1) s_base = all ? atomicAdd(a.d_count, (unsigned long long)all) : 0ull;
-  __syncthreads();
-  const int64_t base = (int64_t)s_base + mine;
-  const uint32_t at = incl - __popc(w);
-  constexpr int B = 8;  // words at a time: their first payload loads are in flight together
-  const PayloadIn in = a.pin[0];
-  const bool one = a.n_pin > 0 && !a.pout[0].valid && (in.width == 8 || in.width == 4);
+  const int64_t base = (int64_t)cta_reserve(__shfl_sync(kFullMask, incl, 31), s_cnt, s_base, a.d_count);
+  const uint32_t mine = incl - __popc(w);
+  const uint32_t room = rows_left(a.capacity, base);
+  constexpr int B = 8;  // words at a time
   for (int q0 = 0; q0 < 32; q0 += B) {
-    uint64_t v[B];
-    int64_t p[B];
-    uint32_t sel = 0;
+    uint32_t row[B], at[B], sel = 0;
 #pragma unroll
     for (int h = 0; h < B; ++h) {
       const uint32_t wq = __shfl_sync(kFullMask, w, q0 + h);
-      p[h] = base + __shfl_sync(kFullMask, at, q0 + h) + __popc(wq & below);
-      v[h] = 0;
-      if (!(wq >> lane & 1u) || p[h] >= a.capacity) continue;
-      sel |= 1u << h;
-      const uint32_t i = (word0 + q0 + h) * 32 + lane;
-      if (one)
-        v[h] = in.width == 8 ? (uint64_t)__ldcs(static_cast<const unsigned long long*>(in.data) + i)
-                             : (uint64_t)__ldcs(static_cast<const unsigned int*>(in.data) + i);
+      row[h] = (word0 + q0 + h) * 32 + lane;
+      at[h] = __shfl_sync(kFullMask, mine, q0 + h) + __popc(wq & below);
+      if ((wq >> lane & 1u) && at[h] < room) sel |= 1u << h;
     }
-#pragma unroll
-    for (int h = 0; h < B; ++h) {
-      if (!(sel >> h & 1u)) continue;
-      const uint32_t i = (word0 + q0 + h) * 32 + lane;
-      if (a.out_prid) __stcs(a.out_prid + p[h], (int32_t)i);
-      if (a.out_brid) __stcs(a.out_brid + p[h], kNoRow);
-      if (one) {
-        if (in.width == 8) __stcs(static_cast<unsigned long long*>(a.pout[0].data) + p[h], (unsigned long long)v[h]);
-        else __stcs(static_cast<unsigned int*>(a.pout[0].data) + p[h], (unsigned int)v[h]);
-      }
-      for (int k = one ? 1 : 0; k < a.n_pin; ++k) {
-        store_elem_cs(a.pout[k].data, p[h], a.pin[k].width, pl_load(a.pin[k], i));
-        if (a.pout[k].valid && payload_valid(a.pin[k], i)) set_out_bit(a.pout[k].valid, p[h]);
-      }
-    }
+    emit_rows<B>(a, row, base, at, sel);
   }
 }
 
@@ -228,7 +295,7 @@ __global__ void __launch_bounds__(kKindThreads) select_rows_kernel(const uint32_
 __global__ void __launch_bounds__(kKindThreads) mark_rows_kernel(const uint32_t* __restrict__ words, const uint32_t* __restrict__ kv,
                                                                  int64_t kvoff, int64_t n, KindArgs a) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, row0 = q * 32;
-  if (row0 >= n) return;
+  if (row0 >= n || !gate_open(a.gate)) return;
   const uint32_t w = __ldg(words + q);
   const int rows = (int)(n - row0 < 32 ? n - row0 : 32);
   uint8_t* out = a.mark + row0;
@@ -443,25 +510,43 @@ static int kind_grid(const sj_table* t, int64_t n) {
 
 template <int MODE>
 static void launch_kind(const sj_table* t, const sj_column& p, const KindArgs& a, cudaStream_t s) {
-  const int grid = kind_grid(t, p.num_rows);
-  const TableDev d = table_dev(t);
+  constexpr int kBlocks = 4;
+  const bool gated = MODE != kFlags && a.gate.rows, few = MODE != kFlags && !gated && p.num_rows <= kFewRows;
+  const int64_t per_cta = (few ? 32 : 128) * kUnitWarps * (gated ? kBlocks : 1);
+  const int grid = (int)((p.num_rows + per_cta - 1) / per_cta);
   const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
+  const TableDev d = table_dev(t);
   KernelTimer timer(MODE == kMark ? "mark" : MODE == kFlags ? "match_flags" : MODE == kSemi ? "semi"
-                    : MODE == kUnmatched ? "unmatched_probe" : "anti", s);
+                    : a.inner_rows ? "unmatched_probe" : "anti", s);
+  auto go = [&](auto k, auto w) {
+    using K = decltype(k);
+    constexpr bool W = decltype(w)::value;
+    auto launch = [&](auto kernel) {
+      kernel<<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(p.data), p.validity, p.validity_offset,
+                                           (uint32_t)p.num_rows, a);
+    };
+    if constexpr (MODE == kFlags) {
+      launch(kind_units_kernel<K, W, MODE, 4, true, 1>);
+    } else {
+      if (gated) launch(p.validity ? kind_units_kernel<K, W, MODE, 4, true, kBlocks> : kind_units_kernel<K, W, MODE, 4, false, kBlocks>);
+      else if (p.validity) launch(few ? kind_units_kernel<K, W, MODE, 1, true, 1> : kind_units_kernel<K, W, MODE, 4, true, 1>);
+      else launch(few ? kind_units_kernel<K, W, MODE, 1, false, 1> : kind_units_kernel<K, W, MODE, 4, false, 1>);
+    }
+  };
   if (t->key_type == SJ_INT32) {
-    if (wide) kind_probe_kernel<int32_t, true, MODE><<<grid, kKindThreads, 0, s>>>(d, static_cast<const int32_t*>(p.data), p.validity, p.validity_offset, p.num_rows, a);
-    else kind_probe_kernel<int32_t, false, MODE><<<grid, kKindThreads, 0, s>>>(d, static_cast<const int32_t*>(p.data), p.validity, p.validity_offset, p.num_rows, a);
+    if (wide) go(int32_t{}, std::true_type{});
+    else go(int32_t{}, std::false_type{});
   } else {
-    if (wide) kind_probe_kernel<int64_t, true, MODE><<<grid, kKindThreads, 0, s>>>(d, static_cast<const int64_t*>(p.data), p.validity, p.validity_offset, p.num_rows, a);
-    else kind_probe_kernel<int64_t, false, MODE><<<grid, kKindThreads, 0, s>>>(d, static_cast<const int64_t*>(p.data), p.validity, p.validity_offset, p.num_rows, a);
+    if (wide) go(int64_t{}, std::true_type{});
+    else go(int64_t{}, std::false_type{});
   }
 }
 
 template <bool WANT>
 static void launch_select(const uint32_t* words, int64_t n, const KindArgs& a, cudaStream_t s) {
   KernelTimer timer("select_rows", s);
-  const int64_t per_cta = (int64_t)kSelectWarps * 1024;
-  select_rows_kernel<WANT><<<(int)((n + per_cta - 1) / per_cta), kKindThreads, 0, s>>>(words, (uint32_t)n, a);
+  const int64_t per_cta = (int64_t)kUnitWarps * 1024;
+  select_rows_kernel<WANT><<<(int)((n + per_cta - 1) / per_cta), kUnitThreads, 0, s>>>(words, (uint32_t)n, a);
 }
 
 static sj_status probe_payloads(const sj_column& p, const GatherSpec& gs, KindArgs& a) {
@@ -492,18 +577,6 @@ static sj_status zero_validity(const sj_mut_column* outs, int n, int64_t capacit
   return SJ_OK;
 }
 
-// Scratch for one bit per probe row. False: the join takes the one pass that needs none, because the allocator
-// refuses, or because the probe is small: a second launch and an allocation cost more than the better lookup gains
-// (SEMI of 14K rows 46 / 69 us, ANTI of 1.9M rows 72 / 83, of 8.5M rows 124 / 130, MARK of 19M rows 191 / 166, one
-// pass / two passes).
-constexpr int64_t kMinMatchBits = 16 << 20;
-static bool match_bits(int64_t n, const Allocator& alloc, cudaStream_t s, Scratch& bits) {
-  if (n < kMinMatchBits) return false;
-  if (bits.get(alloc, (size_t)((n + 31) / 32) * sizeof(uint32_t), s) == SJ_OK) return true;
-  clear_error();
-  return false;
-}
-
 sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const GatherSpec& gs, uint8_t* out_mark,
                      uint32_t* out_mark_valid, const Allocator& alloc, cudaStream_t s, int64_t* d_count) {
   if (kind == SJ_JOIN_INNER) return probe_gather(t, p, gs, alloc, s, d_count);
@@ -525,15 +598,15 @@ sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const 
     a.build_has_null = t->null_rows > 0;
     set_count_kernel<<<1, 1, 0, s>>>(d_count, p.num_rows);
     Scratch bits;
-    if (p.num_rows > 0 && match_bits(p.num_rows, alloc, s, bits)) {
-      SJ_TRY(probe_find(t, p, bits.as<uint32_t>(), alloc, s));
-      const int64_t words = (p.num_rows + 31) / 32;
+    const uint32_t* words = nullptr;
+    SJ_TRY(find_in_order(t, p, alloc, s, bits, &words, &a.gate));
+    if (words) {
+      const int64_t n_words = (p.num_rows + 31) / 32;
       KernelTimer timer("mark_rows", s);
-      mark_rows_kernel<<<(int)((words + kKindThreads - 1) / kKindThreads), kKindThreads, 0, s>>>(
-          bits.as<uint32_t>(), p.validity, p.validity_offset, p.num_rows, a);
-    } else if (p.num_rows > 0) {
-      launch_kind<kMark>(t, p, a, s);
+      mark_rows_kernel<<<(int)((n_words + kKindThreads - 1) / kKindThreads), kKindThreads, 0, s>>>(
+          words, p.validity, p.validity_offset, p.num_rows, a);
     }
+    if (p.num_rows > 0) launch_kind<kMark>(t, p, a, s);
     SJ_CUDA_TRY(cudaGetLastError());
     return SJ_OK;
   }
@@ -543,11 +616,13 @@ sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const 
     SJ_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(int64_t), s));
     SJ_TRY(zero_validity(gs.out_probe_payload, gs.n_probe_payload, gs.capacity, s));
     Scratch bits;
-    if (p.num_rows > 0 && match_bits(p.num_rows, alloc, s, bits)) {
-      SJ_TRY(probe_find(t, p, bits.as<uint32_t>(), alloc, s));
-      if (kind == SJ_JOIN_SEMI) launch_select<true>(bits.as<uint32_t>(), p.num_rows, a, s);
-      else launch_select<false>(bits.as<uint32_t>(), p.num_rows, a, s);
-    } else if (p.num_rows > 0) {
+    const uint32_t* words = nullptr;
+    SJ_TRY(find_in_order(t, p, alloc, s, bits, &words, &a.gate));
+    if (words) {
+      if (kind == SJ_JOIN_SEMI) launch_select<true>(words, p.num_rows, a, s);
+      else launch_select<false>(words, p.num_rows, a, s);
+    }
+    if (p.num_rows > 0) {
       if (kind == SJ_JOIN_SEMI) launch_kind<kSemi>(t, p, a, s);
       else launch_kind<kAnti>(t, p, a, s);
     }
@@ -621,7 +696,7 @@ sj_status probe_join(const sj_table* t, int32_t kind, const sj_column& p, const 
       }
       a.inner_rows = m;
       launch_select<false>(mbits.as<uint32_t>(), p.num_rows, a, s);
-      launch_kind<kUnmatched>(t, p, a, s);
+      launch_kind<kAnti>(t, p, a, s);
     } else {
       launch_kind<kAnti>(t, p, a, s);
     }

@@ -18,15 +18,12 @@
 
 #include "sj_internal.h"
 #include "sj_partition.cuh"
-#include "sj_probe_core.cuh"
 #include "sj_probe_units.h"
+#include "sj_units.cuh"
 
 namespace sj {
 
 TableDev table_dev(const sj_table* t);
-
-constexpr int kUnitThreads = 256;
-constexpr int kUnitWarps = kUnitThreads / 32;
 
 __device__ __forceinline__ uint64_t ld_col(const void* base, uint32_t i, int w) {
   return w == 8 ? (uint64_t)__ldcs(static_cast<const unsigned long long*>(base) + i)
@@ -113,114 +110,7 @@ __device__ __forceinline__ void emit_match(const DirectArgs& a, uint32_t row, in
            ld_at(static_cast<const char*>(a.bin[c]) + (int64_t)(a.bin_by_pos ? (int32_t)pos : brid) * a.bin_stride[c], a.bin_w[c]));
 }
 
-constexpr uint32_t kNoPos = 0xffffffffu;
 constexpr int kUnitCtasPerSm = 6;  // 40 registers
-
-struct Units {
-  uint32_t part, first;  // RUNS: the CTA's partition; its first unit (piece of a run)
-};
-
-template <bool RUNS>
-__device__ __forceinline__ Units cta_units(const RunArgs& ra) {
-  Units u{0, blockIdx.x * kUnitWarps};
-  if constexpr (RUNS) {
-    const uint32_t ctas = ((ra.n_tiles << ra.log2_pieces) + kUnitWarps - 1) / kUnitWarps;
-    u.part = blockIdx.x / ctas;
-    u.first = (blockIdx.x - u.part * ctas) * kUnitWarps;
-  }
-  return u;
-}
-
-// First row and rows of the warp's unit.
-template <bool RUNS, int S>
-__device__ __forceinline__ void unit_rows(const RunArgs& ra, const Units& u, uint32_t n, uint32_t& first, uint32_t& rows) {
-  const uint32_t unit = u.first + (threadIdx.x >> 5);
-  first = rows = 0;
-  if constexpr (RUNS) {
-    const uint32_t tile = unit >> ra.log2_pieces, piece = unit & ((1u << ra.log2_pieces) - 1u);
-    if (tile >= ra.n_tiles) return;
-    const size_t at = (size_t)u.part * ra.n_tiles + tile;
-    const uint32_t cnt = (uint32_t)__ldg(ra.run_cnt + at), lo = cnt * piece >> ra.log2_pieces;
-    first = (uint32_t)__ldg(ra.run_off + at) + lo;
-    rows = (cnt * (piece + 1) >> ra.log2_pieces) - lo;
-  } else {
-    first = unit * (32 * S);
-    rows = first < n ? min(32u * S, n - first) : 0;
-  }
-}
-
-// A warp's rows that go on past their home bucket.
-template <int S>
-struct WaitRows {
-  SectorKey key[32 * S];
-  uint32_t bucket[32 * S];  // then the row's position
-};
-
-// Table positions (SLOT: slots) of rows first + v0 + 32 j + lane (keys k[j]) of the warp's unit, kNoPos where
-// there is none. RUNS: the partition has dropped NULL keys and those outside the build's key range.
-template <typename K, bool WIDE, bool RUNS, int S, bool SLOT = false>
-__device__ __forceinline__ void unit_lookup(const TableDev& t, const K (&k)[S], const uint32_t* __restrict__ kv, int64_t kvoff,
-                                            uint32_t first, uint32_t v0, uint32_t rows, WaitRows<S>& wait, uint32_t (&pos)[S]) {
-  using Ops = SectorOps<WIDE>;
-  const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << lane) - 1u;
-  const uint32_t rid_mask = (1u << t.rbits) - 1u;
-  uint32_t n_wait = 0;
-  uint32_t waits = 0;  // byte j: 1 + place in the list of the lane's row j, or 0
-#pragma unroll
-  for (int j = 0; j < S; ++j) {
-    const uint32_t v = v0 + 32 * j + lane;
-    SectorKey key;
-    uint32_t b, q = 0;
-    pos[j] = kNoPos;
-    bool cont = false;
-    const bool in = sector_key<K, WIDE>(t, k[j], key, b);
-    if (v < rows && (RUNS || (in && bit_valid(kv, kvoff, first + v)))) {
-      const Sector s = load_sector(t.slots, b);
-      uint32_t p;
-      if (SLOT ? Ops::find_slot(s, key, rid_mask, q) : Ops::find(s, key, rid_mask, p, q)) pos[j] = SLOT ? b * Ops::kSlots + q : p;
-      else cont = t.segmask != 0 && !Ops::open(s);
-    }
-    const unsigned bal = __ballot_sync(kFullMask, cont);
-    if (bal) {
-      if (cont) {
-        const uint32_t e = n_wait + __popc(bal & below);
-        wait.key[e] = key;
-        wait.bucket[e] = next_bucket(b, t.segmask);
-        waits |= (e + 1) << (8 * j);
-      }
-      n_wait += __popc(bal);
-    }
-  }
-  if (n_wait) {
-    __syncwarp();
-    for (uint32_t e0 = 0; e0 < n_wait; e0 += 32) {
-      const uint32_t e = e0 + lane;
-      bool act = e < n_wait;
-      SectorKey key{};
-      uint32_t b = 0, res = kNoPos;
-      if (act) {
-        key = wait.key[e];
-        b = wait.bucket[e];
-      }
-      for (uint32_t step = 0; step < t.segmask && __any_sync(kFullMask, act); ++step) {
-        if (act) {
-          const Sector s = load_sector(t.slots, b);
-          uint32_t q = 0, p;
-          const bool f = SLOT ? Ops::find_slot(s, key, rid_mask, q) : Ops::find(s, key, rid_mask, p, q);
-          if (f) res = SLOT ? b * Ops::kSlots + q : p;
-          act = !f && !Ops::open(s);
-          b = next_bucket(b, t.segmask);
-        }
-      }
-      if (e < n_wait) wait.bucket[e] = res;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < S; ++j)
-      if (waits >> (8 * j) & 0xffu) pos[j] = wait.bucket[(waits >> (8 * j) & 0xffu) - 1];
-  }
-}
 
 // Sets the bits of the rows row0 + lane that `found` names: a whole word when the rows are in their own order,
 // else one bit for each partitioned row's row id. (Collected per tile in shared memory and flushed in lines, the
@@ -239,33 +129,36 @@ __device__ __forceinline__ void mark_found(uint32_t* words, const int32_t* prid_
   }
 }
 
-// The lookup alone: bit i of `words` = probe row i has a match. NULL rows match the NULL group if it has rows.
-template <typename K, bool WIDE, bool RUNS>
-__global__ void __launch_bounds__(kUnitThreads, 8) find_units_kernel(TableDev t, const K* __restrict__ keys,
-                                                                     const uint32_t* __restrict__ kv, int64_t kvoff,
-                                                                     uint32_t n, RunArgs ra,
-                                                                     const int32_t* __restrict__ prid_map, uint32_t* words) {
+// The lookup alone, in partition order: bit i of `words` = probe row i has a match. A CTA takes kFindBlocks blocks of
+// units, one after the other in the order of the partitions: a launch whose gate is closed is that much cheaper (64K
+// CTAs that return at once take 37 us). With a grid-stride loop instead the sweep lost its order, 1,457 us for 1,164,
+// and with four blocks 64M rows into 64M keys took 1,214 us instead of 1,157.
+constexpr int kFindBlocks = 2;
+
+template <typename K, bool WIDE>
+__global__ void __launch_bounds__(kUnitThreads, 8) find_units_kernel(TableDev t, const K* __restrict__ keys, uint32_t n,
+                                                                     RunArgs ra, const int32_t* __restrict__ prid_map,
+                                                                     uint32_t* words, RangeGate gate) {
   constexpr int S = 4;
   __shared__ WaitRows<S> s_wait[kUnitWarps];
+  if (!gate_open(gate)) return;
   const int lane = threadIdx.x & 31;
-  const Units u = cta_units<RUNS>(ra);
-  uint32_t first, rows;
-  unit_rows<RUNS, S>(ra, u, n, first, rows);
-  const bool null_found = !RUNS && t.null_group >= 0 && __ldg(t.grp_off + t.null_group + 1) > __ldg(t.grp_off + t.null_group);
-  for (uint32_t v0 = 0; v0 < rows; v0 += 32 * S) {
-    K k[S];
+  const uint32_t end = min(ra.P * run_ctas(ra), (blockIdx.x + 1) * kFindBlocks);
+  for (uint32_t cta = blockIdx.x * kFindBlocks; cta < end; ++cta) {
+    uint32_t first, rows;
+    unit_rows<true, S>(ra, cta_units<true>(ra, cta), n, first, rows);
+    for (uint32_t v0 = 0; v0 < rows; v0 += 32 * S) {
+      K k[S];
 #pragma unroll
-    for (int j = 0; j < S; ++j) {
-      const uint32_t v = v0 + 32 * j + lane;
-      k[j] = v < rows ? __ldcs(keys + first + v) : (K)0;
-    }
-    uint32_t pos[S];
-    unit_lookup<K, WIDE, RUNS, S>(t, k, kv, kvoff, first, v0, rows, s_wait[threadIdx.x >> 5], pos);
+      for (int j = 0; j < S; ++j) {
+        const uint32_t v = v0 + 32 * j + lane;
+        k[j] = v < rows ? __ldcs(keys + first + v) : (K)0;
+      }
+      uint32_t pos[S];
+      unit_lookup<K, WIDE, true, S>(t, k, nullptr, 0, first, v0, rows, s_wait[threadIdx.x >> 5], pos);
 #pragma unroll
-    for (int j = 0; j < S; ++j) {
-      const uint32_t v = v0 + 32 * j + lane;
-      const bool found = pos[j] != kNoPos || (null_found && v < rows && !bit_valid(kv, kvoff, first + v));
-      mark_found<RUNS>(words, prid_map, first + v0 + 32 * j, v0 + 32 * j < rows, __ballot_sync(kFullMask, found));
+      for (int j = 0; j < S; ++j)
+        mark_found<true>(words, prid_map, first + v0 + 32 * j, v0 + 32 * j < rows, __ballot_sync(kFullMask, pos[j] != kNoPos));
     }
   }
 }
@@ -284,7 +177,7 @@ __global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kern
   const unsigned below = (1u << lane) - 1u;
   WaitRows<S>& wait = s_wait[warp];
   const uint32_t cap = (uint32_t)(a.capacity < (int64_t)0x7fffffff ? a.capacity : (int64_t)0x7fffffff);
-  const Units u = cta_units<RUNS>(ra);
+  const Units u = cta_units<RUNS>(ra, blockIdx.x);
   uint32_t first, rows;
   unit_rows<RUNS, S>(ra, u, n, first, rows);
   for (uint32_t v0 = 0; __syncthreads_or(v0 < rows); v0 += 32 * S) {
@@ -330,12 +223,6 @@ __global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kern
   }
 }
 
-// Probes of at most this many rows take units of 32 rows: a row has a thread of its own and the chain of
-// dependent loads is all there is. Units of 32 against units of 128 rows, int32 keys and payloads: 10K rows
-// 4.0 / 7.0 us, 200K 5.4 / 7.6, 400K 8.4 / 8.4, 600K 11.7 / 10.4, 2M 30.6 / 28.3, 4M 61.5 / 50.6 us (two
-// warps of 64 rows with a reservation each, before: 6.5, 8.5, 12.8, 17.7, 50.5, 98.0 us).
-constexpr int64_t kFewRows = 400000;
-
 // GROUPED tables: each probe row's group. COMPACT: appends (row, group start, group size) of the rows with
 // matches; always: adds the matches up. One reservation per CTA (1024 rows): with one per warp of 128 rows the
 // entry counter alone took 176 us of a 32M-row probe (one same-address atomic per 0.67 ns).
@@ -351,7 +238,7 @@ __global__ void __launch_bounds__(kUnitThreads, 6) match_units_kernel(TableDev t
   __shared__ unsigned long long s_sum[kUnitWarps], s_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
-  const Units u = cta_units<false>(RunArgs{});
+  const Units u = cta_units<false>(RunArgs{}, blockIdx.x);
   uint32_t first, rows;
   unit_rows<false, S>(RunArgs{}, u, n, first, rows);
   K k[S];
@@ -477,18 +364,17 @@ void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_
   }
 }
 
-void find_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t kvoff, int64_t n, const RunArgs* runs,
-                const int32_t* prid_map, uint32_t* words, cudaStream_t s) {
+void find_units(const sj_table* t, const void* keys, int64_t n, const RunArgs& runs, const int32_t* prid_map,
+                uint32_t* words, const RangeGate& gate, cudaStream_t s) {
   if (n == 0) return;
-  const RunArgs ra = runs ? unit_pieces(*runs) : RunArgs{};
-  const int grid = unit_grid(n, 128, runs ? &ra : nullptr);
+  const RunArgs ra = unit_pieces(runs);
+  const int grid = (unit_grid(n, 128, &ra) + kFindBlocks - 1) / kFindBlocks;
   const TableDev d = table_dev(t);
   KernelTimer timer("find_units", s);
   auto go = [&](auto k, auto w) {
     using K = decltype(k);
-    constexpr bool W = decltype(w)::value;
-    auto kernel = runs ? find_units_kernel<K, W, true> : find_units_kernel<K, W, false>;
-    kernel<<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(keys), kv, kvoff, (uint32_t)n, ra, prid_map, words);
+    find_units_kernel<K, decltype(w)::value><<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(keys), (uint32_t)n, ra,
+                                                                           prid_map, words, gate);
   };
   const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
   if (t->key_type == SJ_INT32) {

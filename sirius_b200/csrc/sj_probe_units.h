@@ -10,10 +10,10 @@ namespace sj {
 void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t kvoff, int64_t n, const int64_t* d_n,
                  const RunArgs* runs, const DirectArgs& a, cudaStream_t s);
 
-// Bit i of `words` ((n + 31) / 32 of them): probe row i has a match in `t` (any layout). With `runs`, `keys` and
-// `prid_map` are the partitioned arrays, rows that cannot match are not in them, and `words` must be zero before.
-void find_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t kvoff, int64_t n, const RunArgs* runs,
-                const int32_t* prid_map, uint32_t* words, cudaStream_t s);
+// Sets bit i of `words` for every probe row i with a match in `t` (any layout), from the partitioned arrays `keys` and
+// `prid_map`, which lack the rows that cannot match. `words` must be zero before.
+void find_units(const sj_table* t, const void* keys, int64_t n, const RunArgs& runs, const int32_t* prid_map,
+                uint32_t* words, const RangeGate& gate, cudaStream_t s);
 
 // GROUPED table: adds the matches of all probe rows to *d_total and, when m_ent is given, appends {probe row, group
 // start} and the group size of the rows with matches to m_ent / m_cnt at *d_nent.

@@ -1,0 +1,138 @@
+// Units: the rows that a warp looks up together, and their lookup. A unit is 32 * S consecutive probe rows, or a
+// piece of a partition's run of a tile (tile-local partition); a CTA takes kUnitWarps consecutive ones. Shared by
+// the INNER probe, the lookups of GROUPED tables (sj_probe_units.cu) and the other join types (sj_probe_kinds.cu).
+#pragma once
+
+#include "sj_partition.cuh"
+#include "sj_probe_core.cuh"
+#include "sj_probe_direct.h"
+
+namespace sj {
+
+constexpr int kUnitThreads = 256;
+constexpr int kUnitWarps = kUnitThreads / 32;
+
+constexpr uint32_t kNoPos = 0xffffffffu;
+
+// Probes of at most this many rows take units of 32 rows: a row has a thread of its own and the chain of
+// dependent loads is all there is. Units of 32 against units of 128 rows, int32 keys and payloads: 10K rows
+// 4.0 / 7.0 us, 200K 5.4 / 7.6, 400K 8.4 / 8.4, 600K 11.7 / 10.4, 2M 30.6 / 28.3, 4M 61.5 / 50.6 us (two
+// warps of 64 rows with a reservation each, before: 6.5, 8.5, 12.8, 17.7, 50.5, 98.0 us).
+constexpr int64_t kFewRows = 400000;
+
+constexpr uint32_t kSampleRows = 1 << 15;
+
+__device__ __forceinline__ bool gate_open(const RangeGate& g) { return g.rows == nullptr || *g.rows >= g.need; }
+
+struct Units {
+  uint32_t part, first;  // RUNS: the CTA's partition; its first unit (piece of a run)
+};
+
+__device__ __forceinline__ uint32_t run_ctas(const RunArgs& ra) {  // of a partition
+  return ((ra.n_tiles << ra.log2_pieces) + kUnitWarps - 1) / kUnitWarps;
+}
+
+template <bool RUNS>
+__device__ __forceinline__ Units cta_units(const RunArgs& ra, uint32_t cta) {
+  Units u{0, cta * kUnitWarps};
+  if constexpr (RUNS) {
+    const uint32_t ctas = run_ctas(ra);
+    u.part = cta / ctas;
+    u.first = (cta - u.part * ctas) * kUnitWarps;
+  }
+  return u;
+}
+
+// First row and rows of the warp's unit.
+template <bool RUNS, int S>
+__device__ __forceinline__ void unit_rows(const RunArgs& ra, const Units& u, uint32_t n, uint32_t& first, uint32_t& rows) {
+  const uint32_t unit = u.first + (threadIdx.x >> 5);
+  first = rows = 0;
+  if constexpr (RUNS) {
+    const uint32_t tile = unit >> ra.log2_pieces, piece = unit & ((1u << ra.log2_pieces) - 1u);
+    if (tile >= ra.n_tiles) return;
+    const size_t at = (size_t)u.part * ra.n_tiles + tile;
+    const uint32_t cnt = (uint32_t)__ldg(ra.run_cnt + at), lo = cnt * piece >> ra.log2_pieces;
+    first = (uint32_t)__ldg(ra.run_off + at) + lo;
+    rows = (cnt * (piece + 1) >> ra.log2_pieces) - lo;
+  } else {
+    first = unit * (32 * S);
+    rows = first < n ? min(32u * S, n - first) : 0;
+  }
+}
+
+// A warp's rows that go on past their home bucket.
+template <int S>
+struct WaitRows {
+  SectorKey key[32 * S];
+  uint32_t bucket[32 * S];  // then the row's position
+};
+
+// Table positions (SLOT: slots) of rows first + v0 + 32 j + lane (keys k[j]) of the warp's unit, kNoPos where
+// there is none. RUNS: the partition has dropped NULL keys and those outside the build's key range.
+template <typename K, bool WIDE, bool RUNS, int S, bool SLOT = false>
+__device__ __forceinline__ void unit_lookup(const TableDev& t, const K (&k)[S], const uint32_t* __restrict__ kv, int64_t kvoff,
+                                            uint32_t first, uint32_t v0, uint32_t rows, WaitRows<S>& wait, uint32_t (&pos)[S]) {
+  using Ops = SectorOps<WIDE>;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const uint32_t rid_mask = (1u << t.rbits) - 1u;
+  uint32_t n_wait = 0;
+  uint32_t waits = 0;  // byte j: 1 + place in the list of the lane's row j, or 0
+#pragma unroll
+  for (int j = 0; j < S; ++j) {
+    const uint32_t v = v0 + 32 * j + lane;
+    SectorKey key;
+    uint32_t b = 0, q = 0;
+    pos[j] = kNoPos;
+    bool cont = false;
+    const bool in = sector_key<K, WIDE>(t, k[j], key);
+    if (v < rows && (RUNS || (in && bit_valid(kv, kvoff, first + v)))) {
+      b = home_bucket(t, key_u64<K>(k[j]));
+      const Sector s = load_sector(t.slots, b);
+      uint32_t p;
+      if (SLOT ? Ops::find_slot(s, key, rid_mask, q) : Ops::find(s, key, rid_mask, p, q)) pos[j] = SLOT ? b * Ops::kSlots + q : p;
+      else cont = t.segmask != 0 && !Ops::open(s);
+    }
+    const unsigned bal = __ballot_sync(kFullMask, cont);
+    if (bal) {
+      if (cont) {
+        const uint32_t e = n_wait + __popc(bal & below);
+        wait.key[e] = key;
+        wait.bucket[e] = next_bucket(b, t.segmask);
+        waits |= (e + 1) << (8 * j);
+      }
+      n_wait += __popc(bal);
+    }
+  }
+  if (n_wait) {
+    __syncwarp();
+    for (uint32_t e0 = 0; e0 < n_wait; e0 += 32) {
+      const uint32_t e = e0 + lane;
+      bool act = e < n_wait;
+      SectorKey key{};
+      uint32_t b = 0, res = kNoPos;
+      if (act) {
+        key = wait.key[e];
+        b = wait.bucket[e];
+      }
+      for (uint32_t step = 0; step < t.segmask && __any_sync(kFullMask, act); ++step) {
+        if (act) {
+          const Sector s = load_sector(t.slots, b);
+          uint32_t q = 0, p;
+          const bool f = SLOT ? Ops::find_slot(s, key, rid_mask, q) : Ops::find(s, key, rid_mask, p, q);
+          if (f) res = SLOT ? b * Ops::kSlots + q : p;
+          act = !f && !Ops::open(s);
+          b = next_bucket(b, t.segmask);
+        }
+      }
+      if (e < n_wait) wait.bucket[e] = res;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < S; ++j)
+      if (waits >> (8 * j) & 0xffu) pos[j] = wait.bucket[(waits >> (8 * j) & 0xffu) - 1];
+  }
+}
+
+}  // namespace sj
