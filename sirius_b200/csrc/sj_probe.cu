@@ -757,7 +757,7 @@ static sj_status probe_partitioned(const sj_table* t, const sj_column& p, Gather
     SJ_TRY(local_partition(ps, t->key_type, pbits, range.kmin, range.kmax, pd, LocalRuns{run_off, run_cnt}, t->device, s));
     g.prid_map = pd.rid;
     for (int c = 0; c < g.n_pin; ++c) g.pin[c] = column_payload(pd.pay[c], nullptr, 0, g.pin[c].width);
-    const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0};
+    const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0, 0};
     probe_runs(t, pd.keys, n, ra, g, s);
     SJ_CUDA_TRY(cudaGetLastError());
     return SJ_OK;
@@ -845,7 +845,7 @@ sj_status find_in_order(const sj_table* t, const sj_column& p, const Allocator& 
   int32_t* run_cnt = run_off + align256(run_bytes) / sizeof(int32_t);
   *gate = RangeGate{count, slots < 2 * kLeast ? kSampleRows / 4 * 3 : kSampleRows / 2};
   SJ_TRY(local_partition(ps, t->key_type, pbits, d.kmin, d.kmax, pd, LocalRuns{run_off, run_cnt, set, *gate}, t->device, s));
-  const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0};
+  const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0, 0};
   find_units(t, pd.keys, n, ra, pd.rid, set, *gate, s);
   SJ_CUDA_TRY(cudaGetLastError());
   *words = set;

@@ -41,7 +41,8 @@ struct RunArgs {
   const int32_t* run_cnt;
   uint32_t n_tiles;
   uint32_t P;
-  uint32_t log2_pieces;  // a run is split into 2^log2_pieces units
+  uint32_t log2_pieces;  // a run is split into 2^log2_pieces units,
+  uint32_t log2_join;    // or the runs of 2^log2_join consecutive tiles are one
 };
 
 // Fills `a` from a general gather description; false when the output shape needs the staged

@@ -190,8 +190,7 @@ __global__ void __launch_bounds__(kUnitThreads, 8) kind_units_kernel(TableDev t,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool null_found = NULLS && t.null_group >= 0 && __ldg(t.grp_off + t.null_group + 1) > __ldg(t.grp_off + t.null_group);
   for (uint32_t block = 0; block < BLOCKS; ++block) {
-    uint32_t first, rows;
-    unit_rows<false, S>(RunArgs{}, Units{0, (blockIdx.x * BLOCKS + block) * kUnitWarps}, n, first, rows);
+    const auto [first, rows] = unit_rows<false, S>(RunArgs{}, Units{0, (blockIdx.x * BLOCKS + block) * kUnitWarps}, n);
     K k[S];
 #pragma unroll
     for (int j = 0; j < S; ++j) k[j] = 32 * j + lane < rows ? __ldcs(keys + first + 32 * j + lane) : (K)0;

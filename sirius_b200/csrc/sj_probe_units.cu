@@ -112,20 +112,20 @@ __device__ __forceinline__ void emit_match(const DirectArgs& a, uint32_t row, in
 
 constexpr int kUnitCtasPerSm = 6;  // 40 registers
 
-// Sets the bits of the rows row0 + lane that `found` names: a whole word when the rows are in their own order,
-// else one bit for each partitioned row's row id. (Collected per tile in shared memory and flushed in lines, the
-// bits of 64M rows took 605-770 us with the lookup against 570: what shared memory takes from L1 and from the
+// Sets the bits of the lanes' rows that `found` names: a whole word when the rows are in their own order (lane 0's is
+// the word's first), else one bit for each partitioned row's row id. (Collected per tile in shared memory and flushed in
+// lines, the bits of 64M rows took 605-770 us with the lookup against 570: what shared memory takes from L1 and from the
 // warps per SM costs more than the atomics.)
 template <bool RUNS>
-__device__ __forceinline__ void mark_found(uint32_t* words, const int32_t* prid_map, uint32_t row0, bool any, unsigned found) {
+__device__ __forceinline__ void mark_found(uint32_t* words, const int32_t* prid_map, uint32_t row, bool any, unsigned found) {
   const int lane = threadIdx.x & 31;
   if constexpr (RUNS) {
     if (found >> lane & 1u) {
-      const uint32_t r = (uint32_t)__ldg(prid_map + row0 + lane);
+      const uint32_t r = (uint32_t)__ldg(prid_map + row);
       atomicOr(words + (r >> 5), 1u << (r & 31));
     }
   } else {
-    if (lane == 0 && any) words[row0 >> 5] = found;
+    if (lane == 0 && any) words[row >> 5] = found;
   }
 }
 
@@ -135,7 +135,7 @@ __device__ __forceinline__ void mark_found(uint32_t* words, const int32_t* prid_
 // and with four blocks 64M rows into 64M keys took 1,214 us instead of 1,157.
 constexpr int kFindBlocks = 2;
 
-template <typename K, bool WIDE>
+template <typename K, bool WIDE, bool JOIN>
 __global__ void __launch_bounds__(kUnitThreads, 8) find_units_kernel(TableDev t, const K* __restrict__ keys, uint32_t n,
                                                                      RunArgs ra, const int32_t* __restrict__ prid_map,
                                                                      uint32_t* words, RangeGate gate) {
@@ -145,25 +145,26 @@ __global__ void __launch_bounds__(kUnitThreads, 8) find_units_kernel(TableDev t,
   const int lane = threadIdx.x & 31;
   const uint32_t end = min(ra.P * run_ctas(ra), (blockIdx.x + 1) * kFindBlocks);
   for (uint32_t cta = blockIdx.x * kFindBlocks; cta < end; ++cta) {
-    uint32_t first, rows;
-    unit_rows<true, S>(ra, cta_units<true>(ra, cta), n, first, rows);
-    for (uint32_t v0 = 0; v0 < rows; v0 += 32 * S) {
+    const auto u = rows_of_unit<true, S, JOIN>(ra, cta_units<true>(ra, cta), n);
+    for (uint32_t v0 = 0; v0 < u.rows; v0 += 32 * S) {
       K k[S];
+      uint32_t row[S];
 #pragma unroll
       for (int j = 0; j < S; ++j) {
         const uint32_t v = v0 + 32 * j + lane;
-        k[j] = v < rows ? __ldcs(keys + first + v) : (K)0;
+        row[j] = u.row(v);
+        k[j] = v < u.rows ? __ldcs(keys + row[j]) : (K)0;
       }
       uint32_t pos[S];
-      unit_lookup<K, WIDE, true, S>(t, k, nullptr, 0, first, v0, rows, s_wait[threadIdx.x >> 5], pos);
+      unit_lookup<K, WIDE, true, S>(t, k, nullptr, 0, 0, v0, u.rows, s_wait[threadIdx.x >> 5], pos);
 #pragma unroll
       for (int j = 0; j < S; ++j)
-        mark_found<true>(words, prid_map, first + v0 + 32 * j, v0 + 32 * j < rows, __ballot_sync(kFullMask, pos[j] != kNoPos));
+        mark_found<true>(words, prid_map, row[j], v0 + 32 * j < u.rows, __ballot_sync(kFullMask, pos[j] != kNoPos));
     }
   }
 }
 
-template <typename K, bool WIDE, bool RUNS, int S, int SP, int SB>
+template <typename K, bool WIDE, bool RUNS, int S, int SP, int SB, bool JOIN = false>
 __global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kernel(TableDev t, const K* __restrict__ keys,
                                                                       const uint32_t* __restrict__ kv, int64_t kvoff,
                                                                       uint32_t n, const int64_t* d_n, RunArgs ra,
@@ -177,30 +178,32 @@ __global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kern
   const unsigned below = (1u << lane) - 1u;
   WaitRows<S>& wait = s_wait[warp];
   const uint32_t cap = (uint32_t)(a.capacity < (int64_t)0x7fffffff ? a.capacity : (int64_t)0x7fffffff);
-  const Units u = cta_units<RUNS>(ra, blockIdx.x);
-  uint32_t first, rows;
-  unit_rows<RUNS, S>(ra, u, n, first, rows);
-  for (uint32_t v0 = 0; __syncthreads_or(v0 < rows); v0 += 32 * S) {
+  const auto u = rows_of_unit<RUNS, S, JOIN>(ra, cta_units<RUNS>(ra, blockIdx.x), n);
+  uint32_t first = 0;
+  if constexpr (!JOIN) first = u.first;
+  for (uint32_t v0 = 0; __syncthreads_or(v0 < u.rows); v0 += 32 * S) {
     K k[S];
+    uint32_t row[S];
 #pragma unroll
     for (int j = 0; j < S; ++j) {
       const uint32_t v = v0 + 32 * j + lane;
-      k[j] = v < rows ? __ldcs(keys + first + v) : (K)0;
+      row[j] = u.row(v);
+      k[j] = v < u.rows ? __ldcs(keys + row[j]) : (K)0;
     }
     uint32_t pos[S];
-    unit_lookup<K, WIDE, RUNS, S>(t, k, kv, kvoff, first, v0, rows, wait, pos);
+    unit_lookup<K, WIDE, RUNS, S>(t, k, kv, kvoff, first, v0, u.rows, wait, pos);
     uint32_t cnt = 0;
 #pragma unroll
     for (int j = 0; j < S; ++j) {
       const unsigned bal = __ballot_sync(kFullMask, pos[j] != kNoPos);
       cnt += __popc(bal);
-      if constexpr (Sh::kMatched) mark_found<RUNS>(a.matched, a.prid_map, first + v0 + 32 * j, v0 + 32 * j < rows, bal);
+      if constexpr (Sh::kMatched) mark_found<RUNS>(a.matched, a.prid_map, row[j], v0 + 32 * j < u.rows, bal);
     }
     if (lane == 0) s_cnt[warp] = cnt;
     int32_t prid[S];
     uint64_t pv[S];
 #pragma unroll
-    for (int j = 0; j < S; ++j) load_probe_side<Sh>(a, first + v0 + 32 * j + lane, pos[j] != kNoPos, prid[j], pv[j]);
+    for (int j = 0; j < S; ++j) load_probe_side<Sh>(a, row[j], pos[j] != kNoPos, prid[j], pv[j]);
     __syncthreads();
     const uint32_t c = lane < kUnitWarps ? s_cnt[lane] : 0;
     const uint32_t incl = warp_inclusive_sum(c);
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) probe_units_kern
     for (int j = 0; j < S; ++j) {
       const bool hit = pos[j] != kNoPos;
       const unsigned bal = __ballot_sync(kFullMask, hit);
-      emit_match<Sh>(a, first + v0 + 32 * j + lane, prid[j], pv[j], pos[j], hit, [&](uint32_t& p, bool& live) {
+      emit_match<Sh>(a, row[j], prid[j], pv[j], pos[j], hit, [&](uint32_t& p, bool& live) {
         if (j == 0) {  // the reservation is back
           __syncthreads();
           run += s_base;
@@ -238,9 +241,7 @@ __global__ void __launch_bounds__(kUnitThreads, 6) match_units_kernel(TableDev t
   __shared__ unsigned long long s_sum[kUnitWarps], s_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned below = (1u << lane) - 1u;
-  const Units u = cta_units<false>(RunArgs{}, blockIdx.x);
-  uint32_t first, rows;
-  unit_rows<false, S>(RunArgs{}, u, n, first, rows);
+  const auto [first, rows] = unit_rows<false, S>(RunArgs{}, cta_units<false>(RunArgs{}, blockIdx.x), n);
   K k[S];
 #pragma unroll
   for (int j = 0; j < S; ++j) {
@@ -315,24 +316,33 @@ static DirectArgs plain_records(DirectArgs a) {
   return a;
 }
 
-// Runs cut into pieces of about 128 rows (a run holds kPartTileRows / P rows): with whole runs of 1024 rows a
-// warp's chain was eight times as long and the few warps of a 1M-row probe took 100 us instead of 63.
-static RunArgs unit_pieces(RunArgs ra) {
-  ra.log2_pieces = 0;
+// Units of about 128 rows: a run holds kPartTileRows / P rows. Longer ones are cut into pieces: with whole runs of 1024
+// rows a warp's chain was eight times as long and the few warps of a 1M-row probe took 100 us instead of 63. Short ones,
+// of `joined` partitions or more, are joined with those of neighbouring tiles: they lie side by side in the run tables,
+// and a row is found by a search of log2(tiles) shuffles. Unjoined, a unit of 256 partitions has 16 rows for its 128
+// places: 33.5M int64 rows into 4M keys, one payload, 1,271 us and 866 joined; into 100M keys, 128 partitions, 64M rows
+// with three payloads 2,615 and 2,186; their bits (SEMI, 256 partitions) 1,298 and 643. With 64 partitions a unit is
+// half full: bits 658 and 603, but 64M rows with three payloads 1,727 and 1,799.
+static RunArgs run_units(RunArgs ra, uint32_t joined) {
+  ra.log2_pieces = ra.log2_join = 0;
   while (((uint64_t)ra.P * 128 << ra.log2_pieces) < kPartTileRows) ++ra.log2_pieces;
+  if (ra.P < joined) return ra;
+  while (ra.log2_join < 5 && (uint64_t)kPartTileRows << ra.log2_join < (uint64_t)ra.P * 128) ++ra.log2_join;
   return ra;
 }
 
 static int unit_grid(int64_t n, int unit, const RunArgs* ra) {
   auto ctas = [](int64_t units) { return (units + kUnitWarps - 1) / kUnitWarps; };
-  return (int)(ra ? ra->P * ctas((int64_t)ra->n_tiles << ra->log2_pieces) : ctas((n + unit - 1) / unit));
+  if (!ra) return (int)ctas((n + unit - 1) / unit);
+  const int64_t tiles = ra->n_tiles;
+  return (int)(ra->P * ctas(ra->log2_join ? (tiles + (1 << ra->log2_join) - 1) >> ra->log2_join : tiles << ra->log2_pieces));
 }
 
 void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_t kvoff, int64_t n, const int64_t* d_n,
                  const RunArgs* runs, const DirectArgs& a_in, cudaStream_t s) {
   if (n == 0) return;
   const DirectArgs a = plain_records(a_in);
-  const RunArgs ra = runs ? unit_pieces(*runs) : RunArgs{};
+  const RunArgs ra = runs ? run_units(*runs, 128) : RunArgs{};
   const bool few = !runs && n <= kFewRows;
   const int grid = unit_grid(n, few ? 32 : 128, runs ? &ra : nullptr);
   const TableDev d = table_dev(t);
@@ -342,7 +352,8 @@ void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_
     using K = decltype(k);
     constexpr bool W = decltype(w)::value;
     constexpr int SP = decltype(sp)::value, SB = decltype(sb)::value;
-    auto kernel = runs ? probe_units_kernel<K, W, true, 4, SP, SB>
+    auto kernel = runs && ra.log2_join ? probe_units_kernel<K, W, true, 4, SP, SB, true>
+                  : runs ? probe_units_kernel<K, W, true, 4, SP, SB>
                   : few ? probe_units_kernel<K, W, false, 1, SP, SB> : probe_units_kernel<K, W, false, 4, SP, SB>;
     kernel<<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(keys), kv, kvoff, (uint32_t)n, d_n, ra, a);
   };
@@ -367,14 +378,15 @@ void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_
 void find_units(const sj_table* t, const void* keys, int64_t n, const RunArgs& runs, const int32_t* prid_map,
                 uint32_t* words, const RangeGate& gate, cudaStream_t s) {
   if (n == 0) return;
-  const RunArgs ra = unit_pieces(runs);
+  const RunArgs ra = run_units(runs, 64);
   const int grid = (unit_grid(n, 128, &ra) + kFindBlocks - 1) / kFindBlocks;
   const TableDev d = table_dev(t);
   KernelTimer timer("find_units", s);
   auto go = [&](auto k, auto w) {
     using K = decltype(k);
-    find_units_kernel<K, decltype(w)::value><<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(keys), (uint32_t)n, ra,
-                                                                           prid_map, words, gate);
+    constexpr bool W = decltype(w)::value;
+    auto kernel = ra.log2_join ? find_units_kernel<K, W, true> : find_units_kernel<K, W, false>;
+    kernel<<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(keys), (uint32_t)n, ra, prid_map, words, gate);
   };
   const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
   if (t->key_type == SJ_INT32) {

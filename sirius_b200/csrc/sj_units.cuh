@@ -1,5 +1,5 @@
 // Units: the rows that a warp looks up together, and their lookup. A unit is 32 * S consecutive probe rows, or a
-// piece of a partition's run of a tile (tile-local partition); a CTA takes kUnitWarps consecutive ones. Shared by
+// piece of a partition's run of a tile, or short runs of several tiles (tile-local partition); a CTA takes kUnitWarps consecutive ones. Shared by
 // the INNER probe, the lookups of GROUPED tables (sj_probe_units.cu) and the other join types (sj_probe_kinds.cu).
 #pragma once
 
@@ -29,7 +29,8 @@ struct Units {
 };
 
 __device__ __forceinline__ uint32_t run_ctas(const RunArgs& ra) {  // of a partition
-  return ((ra.n_tiles << ra.log2_pieces) + kUnitWarps - 1) / kUnitWarps;
+  const uint32_t units = ra.log2_join ? (ra.n_tiles + (1u << ra.log2_join) - 1u) >> ra.log2_join : ra.n_tiles << ra.log2_pieces;
+  return (units + kUnitWarps - 1) / kUnitWarps;
 }
 
 template <bool RUNS>
@@ -43,22 +44,53 @@ __device__ __forceinline__ Units cta_units(const RunArgs& ra, uint32_t cta) {
   return u;
 }
 
-// First row and rows of the warp's unit.
+// The warp's unit: its rows, numbered from 0, and where they are in the probe arrays.
+struct UnitRows {
+  uint32_t first, rows;
+  __device__ __forceinline__ uint32_t row(uint32_t v) const { return first + v; }
+};
+
+// Runs of up to 32 consecutive tiles, lane l's from the unit's row `before` on, at before + shift of the arrays.
+struct JoinedRows {
+  uint32_t rows, before, shift, log2_join;
+  // Called by the whole warp; v >= rows gives no row.
+  __device__ __forceinline__ uint32_t row(uint32_t v) const {
+    uint32_t tile = 0;  // the last one whose rows start at or before v
+    for (uint32_t step = 1u << log2_join >> 1; step; step >>= 1)
+      if (__shfl_sync(kFullMask, before, tile + step) <= v) tile += step;
+    return v + __shfl_sync(kFullMask, shift, tile);
+  }
+};
+
 template <bool RUNS, int S>
-__device__ __forceinline__ void unit_rows(const RunArgs& ra, const Units& u, uint32_t n, uint32_t& first, uint32_t& rows) {
+__device__ __forceinline__ UnitRows unit_rows(const RunArgs& ra, const Units& u, uint32_t n) {
   const uint32_t unit = u.first + (threadIdx.x >> 5);
-  first = rows = 0;
   if constexpr (RUNS) {
     const uint32_t tile = unit >> ra.log2_pieces, piece = unit & ((1u << ra.log2_pieces) - 1u);
-    if (tile >= ra.n_tiles) return;
+    if (tile >= ra.n_tiles) return {0, 0};
     const size_t at = (size_t)u.part * ra.n_tiles + tile;
     const uint32_t cnt = (uint32_t)__ldg(ra.run_cnt + at), lo = cnt * piece >> ra.log2_pieces;
-    first = (uint32_t)__ldg(ra.run_off + at) + lo;
-    rows = (cnt * (piece + 1) >> ra.log2_pieces) - lo;
+    return {(uint32_t)__ldg(ra.run_off + at) + lo, (cnt * (piece + 1) >> ra.log2_pieces) - lo};
   } else {
-    first = unit * (32 * S);
-    rows = first < n ? min(32u * S, n - first) : 0;
+    const uint32_t first = unit * (32 * S);
+    return {first, first < n ? min(32u * S, n - first) : 0};
   }
+}
+
+__device__ __forceinline__ JoinedRows joined_rows(const RunArgs& ra, const Units& u) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t tile = ((u.first + (threadIdx.x >> 5)) << ra.log2_join) + lane;
+  const bool mine = (uint32_t)lane >> ra.log2_join == 0 && tile < ra.n_tiles;
+  const size_t at = (size_t)u.part * ra.n_tiles + tile;
+  const uint32_t cnt = mine ? (uint32_t)__ldg(ra.run_cnt + at) : 0;
+  const uint32_t incl = warp_inclusive_sum(cnt);
+  return {__shfl_sync(kFullMask, incl, 31), incl - cnt, (mine ? (uint32_t)__ldg(ra.run_off + at) : 0u) - (incl - cnt), ra.log2_join};
+}
+
+template <bool RUNS, int S, bool JOIN>
+__device__ __forceinline__ auto rows_of_unit(const RunArgs& ra, const Units& u, uint32_t n) {
+  if constexpr (JOIN) return joined_rows(ra, u);
+  else return unit_rows<RUNS, S>(ra, u, n);
 }
 
 // A warp's rows that go on past their home bucket.
@@ -83,12 +115,11 @@ __device__ __forceinline__ void unit_lookup(const TableDev& t, const K (&k)[S], 
   for (int j = 0; j < S; ++j) {
     const uint32_t v = v0 + 32 * j + lane;
     SectorKey key;
-    uint32_t b = 0, q = 0;
+    uint32_t b = home_bucket(t, key_u64<K>(k[j])), q = 0;
     pos[j] = kNoPos;
     bool cont = false;
     const bool in = sector_key<K, WIDE>(t, k[j], key);
     if (v < rows && (RUNS || (in && bit_valid(kv, kvoff, first + v)))) {
-      b = home_bucket(t, key_u64<K>(k[j]));
       const Sector s = load_sector(t.slots, b);
       uint32_t p;
       if (SLOT ? Ops::find_slot(s, key, rid_mask, q) : Ops::find(s, key, rid_mask, p, q)) pos[j] = SLOT ? b * Ops::kSlots + q : p;

@@ -40,11 +40,13 @@ def test_unit_edges(cuda, n, dtype, bp_types):
 
 
 @pytest.mark.parametrize("n", [65_536, 16 * 4096 - 1, 16 * 4096 + 1, 300_007])
-@pytest.mark.parametrize("pbits", [1, 4, 10])
+@pytest.mark.parametrize("pbits", [1, 4, 5, 6, 8, 10])
 @pytest.mark.parametrize("wide", [False, True])
 def test_partition_runs(cuda, n, pbits, wide):
+    """From 64 partitions on a unit joins the runs of 2, 8 or 32 tiles, of which there may be fewer. The share is small
+    enough for the probe to take as many partitions as the table has."""
     rng = np.random.default_rng(n + pbits)
-    nb = 40_000
+    nb = 40_000 if pbits < 5 else 40_000 << pbits - 4  # at least 1 MB of slots and records for each partition
     bk = (rng.permutation(3 * nb)[:nb]).astype(np.int64)
     pk = rng.integers(0, 3 * nb, n).astype(np.int64)
     pk[: n // 3] = bk[0]  # one hot key: long runs of one partition
