@@ -655,6 +655,7 @@ __device__ __forceinline__ void col_write(const void* stage, const uint32_t* sds
   }
 }
 
+// At least one column.
 template <typename K>
 __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_columns_kernel(const K* __restrict__ keys, bool key_pairs,
                                                                       uint32_t n, int pbits, uint32_t chunk,
@@ -729,10 +730,7 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_columns_kerne
     __syncthreads();
     // 4. column by column (the key column, if wanted, comes first and is already in registers)
     const uint32_t t1 = t0 + kColTile;
-    if (cols.n == 0 || !cols.c[0].is_key) {
-      if (cols.n > 0) col_load(cols.c[0], t0, hi, v);
-      else if (t1 < hi) col_load_t(ukeys, key_pairs, t1, hi, v);
-    }
+    if (!cols.c[0].is_key) col_load(cols.c[0], t0, hi, v);
     for (int q = 0; q < cols.n; ++q) {
       const PartColumn& col = cols.c[q];
       switch (col.width) {
@@ -752,7 +750,6 @@ __global__ void __launch_bounds__(kColThreads, kColCtasPerSm) part_columns_kerne
       }
       __syncthreads();
     }
-    if (cols.n == 0) __syncthreads();
   }
 }
 
