@@ -6,8 +6,9 @@ sample of the real workload after warm-up:
 
 * batched launches: block size, probe group width, load factor, rows per work item
   (``sj_batch_params``), on a sample of the batch's joins;
-* single joins: radix partition bits ("partition fan-out"), output reservation (per warp or per
-  CTA), probe CTAs per SM and load factor (``sj_join_params``), on the table and a probe sample.
+* single joins: radix partition bits ("partition fan-out") and load factor (``sj_join_params``), on the
+  table and a probe sample; for payloads that take the staged probe also its output reservation (per
+  warp or per CTA) and CTAs per SM, which the unit probe does not look at.
 
 Results are cached per (GPU name, SM count, search, key type, size class) in a JSON file
 (``$SJ_AUTOTUNE_CACHE`` or ``~/.cache/sirius_b200/autotune.json``) so a size class is tuned once
@@ -33,9 +34,11 @@ BATCH_DEFAULT = {"block_size": 256, "group_width": 1, "load_factor": 0.5, "tile_
 
 JOIN_SPACE = {
     "partition_bits": [-1, 0, 3, 4, 5, 6, 7],
+    "load_factor": [0.35, 0.5, 0.7],
+}
+STAGED_SPACE = {  # knobs of the staged probe alone
     "aggregation": [L.SJ_AGG_WARP, L.SJ_AGG_CTA],
     "ctas_per_sm": [2, 3, 4, 6, 8],
-    "load_factor": [0.35, 0.5, 0.7],
 }
 JOIN_DEFAULT = {"partition_bits": 0, "aggregation": L.SJ_AGG_AUTO, "ctas_per_sm": 4, "load_factor": 0.5}
 
@@ -147,6 +150,16 @@ def tune_batch(specs, *, key_type: str = "int32", use_cache: bool = True, rounds
     return best
 
 
+def join_space(attach, probe_payload) -> Dict[str, list]:
+    """The knobs that a join of these payload columns (tensors or (tensor, validity) pairs) depends on: plain 4- and
+    8-byte columns, up to two of the probe and three of the build, are the unit probe's, others the staged probe's."""
+    def plain(c):
+        t, v = c if isinstance(c, (tuple, list)) else (c, None)
+        return v is None and t.element_size() in (4, 8)
+    unit = len(probe_payload) <= 2 and len(attach) <= 3 and all(plain(c) for c in [*attach, *probe_payload])
+    return dict(JOIN_SPACE) if unit else {**JOIN_SPACE, **STAGED_SPACE}
+
+
 def tune_join(build_keys, probe_keys, attach=(), probe_payload=(), *, use_cache: bool = True, rounds: int = 1,
               log: Optional[List] = None) -> Dict:
     """Best single-join parameters for a build table and a probe sample (INNER, attached payloads)."""
@@ -171,7 +184,7 @@ def tune_join(build_keys, probe_keys, attach=(), probe_payload=(), *, use_cache:
             finally:
                 t.close(stream)
 
-    best = coordinate_descent(JOIN_SPACE, JOIN_DEFAULT, measure, rounds, log)
+    best = coordinate_descent(join_space(attach, probe_payload), JOIN_DEFAULT, measure, rounds, log)
     if use_cache:
         cache[key] = best
         _store_cache(cache)

@@ -35,3 +35,13 @@ def test_cache_round_trip(tmp_path, monkeypatch):
 
 def test_size_class():
     assert A.size_class(1) == 0 and A.size_class(1 << 20) == 20 and A.size_class((1 << 20) + 5) == 20
+
+
+def test_only_knobs_that_the_probe_looks_at_are_swept():
+    import torch
+    i8, i4, i2 = (torch.zeros(4, dtype=t) for t in (torch.int64, torch.int32, torch.int16))
+    words = torch.zeros(1, dtype=torch.int32)
+    for attach, pp in (((), ()), ((i8, i4, i8), (i8, i4)), ([(i8, None)], [i4])):
+        assert set(A.join_space(attach, pp)) == {"partition_bits", "load_factor"}
+    for attach, pp in (((i8, i8, i8, i8), ()), ((), (i4, i4, i4)), ((i2,), ()), ((), ((i8, words),))):
+        assert {"aggregation", "ctas_per_sm"} < set(A.join_space(attach, pp))
