@@ -507,10 +507,15 @@ static int kind_grid(const sj_table* t, int64_t n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sm_count(t->device) * 8));
 }
 
+// Probes of at most this many rows take units of 32 rows. Units of 32 against units of 128, int64 keys, SEMI with a
+// payload / MARK: 10K rows 3.7 / 2.8 against 5.1 / 3.6 us, 200K 4.7 / 3.6 against 5.6 / 4.2, 300K 6.3 / 5.0 against
+// 6.3 / 5.0, 400K 7.3 / 5.4 against 6.3 / 4.8.
+constexpr int64_t kFewKindRows = 300000;
+
 template <int MODE>
 static void launch_kind(const sj_table* t, const sj_column& p, const KindArgs& a, cudaStream_t s) {
   constexpr int kBlocks = 4;
-  const bool gated = MODE != kFlags && a.gate.rows, few = MODE != kFlags && !gated && p.num_rows <= kFewRows;
+  const bool gated = MODE != kFlags && a.gate.rows, few = MODE != kFlags && !gated && p.num_rows <= kFewKindRows;
   const int64_t per_cta = (few ? 32 : 128) * kUnitWarps * (gated ? kBlocks : 1);
   const int grid = (int)((p.num_rows + per_cta - 1) / per_cta);
   const bool wide = t->slot_kind == SJ_SLOT_WIDE128;

@@ -14,10 +14,11 @@ constexpr int kUnitWarps = kUnitThreads / 32;
 
 constexpr uint32_t kNoPos = 0xffffffffu;
 
-// Probes of at most this many rows take units of 32 rows: a row has a thread of its own and the chain of
-// dependent loads is all there is. Units of 32 against units of 128 rows, int32 keys and payloads: 10K rows
-// 4.0 / 7.0 us, 200K 5.4 / 7.6, 400K 8.4 / 8.4, 600K 11.7 / 10.4, 2M 30.6 / 28.3, 4M 61.5 / 50.6 us (two
-// warps of 64 rows with a reservation each, before: 6.5, 8.5, 12.8, 17.7, 50.5, 98.0 us).
+// INNER probes of at most this many rows take units of 32 rows: a row has a thread of its own and the chain of
+// dependent loads is all there is. Units of 32 against units of 128 rows, keys and payloads of 4 bytes: 10K rows
+// 4.0 / 6.9 us, 200K 5.4 / 7.6, 400K 8.4 / 8.5, 600K 11.8 / 10.6, 2M 30.2 / 28.6 (two warps of 64 rows with a
+// reservation each, before: 6.5, 8.5, 12.8, 17.7, 50.5); of 8 bytes: 200K 5.5 / 7.9, 400K 8.5 / 9.1, 600K 12.0 / 11.3;
+// 128-bit slots: 200K 5.9 / 8.5, 400K 9.4 / 9.8, 600K 14.0 / 12.3.
 constexpr int64_t kFewRows = 400000;
 
 constexpr uint32_t kSampleRows = 1 << 15;
