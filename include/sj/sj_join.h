@@ -169,7 +169,9 @@ typedef struct sj_join_params {
                                when the table and its attached payloads outgrow L2), -1 = never,
                                1..10 = that many bits (2^bits partitions) */
   int32_t force_wide;       /* 1 = use SJ_SLOT_WIDE128 even when the packed encoding fits */
-  int32_t ctas_per_sm;      /* grid = ctas_per_sm * SM count for grid-stride kernels; default 4 */
+  int32_t ctas_per_sm;      /* grid limit, in CTAs per SM, of the build's kernels (twice as many) and of the
+                               staged and DIRECT_TMA probes; the unit probe's grid follows from the rows.
+                               Default 4 */
   int32_t aggregation;      /* sj_aggregation: how the staged probe reserves output positions */
   int32_t probe_kernel;     /* sj_probe_kernel: write-out of DISTINCT probes; default AUTO */
   int32_t rows_per_lane;    /* 0, 2, 3 or 4: accepted and ignored (the unit probe holds 1 or 4 rows per

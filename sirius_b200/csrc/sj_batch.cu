@@ -274,8 +274,9 @@ __device__ __forceinline__ uint64_t pay_load(const PayloadIn& in, int64_t i) {
 // to 99 ms). So a warp collects its matches in a shared-memory area of kStage rows (probe row id,
 // build row id, both payloads) and reserves output once per ~kStage - 64 matches, then writes the
 // area out in contiguous runs. No holes: a flush reserves exactly the rows it holds.
-// The areas of an SM's 32 warps come out of L1, which the loads in flight need: 256 rows and a list of 128 took
-// 1,518 us on 64 joins of 1K..1M x 10, 192 and 96 take 1,447 (176: 1,452, 160: 1,529, 128: 1,532 us).
+// The areas of an SM's 32 warps come out of L1, which the loads in flight need, and a smaller one flushes more often.
+// The size is the best of five measured on one batch (64 joins of 1K..1M x 10 int32 rows), not derived: 256 rows and a
+// list of 128 took 1,518 us, 192 and 96 take 1,447 (176: 1,452, 160: 1,529, 128: 1,532 us).
 constexpr int kStage = 192;
 // per-warp list of rows that go on to their next bucket: {probe row, bucket}; it holds fewer than
 // 32 rows between passes, plus at most 32 * kBatchR added by one step

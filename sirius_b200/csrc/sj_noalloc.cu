@@ -111,7 +111,7 @@ static size_t noalloc_need(int64_t n_build, int64_t n_probe, double lf) {
   need += std::max(groups_full, groups_shrunk) + a256(1024 * 8);  // + the scan's block sums
   // group members and NULL-key row ids (together at most one per build row), the NULL-row counter
   need += a256(nb * 4) + 256 + a256(8);
-  // probe: the grouped match list in one request (a DISTINCT probe takes a 256-byte tile counter)
+  // probe: the grouped match list in one request (a DISTINCT probe takes none)
   need += a256(3 * a256(np * 4) + a256((np + 1) * 8) + 1024 * 8 + 256);
   return need;
 }
