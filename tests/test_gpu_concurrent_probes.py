@@ -1,9 +1,9 @@
 """GPU stress test of partitioned probes running at the same time on several streams into one
 resident table (the served case: sj_probe_* called concurrently on one built table). Every probe's
 result must be the same as the same probe run alone, and its match count the oracle's. The
-tile-local partition and the run-walking probe of a partitioned table are timing-sensitive (CTAs
-take work items from a shared counter, per-tile run tables are built in shared memory), so the
-probes are repeated with the streams competing for the SMs."""
+tile-local partition and the probe of its runs are timing-sensitive (a call's scratch is reused by
+the next as soon as its stream allows, output is reserved CTA by CTA), so the probes are repeated
+with the streams competing for the SMs."""
 import numpy as np
 import pytest
 import torch

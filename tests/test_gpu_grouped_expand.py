@@ -14,22 +14,29 @@ from sirius_b200 import join as J
 pytestmark = pytest.mark.gpu
 
 
-def _run(cuda, sizes, n_probe, types, seed, capacity=None, null_frac=0.0, absent=0.0):
+def _run(cuda, sizes, n_probe, types, seed, capacity=None, null_frac=0.0, absent=0.0, nulls_equal=False, build_nulls=0):
     rng = np.random.default_rng(seed)
     keys = rng.permutation(4 * len(sizes))[: len(sizes)].astype(np.int64)
     bk = np.repeat(keys, sizes)
     bk = bk[rng.permutation(len(bk))]
+    bv = None
+    if build_nulls:
+        valid = np.ones(len(bk), bool)
+        valid[rng.permutation(len(bk))[:build_nulls]] = False
+        bv = O.pack_validity(valid)
     pk = np.where(rng.random(n_probe) < absent, -5, rng.choice(keys, n_probe)).astype(np.int64)
     pv = O.pack_validity(rng.random(n_probe) >= null_frac) if null_frac else None
     bp = [rng.integers(0, 1 << 30, len(bk)).astype(t) for t in types]
-    inp = D.JoinInput("expand", bk, pk, bp, [], None, pv)
-    with J.HashTable(dev_t(bk, cuda), attach=[dev_t(c, cuda) for c in bp], layout=L.SJ_LAYOUT_GROUPED) as t:
+    inp = D.JoinInput("expand", bk, pk, bp, [], bv, pv)
+    rule = L.SJ_NULLS_EQUAL if nulls_equal else L.SJ_NULLS_UNEQUAL
+    with J.HashTable(dev_t(bk, cuda), dev_valid(bv, cuda), attach=[dev_t(c, cuda) for c in bp],
+                     layout=L.SJ_LAYOUT_GROUPED, null_equality=rule) as t:
         out = J.allocate_output(capacity, (), [dev_t(c, cuda) for c in bp]) if capacity else None
         dc = torch.zeros(1, dtype=torch.int64, device=cuda)
         total = int(t.count(dev_t(pk, cuda), dev_valid(pv, cuda)).item())
         out = t.probe_gather(dev_t(pk, cuda), dev_valid(pv, cuda), attached=True, out=out, d_count=dc, sync=False)
     torch.cuda.synchronize()
-    exp = oracle_join(inp)
+    exp = oracle_join(inp, nulls_equal)
     assert int(dc.item()) == total == len(exp[0])
     n = min(total, capacity or total)
     got = [x[:n].cpu().numpy() for x in [out.probe_rid, out.build_rid] + out.build_payload]
@@ -55,6 +62,20 @@ def test_group_sizes(cuda, sizes, types, n_probe, absent, null_frac):
     if sizes == "mixed":
         n_probe = min(n_probe, 33)
     _run(cuda, s, n_probe, types, n_probe, None, null_frac, absent)
+
+
+@pytest.mark.parametrize("nulls_equal", [False, True])
+@pytest.mark.parametrize("types", [(np.int32,), (), (np.int16, np.int64)])
+@pytest.mark.parametrize("build_nulls,n_probe", [(1, 1), (33, 129), (257, 1025), (2500, 40)])
+def test_null_group(cuda, nulls_equal, types, build_nulls, n_probe):
+    """NULL keys on both sides: the NULL group is matched like any other when NULLs are equal, else by nothing."""
+    _run(cuda, SIZES["ones"](None), n_probe, types, build_nulls, None, 0.3, 0.2, nulls_equal, build_nulls)
+
+
+@pytest.mark.parametrize("nulls_equal", [False, True])
+def test_build_without_null_rows(cuda, nulls_equal):
+    """NULL probe keys, and no NULL group to match."""
+    _run(cuda, SIZES["small"](np.random.default_rng(3)), 1025, (np.int32,), 11, None, 0.4, 0.0, nulls_equal)
 
 
 @pytest.mark.parametrize("capacity", [1, 31, 255, 256, 257, 2047, 2049, 5000])

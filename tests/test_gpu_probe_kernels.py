@@ -61,11 +61,13 @@ def test_kernels_match_oracle(cuda, kernel, dtype, pbits, attach):
     assert_same_rows(got, oracle_join(inp))
 
 
+@pytest.mark.parametrize("kernel", [L.SJ_PROBE_KERNEL_DIRECT, L.SJ_PROBE_KERNEL_STAGED])
 @pytest.mark.parametrize("agg", [L.SJ_AGG_WARP, L.SJ_AGG_CTA, L.SJ_AGG_WARP_DYNAMIC])
-def test_direct_output_reservation_modes(cuda, agg):
+def test_direct_output_reservation_modes(cuda, agg, kernel):
+    """The staged kernel reserves as asked; the direct one per CTA, whatever is asked for."""
     inp = _input(15, np.int64, 300_001, 2_000_003)
     for pbits in (-1, 3):
-        got = _run(inp, cuda, L.SJ_PROBE_KERNEL_DIRECT, True, partition_bits=pbits, aggregation=agg)
+        got = _run(inp, cuda, kernel, True, partition_bits=pbits, aggregation=agg)
         assert_same_rows(got, oracle_join(inp))
 
 
