@@ -792,7 +792,7 @@ __global__ void __launch_bounds__(256) sample_range_kernel(TableDev t, const K* 
 //   512 MB   375 / 355     1,347 / 1,072       784 / 815
 //   1 GB                   1,484 / 1,124       843 / 850
 // So: slots of 256 MB or more, 32M rows or more that touch each sector about once or more, and a key in the build's
-// range for 3/4 of the rows (1/2 from 512 MB on). The last only the device knows: a sample decides there, and what
+// range for 5/8 of the rows (1/2 from 512 MB on). The last only the device knows: a sample decides there, and what
 // runs in vain then takes about 40 us. In place, too, when the scratch is refused, and in a capture, whose graph would go on to use
 // memory that the caller's allocator has got back.
 sj_status find_in_order(const sj_table* t, const sj_column& p, const Allocator& alloc, cudaStream_t s, Scratch& bits,
@@ -825,13 +825,15 @@ sj_status find_in_order(const sj_table* t, const sj_column& p, const Allocator& 
   SJ_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(uint32_t), s));
   uint32_t* set = count + 4;
   const TableDev d = table_dev(t);
-  KernelTimer timer("sample_range", s);
-  if (t->key_type == SJ_INT32)
-    sample_range_kernel<int32_t><<<kSampleRows / 256, 256, 0, s>>>(d, static_cast<const int32_t*>(p.data), p.validity,
-                                                                   p.validity_offset, n, count);
-  else
-    sample_range_kernel<int64_t><<<kSampleRows / 256, 256, 0, s>>>(d, static_cast<const int64_t*>(p.data), p.validity,
-                                                                   p.validity_offset, n, count);
+  {
+    KernelTimer timer("sample_range", s);
+    if (t->key_type == SJ_INT32)
+      sample_range_kernel<int32_t><<<kSampleRows / 256, 256, 0, s>>>(d, static_cast<const int32_t*>(p.data), p.validity,
+                                                                     p.validity_offset, n, count);
+    else
+      sample_range_kernel<int64_t><<<kSampleRows / 256, 256, 0, s>>>(d, static_cast<const int64_t*>(p.data), p.validity,
+                                                                     p.validity_offset, n, count);
+  }
   char* cur = reinterpret_cast<char*>(align256(reinterpret_cast<size_t>(sc.ptr)));
   PartSrc ps{};
   PartDst pd{};
@@ -843,7 +845,7 @@ sj_status find_in_order(const sj_table* t, const sj_column& p, const Allocator& 
   pd.rid = reinterpret_cast<int32_t*>(cur + align256((size_t)n * kw));
   int32_t* run_off = reinterpret_cast<int32_t*>(cur + align256((size_t)n * kw) + align256((size_t)n * 4));
   int32_t* run_cnt = run_off + align256(run_bytes) / sizeof(int32_t);
-  *gate = RangeGate{count, slots < 2 * kLeast ? kSampleRows / 4 * 3 : kSampleRows / 2};
+  *gate = RangeGate{count, slots < 2 * kLeast ? kSampleRows / 8 * 5 : kSampleRows / 2};
   SJ_TRY(local_partition(ps, t->key_type, pbits, d.kmin, d.kmax, pd, LocalRuns{run_off, run_cnt, set, *gate}, t->device, s));
   const RunArgs ra{run_off, run_cnt, (uint32_t)n_tiles, 1u << pbits, 0, 0};
   find_units(t, pd.keys, n, ra, pd.rid, set, *gate, s);

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kUnitThreads, 8) kind_units_kernel(TableDev t,
   __shared__ unsigned long long s_base;
   // the match bits are complete: the rows are emitted, the build rows found by them
   if ((MODE == kAnti || MODE == kFlags) && a.inner_rows && (int64_t)*a.inner_rows <= a.capacity) return;
-  if (BLOCKS > 1 && gate_open(a.gate)) return;  // looked up in partition order
+  if (BLOCKS > 1 && a.gate.rows && gate_open(a.gate)) return;  // looked up in partition order
   const uint32_t* kv = NULLS ? kv_in : nullptr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool null_found = NULLS && t.null_group >= 0 && __ldg(t.grp_off + t.null_group + 1) > __ldg(t.grp_off + t.null_group);
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kUnitThreads) select_rows_kernel(const uint32_
       at[h] = __shfl_sync(kFullMask, mine, q0 + h) + __popc(wq & below);
       if ((wq >> lane & 1u) && at[h] < room) sel |= 1u << h;
     }
-    emit_rows<B>(a, row, base, at, sel);
+    if (__any_sync(kFullMask, sel != 0)) emit_rows<B>(a, row, base, at, sel);
   }
 }
 
@@ -515,8 +515,9 @@ constexpr int64_t kFewKindRows = 300000;
 template <int MODE>
 static void launch_kind(const sj_table* t, const sj_column& p, const KindArgs& a, cudaStream_t s) {
   constexpr int kBlocks = 4;
-  const bool gated = MODE != kFlags && a.gate.rows, few = MODE != kFlags && !gated && p.num_rows <= kFewKindRows;
-  const int64_t per_cta = (few ? 32 : 128) * kUnitWarps * (gated ? kBlocks : 1);
+  const bool idle = a.gate.rows || a.inner_rows;  // may have nothing to do
+  const bool few = MODE != kFlags && !idle && p.num_rows <= kFewKindRows;
+  const int64_t per_cta = (few ? 32 : 128) * kUnitWarps * (idle ? kBlocks : 1);
   const int grid = (int)((p.num_rows + per_cta - 1) / per_cta);
   const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
   const TableDev d = table_dev(t);
@@ -530,9 +531,9 @@ static void launch_kind(const sj_table* t, const sj_column& p, const KindArgs& a
                                            (uint32_t)p.num_rows, a);
     };
     if constexpr (MODE == kFlags) {
-      launch(kind_units_kernel<K, W, MODE, 4, true, 1>);
+      launch(idle ? kind_units_kernel<K, W, MODE, 4, true, kBlocks> : kind_units_kernel<K, W, MODE, 4, true, 1>);
     } else {
-      if (gated) launch(p.validity ? kind_units_kernel<K, W, MODE, 4, true, kBlocks> : kind_units_kernel<K, W, MODE, 4, false, kBlocks>);
+      if (idle) launch(p.validity ? kind_units_kernel<K, W, MODE, 4, true, kBlocks> : kind_units_kernel<K, W, MODE, 4, false, kBlocks>);
       else if (p.validity) launch(few ? kind_units_kernel<K, W, MODE, 1, true, 1> : kind_units_kernel<K, W, MODE, 4, true, 1>);
       else launch(few ? kind_units_kernel<K, W, MODE, 1, false, 1> : kind_units_kernel<K, W, MODE, 4, false, 1>);
     }
