@@ -175,7 +175,8 @@ __device__ __forceinline__ void mark_bytes(uint8_t* mark, const unsigned (&found
 // and 477 / -). With 48 warps: 706 / 1,250 and 512 / 1,069. NULLS: the probe keys have NULLs (apart, since the test for
 // the bitmask alone took 38 of 387 us of a MARK). Where all of a unit lies outside the build's range nothing is looked
 // up (64M rows, SEMI 277 -> 127 us); MARK, for which it cost 4 %, does not ask. BLOCKS: consecutive blocks of units per
-// CTA, for a launch that may have nothing to do (64K CTAs that return at once take 37 us).
+// CTA, for a launch that may have nothing to do (64K CTAs that return at once take 37 us). Not every form has a variant
+// of its own: the first call of a process loads them all (64 take 5.3 ms).
 template <typename K, bool WIDE, int MODE, int S, bool NULLS, int BLOCKS>
 __global__ void __launch_bounds__(kUnitThreads, 8) kind_units_kernel(TableDev t, const K* __restrict__ keys,
                                                                      const uint32_t* __restrict__ kv_in, int64_t kvoff,
@@ -508,15 +509,15 @@ static int kind_grid(const sj_table* t, int64_t n) {
 }
 
 // Probes of at most this many rows take units of 32 rows. Units of 32 against units of 128, int64 keys, SEMI with a
-// payload / MARK: 10K rows 3.7 / 2.8 against 5.1 / 3.6 us, 200K 4.7 / 3.6 against 5.6 / 4.2, 300K 6.3 / 5.0 against
+// payload / MARK: 10K rows 3.8 / 2.9 against 5.1 / 3.6 us, 200K 4.9 / 3.8 against 5.6 / 4.2, 300K 6.6 / 5.3 against
 // 6.3 / 5.0, 400K 7.3 / 5.4 against 6.3 / 4.8.
-constexpr int64_t kFewKindRows = 300000;
+constexpr int64_t kFewKindRows = 1 << 18;
 
 template <int MODE>
 static void launch_kind(const sj_table* t, const sj_column& p, const KindArgs& a, cudaStream_t s) {
   constexpr int kBlocks = 4;
-  const bool idle = a.gate.rows || a.inner_rows;  // may have nothing to do
-  const bool few = MODE != kFlags && !idle && p.num_rows <= kFewKindRows;
+  const bool idle = MODE == kFlags || a.gate.rows || a.inner_rows;  // may have nothing to do
+  const bool few = !idle && p.num_rows <= kFewKindRows;
   const int64_t per_cta = (few ? 32 : 128) * kUnitWarps * (idle ? kBlocks : 1);
   const int grid = (int)((p.num_rows + per_cta - 1) / per_cta);
   const bool wide = t->slot_kind == SJ_SLOT_WIDE128;
@@ -531,11 +532,11 @@ static void launch_kind(const sj_table* t, const sj_column& p, const KindArgs& a
                                            (uint32_t)p.num_rows, a);
     };
     if constexpr (MODE == kFlags) {
-      launch(idle ? kind_units_kernel<K, W, MODE, 4, true, kBlocks> : kind_units_kernel<K, W, MODE, 4, true, 1>);
+      launch(kind_units_kernel<K, W, MODE, 4, true, kBlocks>);
     } else {
       if (idle) launch(p.validity ? kind_units_kernel<K, W, MODE, 4, true, kBlocks> : kind_units_kernel<K, W, MODE, 4, false, kBlocks>);
-      else if (p.validity) launch(few ? kind_units_kernel<K, W, MODE, 1, true, 1> : kind_units_kernel<K, W, MODE, 4, true, 1>);
-      else launch(few ? kind_units_kernel<K, W, MODE, 1, false, 1> : kind_units_kernel<K, W, MODE, 4, false, 1>);
+      else if (few) launch(kind_units_kernel<K, W, MODE, 1, true, 1>);
+      else launch(p.validity ? kind_units_kernel<K, W, MODE, 4, true, 1> : kind_units_kernel<K, W, MODE, 4, false, 1>);
     }
   };
   if (t->key_type == SJ_INT32) {

@@ -352,7 +352,9 @@ void probe_units(const sj_table* t, const void* keys, const uint32_t* kv, int64_
     using K = decltype(k);
     constexpr bool W = decltype(w)::value;
     constexpr int SP = decltype(sp)::value, SB = decltype(sb)::value;
-    auto kernel = runs && ra.log2_join ? probe_units_kernel<K, W, true, 4, SP, SB, true>
+    // joined runs, of very large tables, in the general shapes and the widest: a first call loads every variant
+    constexpr int JP = SP < 0 || SP == 1 ? SP : -1, JB = SP < 0 || SP == 1 ? SB : -1;
+    auto kernel = runs && ra.log2_join ? probe_units_kernel<K, W, true, 4, JP, JB, true>
                   : runs ? probe_units_kernel<K, W, true, 4, SP, SB>
                   : few ? probe_units_kernel<K, W, false, 1, SP, SB> : probe_units_kernel<K, W, false, 4, SP, SB>;
     kernel<<<grid, kUnitThreads, 0, s>>>(d, static_cast<const K*>(keys), kv, kvoff, (uint32_t)n, d_n, ra, a);
