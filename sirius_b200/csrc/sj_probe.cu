@@ -787,13 +787,14 @@ __global__ void __launch_bounds__(256) sample_range_kernel(TableDev t, const K* 
 // Which probe rows have a match, as one bit per row (SEMI, ANTI, MARK), in partition order. Against the lookup in
 // place (kind_units_kernel), us for SEMI of int64 keys, 70 % of the rows with a match and the others in the range:
 //   slots      16M rows        64M rows      64M, half of them out of range
-//   128 MB   237 / 326       782 / 1,024         (in place / in partition order)
-//   256 MB   312 / 334     1,102 / 1,035       713 / 790
-//   512 MB   375 / 355     1,347 / 1,072       784 / 815
-//   1 GB                   1,484 / 1,124       843 / 850
-// So: slots of 256 MB or more, 32M rows or more that touch each sector about once or more, and a key in the build's
-// range for 5/8 of the rows (1/2 from 512 MB on). The last only the device knows: a sample decides there, and what
-// runs in vain then takes about 40 us. In place, too, when the scratch is refused, and in a capture, whose graph would go on to use
+//   128 MB   223 / 328       732 / 1,022       535 / 775       (in place / in partition order)
+//   256 MB   311 / 336     1,093 / 1,026       643 / 788
+//   512 MB   374 / 370     1,349 / 1,061       737 / 804
+//   1 GB                   1,484 / 1,115       805 / 839
+// In place after the choice takes about 80 us more on 64M rows: the kernels of the other way return at once, and the
+// blocks of its CTAs follow one another. So: slots of 256 MB or more, 32M rows or more that touch each sector about
+// once or more, and a key in the build's range for 5/8 of the rows (1/2 from 512 MB on). The last only the device
+// knows: a sample decides there. In place, too, when the scratch is refused, and in a capture, whose graph would go on to use
 // memory that the caller's allocator has got back.
 sj_status find_in_order(const sj_table* t, const sj_column& p, const Allocator& alloc, cudaStream_t s, Scratch& bits,
                         const uint32_t** words, RangeGate* gate) {

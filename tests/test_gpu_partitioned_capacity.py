@@ -1,6 +1,6 @@
 """The partitioned probe's output contract at sizes that take the tile-local partition and the
-run-walking probe: the output against the oracle, under both output reservations (AUTO and one
-atomicAdd per CTA chunk), at match rates from none to all, with capacities equal to the match
+probe of its runs: the output against the oracle, with the output reservation left open (AUTO) and
+asked for per CTA, at match rates from none to all, with capacities equal to the match
 count, above it and below it. Below it the full count is reported, nothing past the capacity is
 written, and every row written is a real match."""
 import numpy as np
