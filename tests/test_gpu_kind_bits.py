@@ -227,6 +227,42 @@ def test_captured_join_asks_for_no_scratch(cuda, kind):
         del g
 
 
+@pytest.mark.parametrize("n", [33, 1025, 300_001])
+@pytest.mark.parametrize("kind", [L.SJ_JOIN_SEMI, L.SJ_JOIN_ANTI, L.SJ_JOIN_MARK])
+def test_validity_at_odd_bit_offsets(cuda, kind, n):
+    """Slices of columns: key and payload bitmasks that do not start at a word, mark bytes that do not start at four."""
+    rng = np.random.default_rng(n)
+    bk, pk = rng.permutation(4000)[:2000].astype(np.int32), rng.integers(-500, 4500, n).astype(np.int32)
+    pv, av = rng.random(n) > 0.2, rng.random(n) > 0.4
+    hit = np.isin(pk, bk) & pv
+    pay = dev_t(rng.integers(0, 100, n).astype(np.int16), cuda)
+
+    def words(v, offset):
+        return dev_valid(O.pack_validity(np.concatenate([rng.random(offset) > 0.5, v])), cuda)
+    kw, aw = words(pv, 37), words(av, 5)
+    dpk = dev_t(pk, cuda)
+    keys = J._cols([J.make_column(dpk, kw, 37)])
+    pin = J._cols([J.make_column(pay, aw, 5)])
+    rid = torch.empty(n, dtype=torch.int32, device=cuda)
+    out, ow = torch.empty_like(pay), torch.empty((n + 31) // 32, dtype=torch.int32, device=cuda)
+    mark, mw = torch.empty(n + 3, dtype=torch.uint8, device=cuda)[3:], torch.empty_like(ow)
+    dc = torch.zeros(1, dtype=torch.int64, device=cuda)
+    with J.HashTable(dev_t(bk, cuda)) as t:
+        L.check(L.load().sj_probe_join(t.handle, kind, keys, 1, pin, 1, None, 0, rid.data_ptr(), None,
+                                       J._cols([J._mut(out, ow)], L.SjMutColumn), None, n, mark.data_ptr(),
+                                       mw.data_ptr(), None, None, dc.data_ptr()), "sj_probe_join")
+        torch.cuda.synchronize()
+    if kind == L.SJ_JOIN_MARK:
+        assert np.array_equal(mark.cpu().numpy().astype(bool), hit)
+        assert np.array_equal(_bits(mw, n).cpu().numpy(), hit | pv)
+        return
+    m = int(dc.item())
+    r = rid[:m].cpu().numpy()
+    assert np.array_equal(np.sort(r), np.nonzero(hit if kind == L.SJ_JOIN_SEMI else ~hit)[0])
+    assert np.array_equal(out[:m].cpu().numpy(), pay.cpu().numpy()[r])
+    assert np.array_equal(_bits(ow, m).cpu().numpy(), av[r])
+
+
 @pytest.mark.parametrize("kind", [L.SJ_JOIN_SEMI, L.SJ_JOIN_ANTI])
 def test_nulls_equal_and_null_build_keys_in_place(cuda, kind):
     """NULL probe keys match the NULL group, if the build has one (MARK compares NULLs as unequal)."""
