@@ -791,11 +791,11 @@ __global__ void __launch_bounds__(256) sample_range_kernel(TableDev t, const K* 
 //   256 MB   311 / 336     1,093 / 1,026       643 / 788
 //   512 MB   374 / 370     1,349 / 1,061       737 / 804
 //   1 GB                   1,484 / 1,115       805 / 839
-// In place after the choice takes about 80 us more on 64M rows: the kernels of the other way return at once, and the
+// In place after the choice takes about 40 us more on 64M rows: the kernels of the other way return at once, and the
 // blocks of its CTAs follow one another. So: slots of 256 MB or more, 32M rows or more that touch each sector about
 // once or more, and a key in the build's range for 5/8 of the rows (1/2 from 512 MB on). The last only the device
-// knows: a sample decides there. In place, too, when the scratch is refused, and in a capture, whose graph would go on to use
-// memory that the caller's allocator has got back.
+// knows: a sample decides there. In place, too, when the scratch is refused, and in a capture, whose graph would go
+// on to use memory that the caller's allocator has got back.
 sj_status find_in_order(const sj_table* t, const sj_column& p, const Allocator& alloc, cudaStream_t s, Scratch& bits,
                         const uint32_t** words, RangeGate* gate) {
   SJ_TRY(check_probe(t, p));

@@ -515,7 +515,9 @@ constexpr int64_t kFewKindRows = 1 << 18;
 
 template <int MODE>
 static void launch_kind(const sj_table* t, const sj_column& p, const KindArgs& a, cudaStream_t s) {
-  constexpr int kBlocks = 4;
+  // 64M rows, SEMI with two / four blocks: 539 / 563 us in place after the choice (70 % out of range), 1,034 / 1,023 in
+  // partition order; MARK 487 / 485 and 958 / 952
+  constexpr int kBlocks = MODE == kSemi || MODE == kAnti ? 2 : 4;
   const bool idle = MODE == kFlags || a.gate.rows || a.inner_rows;  // may have nothing to do
   const bool few = !idle && p.num_rows <= kFewKindRows;
   const int64_t per_cta = (few ? 32 : 128) * kUnitWarps * (idle ? kBlocks : 1);
